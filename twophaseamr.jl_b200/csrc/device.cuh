@@ -111,7 +111,6 @@ struct TuneConfig {
                              // 1 every level, above 1 levels of at most that many cells)
     int persistent = -1;     // all-CSR hierarchies: the V-cycle as one cooperative launch
     int tiles = -1;          // CSR levels: two launches per level on haloed block tiles (tiles.cuh)
-    int tail_smem = -1;      // 1: the coarse tail staged in shared memory (default: global memory)
 };
 
 struct SolveStats {
@@ -261,7 +260,11 @@ public:
 private:
     int tail_first_ = 0;
     int tail_ctas_ = 1;  // CTAs of the coarse-tail cluster
-    size_t tail_smem_[2] = {0, 0};  // > 0: dynamic shared bytes of the staged tail (FP64, FP32 cycle)
+    // the coarse tail as a dense map (tail_dense.cuh): cells of its first level
+    // (0: the tail's phases run in k_tail), row stride and entries
+    void build_dense_tail();
+    int dense_n_ = 0, dense_ld_ = 0;
+    DevArray<double> dense_M_;
     std::vector<LevelView<double>> vd_;
     std::vector<LevelView<float>> vf_;
     DevArray<LevelView<double>> vd_dev_;

@@ -11,7 +11,9 @@
 //                   with the coarse RHS sum folded in the same launch
 //   k_prolong       x += e - wt Dt^-1 A e with e = P_tent x_c, in place (it
 //                   reads no neighbouring fine value)
-//   k_tail          every level with at most kTailCells cells in one CTA
+//   k_tail          every level with at most kTailCells cells in one CTA: the
+//                   red-black tails and those above kDenseTailCells cells (the
+//                   others are one dense product, tail_dense.cuh)
 // Reductions fold their per-block partials in the last block to finish (a
 // fixed-order fold: results do not depend on block scheduling).
 #pragma once
@@ -23,9 +25,10 @@ namespace tpa {
 
 // Levels at or below this many cells run in the coarse tail, one cluster of
 // kTailCtasDefault CTAs of kTailThreads threads (TPAGMG_TAIL_CELLS, TPAGMG_TAIL_CTAS).
-// Measured on the B200 (droplet AMR and uniform 2048^2 solves): the tail is bound
-// by the latency of its dependent loads, so more CTAs or a larger tail (4096 to
-// 32768 cells, 4 or 8 CTAs) were 2-15 % slower than 2048 cells in one CTA.
+// At most kDenseTailCells cells run as one dense product (tail_dense.cuh, 3 us);
+// k_tail walks the rest: it is bound by the latency of its dependent loads, so
+// more CTAs or a larger tail (4096 to 32768 cells, 4 or 8 CTAs) were 2-15 %
+// slower than 2048 cells in one CTA (droplet AMR and uniform 2048^2 solves).
 constexpr int kTailCellsDefault = 2048;
 constexpr int kTailCtasDefault = 1;
 constexpr int kTailThreads = 1024;

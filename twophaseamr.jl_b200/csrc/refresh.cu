@@ -781,6 +781,7 @@ void DeviceSolver::refresh_levels() {
     // the level views (and the captured graphs, which hold them by value) change
     vd_dev_.upload(vd_.data(), vd_.size(), s);
     vf_dev_.upload(vf_.data(), vf_.size(), s);
+    build_dense_tail();
     // the face kernels' sqrt(kappa) (same faces, same zero set)
     if (nfaces_ >= 0 && rl_[0].nf > 0)
         TPA_CUDA(cudaMemcpyAsync(f_sqrtk_.p, rl_[0].sk.p, sizeof(double) * size_t(rl_[0].nf), cudaMemcpyDeviceToDevice,

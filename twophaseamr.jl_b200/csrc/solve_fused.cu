@@ -16,7 +16,7 @@
 #include "device.cuh"
 #include "persistent.cuh"
 #include "stream.cuh"
-#include "tail_smem.cuh"
+#include "tail_dense.cuh"
 
 namespace tpa {
 
@@ -779,35 +779,6 @@ void DeviceSolver::build_views() {
     }
     vd_dev_.upload(vd_.data(), vd_.size(), stream_);
     vf_dev_.upload(vf_.data(), vf_.size(), stream_);
-    // the coarse tail staged in shared memory when its levels fit (one CTA,
-    // Jacobi), on request only (TPAGMG_TAIL_SMEM or tail_smem = 1): measured on
-    // the droplet its copy-in costs more than the global-load chains it removes
-    // (V-cycle 101.6 against 97.9 us)
-    tail_smem_[0] = tail_smem_[1] = 0;
-    const bool want_tail_smem = tune_.tail_smem >= 0 ? tune_.tail_smem != 0 : std::getenv("TPAGMG_TAIL_SMEM") != nullptr;
-    if (fused_ok_ && !rb_ && tail_ctas_ == 1 && nl <= kTailSmemMaxLevels && want_tail_smem) {
-        size_t bd = 0, bf = 0;
-        for (int l = tail_first_; l < nl; ++l) {
-            const DevLevel& L = levels_[size_t(l)];
-            const bool last = l == nl - 1;
-            bd += tail_level_bytes<double>(L.n, int(L.nnz), last ? 0 : L.nc, last);
-            bf += tail_level_bytes<float>(L.n, int(L.nnz), last ? 0 : L.nc, last);
-        }
-        int optin = 0;
-        TPA_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
-        // room for the kernel's static shared memory (views, reductions)
-        const size_t room = size_t(optin) > 16384 ? size_t(optin) - 16384 : 0;
-        if (bd <= room) {
-            TPA_CUDA(cudaFuncSetAttribute(k_tail_smem<double, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          int(bd)));
-            tail_smem_[0] = bd;
-        }
-        if (bf <= room) {
-            TPA_CUDA(cudaFuncSetAttribute(k_tail_smem<float, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          int(bf)));
-            tail_smem_[1] = bf;
-        }
-    }
     // every folding launch has at most max(maxgrid, kMaxGrid) CTAs
     fpartial_.alloc(size_t(std::max<int64_t>(maxgrid, kMaxGrid)));
     fpartial2_.alloc(size_t(std::max<int64_t>(maxgrid, kMaxGrid)));
@@ -820,12 +791,45 @@ void DeviceSolver::build_views() {
     TPA_CUDA(cudaMemsetAsync(cgs_.p, 0, sizeof(CgState), stream_));
     spartial_.alloc(size_t(4) * size_t(kMaxGrid));
     spres_.alloc(8);
+    build_dense_tail();
     bar_.alloc(2);
     err_.alloc(1);
     TPA_CUDA(cudaMemsetAsync(bar_.p, 0, 2 * sizeof(unsigned), stream_));
     TPA_CUDA(cudaMemsetAsync(err_.p, 0, sizeof(int), stream_));
     TPA_CUDA(cudaStreamSynchronize(stream_));
     destroy_graphs();
+}
+
+// The coarse tail's linear map (tail_dense.cuh) for the default cycle with the
+// damped-Jacobi smoother: tails of at most kDenseTailCells cells, and a tail
+// that is the coarsest level alone at any size.  The level views on the device
+// are current.  The caller synchronizes before the next V-cycle.
+void DeviceSolver::build_dense_tail() {
+    const int nl = int(levels_.size()), t = tail_first_;
+    const int n = levels_[size_t(t)].n;
+    dense_n_ = 0;
+    if (!fused_ok_ || rb_ || (n > kDenseTailCells && t != nl - 1)) return;
+    int optin = 0;
+    TPA_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
+    const size_t room = size_t(optin) - 2048;  // the kernel's static shared memory
+    const int ld = (n + 1) & ~1;
+    auto build = [&](auto kernel, int C) {
+        const size_t bytes = dense_build_smem(vd_, t, C);
+        if (dense_n_ > 0 || bytes > room) return;
+        if (dense_M_.n != size_t(n) * size_t(ld)) {
+            dense_M_.alloc(size_t(n) * size_t(ld));
+            TPA_CUDA(cudaMemsetAsync(dense_M_.p, 0, dense_M_.n * sizeof(double), stream_));
+        }
+        TPA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
+        kernel<<<(n + C - 1) / C, kDenseBuildThreads, bytes, stream_>>>(
+            vd_dev_.p, t, nl, coarse_inv_.p, coarse_n_, t == 0 && vd_[0].singular ? 1 : 0, dense_M_.p, ld);
+        TPA_CUDA(cudaGetLastError());
+        dense_n_ = n;
+        dense_ld_ = ld;
+    };
+    build(k_dense_tail_build<4>, 4);
+    build(k_dense_tail_build<2>, 2);
+    build(k_dense_tail_build<1>, 1);
 }
 
 void DeviceSolver::destroy_graphs() {
@@ -996,18 +1000,22 @@ void DeviceSolver::enqueue_vcycle_epi(const R* r, const double* rsum, double* me
            next_sum ? lsum_.p + l + 1 : nullptr);
         launches_ += 3;
     }
-    const size_t tsm = tail_smem_[std::is_same<T, double>::value ? 0 : 1];
-    if (tsm > 0) {
-        // the tail's levels staged in shared memory (tail_smem.cuh)
-        go(k_tail_smem<T, R>, 1, kTailThreads, tsm, Vdev, t, nl, t == 0 ? r : nullptr, coarse_inv_.p, coarse_n_,
-           t == 0 && V[0].singular ? mean_out : nullptr);
-        ++launches_;
+    double* tail_mean = t == 0 && V[0].singular ? mean_out : nullptr;
+    if (dense_n_ > 0) {
+        // the tail as one dense product (tail_dense.cuh)
+        const int grid = (dense_n_ + kDenseRows - 1) / kDenseRows;
+        if (t == 0)
+            go(k_tail_dense<T, R>, grid, 32 * kDenseRows, 0, dense_n_, dense_ld_, (const double*)dense_M_.p, r,
+               V[0].x, tail_mean);
+        else
+            go(k_tail_dense<T, T>, grid, 32 * kDenseRows, 0, dense_n_, dense_ld_, (const double*)dense_M_.p,
+               (const T*)V[size_t(t)].b, V[size_t(t)].x, nullptr);
     } else {
-    const Launch gt{stream_, pdl_, tail_ctas_};
-    gt(k_tail<T, R>, tail_ctas_, kTailThreads, 0, Vdev, t, nl, t == 0 ? r : nullptr, coarse_inv_.p, coarse_n_,
-                                                         t == 0 && V[0].singular ? mean_out : nullptr);
-    ++launches_;
+        const Launch gt{stream_, pdl_, tail_ctas_};
+        gt(k_tail<T, R>, tail_ctas_, kTailThreads, 0, Vdev, t, nl, t == 0 ? r : nullptr, coarse_inv_.p, coarse_n_,
+           tail_mean);
     }
+    ++launches_;
     for (int l = t - 1; l >= 0; --l) {
         const LevelView<T>& L = V[size_t(l)];
         if (sdev_[size_t(l)].vec) {
