@@ -43,6 +43,14 @@ __device__ __forceinline__ void pdl_entry() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// The two halves of pdl_entry for a kernel that first loads what no kernel of
+// the cycle writes: the lists and operator values of its level, which only
+// set-up and refresh write, and the host waits for those before it launches a
+// cycle.  Such loads may run while the kernels before this one drain; anything a
+// kernel of the cycle writes is read after pdl_wait.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Pointers of one level in precision T, read by the fused kernels.
 template <typename T>
 struct LevelView {

@@ -482,14 +482,38 @@ __device__ __forceinline__ NextDir<T, P> next_dir(const T* xv, const double* mea
 template <typename T, typename P>
 __global__ void k_cg_dir_ap(LevelView<double> A, const T* __restrict__ xv, const double* mean, P* pa, P* pb,
                             P* __restrict__ ap, double* partial, unsigned* counter, CgState* s) {
-    pdl_entry();
+    pdl_launch();
+    // the first row's operator entries, which no kernel of the loop writes: up to
+    // kPre of them before the wait
+    constexpr int kPre = 8;
+    const int i0 = blockIdx.x * blockDim.x + threadIdx.x;
+    int b0 = 0, e0 = 0, c0[kPre];
+    double a0[kPre];
+    if (i0 < A.n) {
+        b0 = A.rp[i0];
+        e0 = A.rp[i0 + 1];
+    }
+#pragma unroll
+    for (int u = 0; u < kPre; ++u)
+        if (b0 + u < e0) {
+            c0[u] = A.ci[b0 + u];
+            a0[u] = A.val[b0 + u];
+        }
+    pdl_wait();
     if (s->flags & kCgHalt) return;  // the run ended at this body's r'z
     const NextDir<T, P> d = next_dir(xv, mean, pa, pb, s);
     P* __restrict__ pn = dir_new(pa, pb, s->iter);
     double v = 0;
     TPA_GRID_STRIDE(i, A.n) {
         double y = 0;
-        for (int k = A.rp[i]; k < A.rp[i + 1]; ++k) y += A.val[k] * d(A.ci[k]);
+        if (i == i0) {
+#pragma unroll
+            for (int u = 0; u < kPre; ++u)
+                if (b0 + u < e0) y += a0[u] * d(c0[u]);
+            for (int k = b0 + kPre; k < e0; ++k) y += A.val[k] * d(A.ci[k]);
+        } else {
+            for (int k = A.rp[i]; k < A.rp[i + 1]; ++k) y += A.val[k] * d(A.ci[k]);
+        }
         const double pi = d(i);
         pn[i] = P(pi);
         ap[i] = P(y);

@@ -176,7 +176,7 @@ template <typename T, typename TB>
 __global__ void __launch_bounds__(32 * kDenseRows)
     k_tail_dense(int n, int ld, const double* __restrict__ M, const TB* __restrict__ b, T* __restrict__ x,
                  double* mean_out) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    pdl_launch();
     constexpr int kChunk = 2048;
     __shared__ __align__(16) double sb[kChunk];
     const int lane = threadIdx.x & 31, row = blockIdx.x * kDenseRows + (threadIdx.x >> 5);
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(32 * kDenseRows)
         }
     };
     load(0);
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    pdl_wait();
     double acc[4] = {0, 0, 0, 0};
     for (int k0 = 0; k0 < n; k0 += 1024) {
         if (k0 % kChunk == 0) {

@@ -67,7 +67,9 @@ __host__ __device__ inline size_t tile_up_smem(int n3, int n2, int n1, int e) {
 
 // Loads in flight per thread in the prologues: a CTA's latency is that of its
 // dependent load chains, so every batch of independent loads is issued before
-// any of them is used.
+// any of them is used.  The lists, operator values, diagonals and volumes are
+// loaded before the programmatic-launch wait (pdl_wait), under the tail of the
+// kernel before; only the vectors the cycle writes are loaded after it.
 constexpr int kTileEntriesPerThread = 8;
 
 // the tile's local CSR into shared memory (coalesced copies, 8 entries in flight)
@@ -119,7 +121,7 @@ template <typename T, typename TB, int NT>
 __global__ void __launch_bounds__(NT)
     k_tile_down(LevelView<T> L, TileView<T> V, const TB* __restrict__ b, const double* level_sum,
                 T* __restrict__ bc, double* partial, unsigned* counter, double* coarse_sum) {
-    pdl_entry();
+    pdl_launch();
     extern __shared__ __align__(16) unsigned char tile_smem[];
     T* bp = reinterpret_cast<T*>(tile_smem);
     T* dv = bp + V.n3max;
@@ -141,19 +143,32 @@ __global__ void __launch_bounds__(NT)
         const int k = threadIdx.x + u * NT;
         g[u] = k < R.w ? cell[k] : -1;
     }
-    tile_stage_csr<T, NT>(V, t, R.z, val, lrp, lc);
-    const double mean = (L.singular && level_sum) ? *level_sum * L.cvol_inv : 0.0;
-    TB bb[CU];
     T vv[CU], dd[CU], tt[CU];
 #pragma unroll
     for (int u = 0; u < CU; ++u) {
         if (g[u] >= 0) {
-            bb[u] = b[g[u]];
             vv[u] = L.singular ? L.vol[g[u]] : T(0);
             dd[u] = L.dinv[g[u]];
             tt[u] = L.tinv[g[u]];
         }
     }
+    // the restriction's lists: one lane per child, four per coarse cell
+    const int c0 = V.co_off[t];
+    const int nco = V.co_off[t + 1] - c0;
+    const int J0 = threadIdx.x >> 2;
+    short4 ch0 = make_short4(-1, -1, -1, -1);
+    int co0 = 0;
+    if (J0 < nco) {
+        ch0 = V.ch[c0 + J0];
+        co0 = V.co[c0 + J0];
+    }
+    tile_stage_csr<T, NT>(V, t, R.z, val, lrp, lc);
+    pdl_wait();
+    const double mean = (L.singular && level_sum) ? *level_sum * L.cvol_inv : 0.0;
+    TB bb[CU];
+#pragma unroll
+    for (int u = 0; u < CU; ++u)
+        if (g[u] >= 0) bb[u] = b[g[u]];
 #pragma unroll
     for (int u = 0; u < CU; ++u) {
         const int k = threadIdx.x + u * NT;
@@ -179,28 +194,29 @@ __global__ void __launch_bounds__(NT)
         rr[k] = rk;
         ss[k] = ti[k] * rk;
     }
-    for (int k = threadIdx.x; k < R.x; k += blockDim.x) {
-        const int g = cell[k];
-        L.y[g] = xb[k];  // the pre-smoothed iterate, read by k_tile_up
-        L.bp[g] = bp[k];
+#pragma unroll
+    for (int u = 0; u < CU; ++u) {
+        const int k = threadIdx.x + u * NT;
+        if (k < R.x) {
+            L.y[g[u]] = xb[k];  // the pre-smoothed iterate, read by k_tile_up
+            L.bp[g[u]] = bp[k];
+        }
     }
     __syncthreads();
     // four lanes per coarse cell, lane q takes child q; whole warps (shuffles)
-    const int c0 = V.co_off[t];
-    const int nco = V.co_off[t + 1] - c0;
     const int quads = (4 * nco + 31) & ~31;
     double part = 0;
     for (int gq = threadIdx.x; gq < quads; gq += blockDim.x) {
         const int J = gq >> 2, q = gq & 3;
         T acc = T(0);
         if (J < nco) {
-            const int i = short4_at(V.ch[c0 + J], q);
+            const int i = short4_at(J == J0 ? ch0 : V.ch[c0 + J], q);
             if (i >= 0) acc = rr[i] - L.tw * tile_rowdot(val, lc, lrp, ss, i);
         }
         acc += __shfl_xor_sync(0xffffffffu, acc, 1);
         acc += __shfl_xor_sync(0xffffffffu, acc, 2);
         if (q == 0 && J < nco) {
-            bc[V.co[c0 + J]] = acc;
+            bc[J == J0 ? co0 : V.co[c0 + J]] = acc;
             part += double(acc);
         }
     }
@@ -221,7 +237,7 @@ template <typename T, typename Epi, int NT>
 __global__ void __launch_bounds__(NT)
     k_tile_up(LevelView<T> L, TileView<T> V, const T* __restrict__ xc, double* partial, unsigned* counter,
               double* mean_out, Epi epi) {
-    pdl_entry();
+    pdl_launch();
     extern __shared__ __align__(16) unsigned char tile_smem[];
     T* e = reinterpret_cast<T*>(tile_smem);
     T* xp = e + V.n3max;
@@ -244,19 +260,28 @@ __global__ void __launch_bounds__(NT)
         g[u] = k < R.w ? cell[k] : -1;
         o[u] = k < R.w ? own[k] : -1;
     }
+    T ee[CU], yy[CU], dd[CU], tt[CU], bb[CU], vv[CU];
+    double rv[CU];
+#pragma unroll
+    for (int u = 0; u < CU; ++u) {
+        const int k = threadIdx.x + u * NT;
+        if (k < R.z) {
+            dd[u] = L.dinv[g[u]];
+            tt[u] = L.tinv[g[u]];
+        }
+        if (mean_out && k < R.x) vv[u] = L.vol[g[u]];
+    }
     tile_stage_csr<T, NT>(V, t, R.z, val, lrp, lc);
-    T ee[CU], yy[CU], dd[CU], tt[CU], bb[CU];
+    pdl_wait();
 #pragma unroll
     for (int u = 0; u < CU; ++u) {
         const int k = threadIdx.x + u * NT;
         if (g[u] >= 0) {
             ee[u] = xc[o[u]];
-            if (k < R.z) {
-                yy[u] = L.y[g[u]];
-                dd[u] = L.dinv[g[u]];
-                tt[u] = L.tinv[g[u]];
-            }
+            if (k < R.z) yy[u] = L.y[g[u]];
             if (k < R.y) bb[u] = L.bp[g[u]];
+            if constexpr (Epi::kRz)
+                if (mean_out && k < R.x) rv[u] = epi.r[g[u]];
         }
     }
 #pragma unroll
@@ -282,13 +307,15 @@ __global__ void __launch_bounds__(NT)
         xq[k] = xp[k] + L.w * dv[k] * (bp[k] - tile_rowdot(val, lc, lrp, xp, k));
     __syncthreads();
     double v = 0, w = 0;
-    for (int k = threadIdx.x; k < R.x; k += blockDim.x) {
+#pragma unroll
+    for (int u = 0; u < CU; ++u) {
+        const int k = threadIdx.x + u * NT;
+        if (k >= R.x) break;
         const T out = xq[k] + L.w * dv[k] * (bp[k] - tile_rowdot(val, lc, lrp, xq, k));
-        const int g = cell[k];
-        L.x[g] = out;
+        L.x[g[u]] = out;
         if (mean_out) {
-            v += double(L.vol[g]) * double(out);
-            if constexpr (Epi::kRz) w += epi.r[g] * double(out);
+            v += double(vv[u]) * double(out);
+            if constexpr (Epi::kRz) w += rv[u] * double(out);
         }
     }
     if (mean_out) fold_mean(v, w, partial, counter, mean_out, L.cvol_inv, epi);
