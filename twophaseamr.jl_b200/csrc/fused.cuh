@@ -8,12 +8,18 @@
 //                   neighbours on the fly; the RHS projection of the level
 //                   (`_multigrid_project_component_rhs!`) is applied inline
 //   k_residual, k_restrict  r = b - A x, s = Dt^-1 r, then b_c = P_tent.(r - wt A s)
-//                   with the coarse RHS sum folded in the same launch
 //   k_prolong       x += e - wt Dt^-1 A e with e = P_tent x_c, in place (it
 //                   reads no neighbouring fine value)
 //   k_tail          every level with at most kTailCells cells in one CTA: the
 //                   red-black tails and those above kDenseTailCells cells (the
 //                   others are one dense product, tail_dense.cuh)
+// Only the finest level and the tail project their right-hand side (and the
+// tail's map removes the mean of whatever reaches it).  The reference projects
+// every level's (cycles.jl:46-77), but a restricted right-hand side has zero sum
+// already: P_tent' keeps sums, 1'A = 0 on a closed component, so sum b_c =
+// sum(r - wt A s) = sum(bp - A x) = sum bp = 0, up to the rounding that the sums
+// themselves carry.  Folding that sum in each restriction cost a fence, an
+// atomic and a one-CTA fold, about 2 us per level and V-cycle.
 // Reductions fold their per-block partials in the last block to finish (a
 // fixed-order fold: results do not depend on block scheduling).
 #pragma once
@@ -399,29 +405,17 @@ __global__ void k_residual(LevelView<T> L) {
     if (i < L.n) residual_cell(L, i);
 }
 
-// b_c = P_tent'(r - wt A s), four threads per coarse cell (grid over 4 nc);
-// coarse RHS sum folded into `coarse_sum` when non-null.
+// b_c = P_tent'(r - wt A s), four threads per coarse cell (grid over 4 nc)
 template <typename T>
-__global__ void k_restrict(LevelView<T> L, T* __restrict__ bc, double* partial, unsigned* counter, double* coarse_sum) {
+__global__ void k_restrict(LevelView<T> L, T* __restrict__ bc) {
     pdl_entry();
     // grid-stride over whole warps (the shuffles need every lane of a warp)
     const int quads = (4 * L.nc + 31) & ~31;
-    double part = 0;
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < quads; g += gridDim.x * blockDim.x) {
         const int J = g >> 2;
         const T v = restrict_quad(L, J, g & 3);
         if ((g & 3) == 0 && J < L.nc) {
             bc[J] = v;
-            part += double(v);
-        }
-    }
-    if (coarse_sum) {
-        if (publish_partial(part, partial, counter)) {
-            double s = fold_partials(partial, gridDim.x);
-            if (threadIdx.x == 0) {
-                *coarse_sum = s;
-                *counter = 0;
-            }
         }
     }
 }
@@ -431,11 +425,9 @@ __global__ void k_restrict(LevelView<T> L, T* __restrict__ bc, double* partial, 
 // cell, as k_restrict).  Saves the residual phase and the r / s round trip at
 // the price of about nnz_row^2 products per fine cell.
 template <typename T>
-__global__ void k_resrest(LevelView<T> L, T* __restrict__ bc, double* partial, unsigned* counter,
-                          double* coarse_sum) {
+__global__ void k_resrest(LevelView<T> L, T* __restrict__ bc) {
     pdl_entry();
     const int quads = (4 * L.nc + 31) & ~31;
-    double part = 0;
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < quads; g += gridDim.x * blockDim.x) {
         const int J = g >> 2, q = g & 3;
         T acc = T(0);
@@ -455,16 +447,6 @@ __global__ void k_resrest(LevelView<T> L, T* __restrict__ bc, double* partial, u
         acc += __shfl_xor_sync(0xffffffffu, acc, 2);
         if (q == 0 && J < L.nc) {
             bc[J] = acc;
-            part += double(acc);
-        }
-    }
-    if (coarse_sum) {
-        if (publish_partial(part, partial, counter)) {
-            double s = fold_partials(partial, gridDim.x);
-            if (threadIdx.x == 0) {
-                *coarse_sum = s;
-                *counter = 0;
-            }
         }
     }
 }

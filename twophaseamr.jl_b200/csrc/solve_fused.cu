@@ -72,7 +72,7 @@ struct CgState {
 // update of that body do nothing
 constexpr int kCgHalt = 2 | 4 | 8;
 
-enum Counter { kRestrictSum = 0, kPostMean = 1, kCgAp = 2, kCgUpdate = 3, kCgZ = 4, kCgRes = 5, kRsum = 6 };
+enum Counter { kPostMean = 1, kCgAp = 2, kCgUpdate = 3, kCgZ = 4, kCgRes = 5, kRsum = 6 };
 
 inline int blocks_for(int64_t n) {
     int64_t g = (n + kThreads - 1) / kThreads;
@@ -907,12 +907,12 @@ void DeviceSolver::enqueue_vcycle_epi(const R* r, const double* rsum, double* me
     const std::vector<SView<T>>* Sp;
     if constexpr (std::is_same<T, double>::value) Sp = &sd_;
     else Sp = &sf_;
+    const double* no_sum = nullptr;  // below the finest level the right-hand sides have zero sum (fused.cuh)
     for (int l = 0; l < t; ++l) {
         const LevelView<T>& L = V[size_t(l)];
         if (sdev_[size_t(l)].vec) {
             const SView<T>& S = (*Sp)[size_t(l)];
             const int groups = (S.nblocks + 3) / 4;
-            const bool next_sum = (l + 1 < t) && V[size_t(l + 1)].singular;
             if (tdev_.size() > size_t(l) && tdev_[size_t(l)].stream) {
                 // both pre-sweeps, the residual and the restriction, streamed by rows
                 constexpr bool fp32 = std::is_same<T, float>::value;
@@ -921,12 +921,10 @@ void DeviceSolver::enqueue_vcycle_epi(const R* r, const double* rsum, double* me
                 with_stream_rows(g.rows, [&](auto rows) {
                     constexpr int RW = decltype(rows)::value;
                     if (l == 0)
-                        go(v_stream_down<T, R, RW>, grid, kStreamWarps * 32, 0, S, g, r, rsum, V[size_t(l + 1)].b,
-                           fpartial_.p, counters_.p + kRestrictSum, next_sum ? lsum_.p + l + 1 : nullptr);
+                        go(v_stream_down<T, R, RW>, grid, kStreamWarps * 32, 0, S, g, r, rsum, V[size_t(l + 1)].b, S.bp);
                     else
-                        go(v_stream_down<T, T, RW>, grid, kStreamWarps * 32, 0, S, g, (const T*)S.b,
-                           (const double*)(lsum_.p + l), V[size_t(l + 1)].b, fpartial_.p,
-                           counters_.p + kRestrictSum, next_sum ? lsum_.p + l + 1 : nullptr);
+                        go(v_stream_down<T, T, RW>, grid, kStreamWarps * 32, 0, S, g, (const T*)S.b, no_sum,
+                           V[size_t(l + 1)].b, (T*)nullptr);
                 });
                 ++launches_;
                 continue;
@@ -934,37 +932,29 @@ void DeviceSolver::enqueue_vcycle_epi(const R* r, const double* rsum, double* me
             if (tdev_.size() > size_t(l) && tdev_[size_t(l)].vec) {
                 // both pre-sweeps, the residual and the restriction on 22 x 22 tiles
                 if (l == 0)
-                    go(v_tile_down<T, R>, S.nblocks, kTileThreads, 0, S, r, rsum, V[size_t(l + 1)].b, fpartial_.p,
-                       counters_.p + kRestrictSum, next_sum ? lsum_.p + l + 1 : nullptr);
+                    go(v_tile_down<T, R>, S.nblocks, kTileThreads, 0, S, r, rsum, V[size_t(l + 1)].b, S.bp);
                 else
-                    go(v_tile_down<T, T>, S.nblocks, kTileThreads, 0, S, (const T*)S.b,
-                       (const double*)(lsum_.p + l), V[size_t(l + 1)].b, fpartial_.p, counters_.p + kRestrictSum,
-                       next_sum ? lsum_.p + l + 1 : nullptr);
+                    go(v_tile_down<T, T>, S.nblocks, kTileThreads, 0, S, (const T*)S.b, no_sum, V[size_t(l + 1)].b,
+                       (T*)nullptr);
                 ++launches_;
                 continue;
             }
             if (l == 0) go(v_pre2<T, R>, groups, 256, 0, S, r, rsum);
-            else go(v_pre2<T, T>, groups, 256, 0, S, S.b, lsum_.p + l);
+            else go(v_pre2<T, T>, groups, 256, 0, S, S.b, no_sum);
             go(v_residual<T>, groups, 256, 0, S);
-            go(v_restrict<T>, next_sum ? fold_grid(v_restrict<T>, 256, groups, kMaxGrid) : groups, 256, 0, S,
-               V[size_t(l + 1)].b,
-               fpartial_.p, counters_.p + kRestrictSum, next_sum ? lsum_.p + l + 1 : nullptr);
+            go(v_restrict<T>, groups, 256, 0, S, V[size_t(l + 1)].b);
             launches_ += 3;
             continue;
         }
         if (sdev_[size_t(l)].on) {
             const SView<T>& S = (*Sp)[size_t(l)];
             const int g = S.nblocks, th = S.cpb;
-            const bool next_sum = (l + 1 < t) && V[size_t(l + 1)].singular;
             with_nxc(S, [&](auto nxc) {
                 constexpr int N = decltype(nxc)::value;
                 if (l == 0) go(s_pre2<T, R, N>, g, th, 0, S, r, rsum);
-                else go(s_pre2<T, T, N>, g, th, 0, S, S.b, lsum_.p + l);
+                else go(s_pre2<T, T, N>, g, th, 0, S, S.b, no_sum);
                 go(s_residual<T, N>, g, th, 0, S);
-                go(s_restrict<T, N>, next_sum ? fold_grid(s_restrict<T, N>, th, g, kMaxGrid, th * sizeof(T)) : g,
-                   th, th * sizeof(T),
-                    S, V[size_t(l + 1)].b, fpartial_.p, counters_.p + kRestrictSum,
-                    next_sum ? lsum_.p + l + 1 : nullptr);
+                go(s_restrict<T, N>, g, th, th * sizeof(T), S, V[size_t(l + 1)].b);
             });
             launches_ += 3;
             continue;
@@ -973,17 +963,14 @@ void DeviceSolver::enqueue_vcycle_epi(const R* r, const double* rsum, double* me
             // both pre-sweeps, the residual and the restriction in one launch
             const TileDev& D = tdev_[size_t(l)];
             const TileView<T>& TV = tile_view<T>(l);
-            const bool next_sum = (l + 1 < t) && V[size_t(l + 1)].singular;
             const size_t sm = tile_down_smem<T>(D.n3max, D.n2max, D.n1max, D.emax);
             with_tile_threads(D.nt, [&](auto nt) {
                 constexpr int NT = decltype(nt)::value;
                 if (l == 0)
-                    go(k_tile_down<T, R, NT>, D.ntiles, NT, sm, L, TV, r, rsum, V[size_t(l + 1)].b, fpartial_.p,
-                       counters_.p + kRestrictSum, next_sum ? lsum_.p + l + 1 : nullptr);
+                    go(k_tile_down<T, R, NT>, D.ntiles, NT, sm, L, TV, r, rsum, V[size_t(l + 1)].b, L.bp);
                 else
-                    go(k_tile_down<T, T, NT>, D.ntiles, NT, sm, L, TV, (const T*)L.b, (const double*)(lsum_.p + l),
-                       V[size_t(l + 1)].b, fpartial_.p, counters_.p + kRestrictSum,
-                       next_sum ? lsum_.p + l + 1 : nullptr);
+                    go(k_tile_down<T, T, NT>, D.ntiles, NT, sm, L, TV, (const T*)L.b, no_sum, V[size_t(l + 1)].b,
+                       (T*)nullptr);
             });
             ++launches_;
             continue;
@@ -994,7 +981,7 @@ void DeviceSolver::enqueue_vcycle_epi(const R* r, const double* rsum, double* me
             const bool pair = L.n <= rb_pair_cells_;
             T* first = pair ? L.y : L.x;
             if (l == 0) go(k_rb_pre<T, R>, blocks_for(L.n), kThreads, 0, L, r, rsum, first);
-            else go(k_rb_pre<T, T>, blocks_for(L.n), kThreads, 0, L, L.b, lsum_.p + l, first);
+            else go(k_rb_pre<T, T>, blocks_for(L.n), kThreads, 0, L, L.b, no_sum, first);
             if (pair) {
                 go(k_rb_pair<T>, blocks_for(L.n), kThreads, 0, L, (const T*)L.y, L.x, 0, nullptr, nullptr, nullptr);
                 ++launches_;
@@ -1006,22 +993,16 @@ void DeviceSolver::enqueue_vcycle_epi(const R* r, const double* rsum, double* me
         } else if (l == 0) {
             go(k_pre2<T, R>, blocks_for(L.n), kThreads, 0, L, r, rsum);
         } else {
-            go(k_pre2<T, T>, blocks_for(L.n), kThreads, 0, L, L.b, lsum_.p + l);
+            go(k_pre2<T, T>, blocks_for(L.n), kThreads, 0, L, L.b, no_sum);
         }
-        const bool next_sum = (l + 1 < t) && V[size_t(l + 1)].singular;
-        const int64_t quads = blocks_for(4 * int64_t(L.nc));
-        const int rgrid = !next_sum ? int(quads)
-                          : L.n <= rr_cells_ ? fold_grid(k_resrest<T>, kThreads, quads, kMaxGrid)
-                                     : fold_grid(k_restrict<T>, kThreads, quads, kMaxGrid);
+        const int rgrid = blocks_for(4 * int64_t(L.nc));
         if (L.n <= rr_cells_) {
-            go(k_resrest<T>, rgrid, kThreads, 0, L, V[size_t(l + 1)].b, fpartial_.p, counters_.p + kRestrictSum,
-               next_sum ? lsum_.p + l + 1 : nullptr);
+            go(k_resrest<T>, rgrid, kThreads, 0, L, V[size_t(l + 1)].b);
             launches_ += 2;
             continue;
         }
         go(k_residual<T>, blocks_for(L.n), kThreads, 0, L);
-        go(k_restrict<T>, rgrid, kThreads, 0, L, V[size_t(l + 1)].b, fpartial_.p, counters_.p + kRestrictSum,
-           next_sum ? lsum_.p + l + 1 : nullptr);
+        go(k_restrict<T>, rgrid, kThreads, 0, L, V[size_t(l + 1)].b);
         launches_ += 3;
     }
     double* tail_mean = t == 0 && V[0].singular ? mean_out : nullptr;
@@ -1054,14 +1035,15 @@ void DeviceSolver::enqueue_vcycle_epi(const R* r, const double* rsum, double* me
                 with_stream_rows(g.rows, [&](auto rows) {
                     constexpr int RW = decltype(rows)::value;
                     go(v_stream_up<T, Epi, RW>, grid, kStreamWarps * 32, 0, S, g, (const T*)V[size_t(l + 1)].x,
-                       fpartial_.p, counters_.p + kPostMean, want_mean ? mean_out : nullptr, epi);
+                       (const T*)(l == 0 ? S.bp : S.b), fpartial_.p, counters_.p + kPostMean, want_mean ? mean_out : nullptr, epi);
                 });
                 ++launches_;
                 continue;
             }
             if (tdev_.size() > size_t(l) && tdev_[size_t(l)].vec) {
                 // prolongation and both post-sweeps on 22 x 22 tiles
-                go(v_tile_up<T, Epi>, S.nblocks, kTileThreads, 0, S, (const T*)V[size_t(l + 1)].x, fpartial_.p,
+                go(v_tile_up<T, Epi>, S.nblocks, kTileThreads, 0, S, (const T*)V[size_t(l + 1)].x,
+                   (const T*)(l == 0 ? S.bp : S.b), fpartial_.p,
                    counters_.p + kPostMean, want_mean ? mean_out : nullptr, epi);
                 ++launches_;
                 continue;
@@ -1097,7 +1079,7 @@ void DeviceSolver::enqueue_vcycle_epi(const R* r, const double* rsum, double* me
             with_tile_threads(D.nt, [&](auto nt) {
                 constexpr int NT = decltype(nt)::value;
                 go(k_tile_up<T, Epi, NT>, D.ntiles, NT, tile_up_smem<T>(D.n3max, D.n2max, D.n1max, D.emax), L,
-                   tile_view<T>(l), (const T*)V[size_t(l + 1)].x, fpartial_.p, counters_.p + kPostMean,
+                   tile_view<T>(l), (const T*)V[size_t(l + 1)].x, (const T*)(l == 0 ? L.bp : L.b), fpartial_.p, counters_.p + kPostMean,
                    want_mean ? mean_out : nullptr, epi);
             });
             ++launches_;
@@ -1342,9 +1324,7 @@ double DeviceSolver::time_fused(int which, int level, int precision, int iters) 
         switch (which) {
             case 0: k_post2<T><<<blocks_for(L.n), kThreads, 0, stream_>>>(L, fpartial_.p, counters_.p, nullptr); break;
             case 1:
-                k_restrict<T><<<blocks_for(4 * int64_t(L.nc)), kThreads, 0, stream_>>>(L, V[size_t(level + 1)].b,
-                                                                                        fpartial_.p, counters_.p,
-                                                                                        nullptr);
+                k_restrict<T><<<blocks_for(4 * int64_t(L.nc)), kThreads, 0, stream_>>>(L, V[size_t(level + 1)].b);
                 break;
             case 2: k_prolong<T><<<blocks_for(L.n), kThreads, 0, stream_>>>(L, V[size_t(level + 1)].x); break;
             case 4: k_pre2<T, T><<<blocks_for(L.n), kThreads, 0, stream_>>>(L, L.b, nullptr); break;
@@ -1362,7 +1342,7 @@ double DeviceSolver::time_fused(int which, int level, int precision, int iters) 
             const int groups = (L.nblocks + 3) / 4;
             switch (which) {
                 case 0: v_sweep<T, false><<<groups, 256, 0, stream_>>>(L, L.y, L.x, nullptr, nullptr, nullptr); break;
-                case 1: v_restrict<T><<<groups, 256, 0, stream_>>>(L, bc, fpartial_.p, counters_.p, nullptr); break;
+                case 1: v_restrict<T><<<groups, 256, 0, stream_>>>(L, bc); break;
                 case 2: v_prolong<T><<<groups, 256, 0, stream_>>>(L, xc); break;
                 case 4: v_pre2<T, T><<<groups, 256, 0, stream_>>>(L, L.b, nullptr); break;
                 case 5: v_residual<T><<<groups, 256, 0, stream_>>>(L); break;
@@ -1374,7 +1354,7 @@ double DeviceSolver::time_fused(int which, int level, int precision, int iters) 
             constexpr int N = decltype(nxc)::value;
             switch (which) {
                 case 0: s_post2<T, N><<<g, th, 0, stream_>>>(L, fpartial_.p, counters_.p, nullptr); break;
-                case 1: s_restrict<T, N><<<g, th, th * sizeof(T), stream_>>>(L, bc, fpartial_.p, counters_.p, nullptr); break;
+                case 1: s_restrict<T, N><<<g, th, th * sizeof(T), stream_>>>(L, bc); break;
                 case 2: s_prolong<T, N><<<g, th, 0, stream_>>>(L, xc); break;
                 case 4: s_pre2<T, T, N><<<g, th, 0, stream_>>>(L, L.b, nullptr); break;
                 case 5: s_residual<T, N><<<g, th, 0, stream_>>>(L); break;
@@ -1393,14 +1373,14 @@ double DeviceSolver::time_fused(int which, int level, int precision, int iters) 
             const size_t sm = tile_down_smem<T>(D.n3max, D.n2max, D.n1max, D.emax);
             if (which == 6 && level == 0)  // the finest level reads the FP64 residual, as in the cycle
                 k_tile_down<T, double, NT><<<D.ntiles, NT, sm, stream_>>>(
-                    L, TV, (const double*)r_.p, nullptr, V[size_t(level + 1)].b, fpartial_.p, counters_.p, nullptr);
+                    L, TV, (const double*)r_.p, nullptr, V[size_t(level + 1)].b, L.bp);
             else if (which == 6)
                 k_tile_down<T, T, NT><<<D.ntiles, NT, sm, stream_>>>(L, TV, (const T*)L.b, nullptr,
-                                                                     V[size_t(level + 1)].b, fpartial_.p,
-                                                                     counters_.p, nullptr);
+                                                                     V[size_t(level + 1)].b, (T*)nullptr);
             else
                 k_tile_up<T, MeanOnly, NT><<<D.ntiles, NT, tile_up_smem<T>(D.n3max, D.n2max, D.n1max, D.emax),
-                                            stream_>>>(L, TV, (const T*)V[size_t(level + 1)].x, fpartial_.p,
+                                            stream_>>>(L, TV, (const T*)V[size_t(level + 1)].x,
+                                                       (const T*)(level == 0 ? L.bp : L.b), fpartial_.p,
                                                        counters_.p, nullptr, MeanOnly());
         });
     };
@@ -1415,13 +1395,14 @@ double DeviceSolver::time_fused(int which, int level, int precision, int iters) 
             constexpr int RW = decltype(rows)::value;
             if (which == 8 && level == 0)  // the finest level reads the FP64 residual, as in the cycle
                 v_stream_down<T, double, RW><<<grid, kStreamWarps * 32, 0, stream_>>>(
-                    L, g, (const double*)r_.p, nullptr, V[size_t(level + 1)].b, fpartial_.p, counters_.p, nullptr);
+                    L, g, (const double*)r_.p, nullptr, V[size_t(level + 1)].b, L.bp);
             else if (which == 8)
                 v_stream_down<T, T, RW><<<grid, kStreamWarps * 32, 0, stream_>>>(
-                    L, g, (const T*)L.b, nullptr, V[size_t(level + 1)].b, fpartial_.p, counters_.p, nullptr);
+                    L, g, (const T*)L.b, nullptr, V[size_t(level + 1)].b, (T*)nullptr);
             else
                 v_stream_up<T, MeanOnly, RW><<<grid, kStreamWarps * 32, 0, stream_>>>(
-                    L, g, (const T*)V[size_t(level + 1)].x, fpartial_.p, counters_.p, nullptr, MeanOnly());
+                    L, g, (const T*)V[size_t(level + 1)].x, (const T*)(level == 0 ? L.bp : L.b), fpartial_.p, counters_.p,
+                    nullptr, MeanOnly());
         });
     };
     auto launch = [&]() {

@@ -145,16 +145,14 @@ __global__ void s_residual(SView<T> L) {
 }
 
 // t = r - wt A s per fine cell, aggregated over the 2x2 (or 1x1) children into
-// the coarse block quadrant; optional fold of the coarse RHS sum.  Strides over
-// blocks so that the fold reads at most gridDim.x partials.
+// the coarse block quadrant.
 template <typename T, int NXC>
-__global__ void s_restrict(SView<T> L, T* __restrict__ bc, double* partial, unsigned* counter, double* coarse_sum) {
+__global__ void s_restrict(SView<T> L, T* __restrict__ bc) {
     pdl_entry();
     extern __shared__ unsigned char smem_raw[];
     T* tile = reinterpret_cast<T*>(smem_raw);
     const T* sv = L.s;
     const int nx = Blk<NXC>::nx(L), ny = Blk<NXC>::ny(L), cpb = Blk<NXC>::cpb(L);
-    double part = 0;
     for (int b = blockIdx.x; b < L.nblocks; b += gridDim.x) {
         TPA_S_CELL(b);
         __syncthreads();
@@ -165,21 +163,10 @@ __global__ void s_restrict(SView<T> L, T* __restrict__ bc, double* partial, unsi
         if (sc == 1) {
             T v = tile[t];
             bc[cb * cpb + t] = v;
-            part += double(v);
         } else if (i < nx / 2 && j < ny / 2) {
             const int f = 2 * j * nx + 2 * i;
             T v = tile[f] + tile[f + 1] + tile[f + nx] + tile[f + nx + 1];
             bc[cb * cpb + (oy + j) * nx + (ox + i)] = v;
-            part += double(v);
-        }
-    }
-    if (coarse_sum) {
-        if (publish_partial(part, partial, counter)) {
-            double s = fold_partials(partial, gridDim.x);
-            if (threadIdx.x == 0) {
-                *coarse_sum = s;
-                *counter = 0;
-            }
         }
     }
 }

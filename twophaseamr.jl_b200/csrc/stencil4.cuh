@@ -245,13 +245,11 @@ __global__ void __launch_bounds__(256) v_residual(SView<T> L) {
 }
 
 // b_c = P_tent'(r - wt A s): 2x2 (scale 2) or 1x1 (scale 1) aggregation into the
-// coarse block's quadrant; optional fold of the coarse RHS sum
+// coarse block's quadrant
 template <typename T>
-__global__ void __launch_bounds__(256) v_restrict(SView<T> L, T* __restrict__ bc, double* partial, unsigned* counter,
-                                                  double* coarse_sum) {
+__global__ void __launch_bounds__(256) v_restrict(SView<T> L, T* __restrict__ bc) {
     pdl_entry();
     const int groups = (L.nblocks + 3) / 4;
-    double part = 0;
     TPA_Q_LOOP(groups) {
         const QPos p = q_pos(grp);
         const bool valid = p.b < L.nblocks;
@@ -274,23 +272,12 @@ __global__ void __launch_bounds__(256) v_restrict(SView<T> L, T* __restrict__ bc
             T* dst = bc + mp.x * 256 + (mp.z + p.j) * 16 + mp.y + 4 * p.q;
             for (int m = 0; m < 4; ++m) {
                 dst[m] = t.v[m];
-                part += double(t.v[m]);
             }
         } else if ((p.j & 1) == 0) {
             const T c0 = h0 + d0, c1 = h1 + d1;
             T* dst = bc + mp.x * 256 + (mp.z + (p.j >> 1)) * 16 + mp.y + 2 * p.q;
             dst[0] = c0;
             dst[1] = c1;
-            part += double(c0) + double(c1);
-        }
-    }
-    if (coarse_sum) {
-        if (publish_partial(part, partial, counter)) {
-            const double s = fold_partials(partial, gridDim.x);
-            if (threadIdx.x == 0) {
-                *coarse_sum = s;
-                *counter = 0;
-            }
         }
     }
 }

@@ -100,15 +100,15 @@ __device__ __forceinline__ P2<T> st_apply(const SView<T>& L, const P2<T>& s, con
 }
 
 // Both pre-sweeps from x = 0 with the level's RHS projection, the residual, and
-// the restriction b_c = P_tent'(r - wt A D^-1 r) with the optional coarse RHS sum.
-// The pre-smoothed iterate goes to L.y and the projected RHS to L.bp (read by
-// v_stream_up); the residual stays in registers.  The warps of the grid take the
-// strips in turn (the last strip across or up the level may be cut short: its
+// the restriction b_c = P_tent'(r - wt A D^-1 r).
+// The pre-smoothed iterate goes to L.y and the projected RHS to bp_out (null: not
+// written; v_stream_up then reads the level's own right-hand side); the residual
+// stays in registers.  The warps of the grid take the strips in turn (the last strip across or up the level may be cut short: its
 // cells past the edge are walked but not written).
 template <typename T, typename TB, int ROWS>
 __global__ void __launch_bounds__(kStreamWarps * 32, stream_ctas_per_sm<T>())
     v_stream_down(SView<T> L, StreamGeom g, const TB* __restrict__ bin, const double* level_sum,
-                  T* __restrict__ bc, double* partial, unsigned* counter, double* coarse_sum) {
+                  T* __restrict__ bc, T* bp_out) {
     pdl_entry();
     constexpr int S = ROWS + 6, D = kStreamDepth;
     __shared__ P2<TB> stage[kStreamWarps][D][32];
@@ -118,7 +118,6 @@ __global__ void __launch_bounds__(kStreamWarps * 32, stream_ctas_per_sm<T>())
     const double vol0 = double(L.vol0);
     const T wd = L.w * L.dinv0;
     auto proj = [&](TB a) { return mean != 0.0 ? T(double(a) - vol0 * mean) : T(a); };
-    double part = 0;
     for (int strip = blockIdx.x * kStreamWarps + wid; strip < g.nsx * g.nsy; strip += gridDim.x * kStreamWarps) {
         const int x0 = (strip % g.nsx) * kStreamCols, y0 = (strip / g.nsx) * ROWS;
         const int gx0 = x0 - 4 + 2 * lane;
@@ -147,7 +146,7 @@ __global__ void __launch_bounds__(kStreamWarps * 32, stream_ctas_per_sm<T>())
                 if (j >= 3 && j < 3 + ROWS && out_col && in_row(j)) {
                     const int c = cell(j);
                     *reinterpret_cast<P2<T>*>(L.y + c) = x2[j];
-                    *reinterpret_cast<P2<T>*>(L.bp + c) = bp[j];
+                    if (bp_out) *reinterpret_cast<P2<T>*>(bp_out + c) = bp[j];
                 }
             }
             if (k >= 4) {  // rows 2 .. S - 3: their x2 neighbours exist
@@ -167,17 +166,7 @@ __global__ void __launch_bounds__(kStreamWarps * 32, stream_ctas_per_sm<T>())
                     const T d0 = t[j].l + t[j].r;
                     const T v = h0 + d0;
                     bc[st_coarse(g, gx, y0 + j - 4)] = v;
-                    part += double(v);
                 }
-            }
-        }
-    }
-    if (coarse_sum) {
-        if (publish_partial(part, partial, counter)) {
-            const double sum = fold_partials(partial, gridDim.x);
-            if (threadIdx.x == 0) {
-                *coarse_sum = sum;
-                *counter = 0;
             }
         }
     }
@@ -189,8 +178,8 @@ __global__ void __launch_bounds__(kStreamWarps * 32, stream_ctas_per_sm<T>())
 // of L.x (and the epilogue's sums) folded.
 template <typename T, typename Epi, int ROWS>
 __global__ void __launch_bounds__(kStreamWarps * 32, stream_ctas_per_sm<T>())
-    v_stream_up(SView<T> L, StreamGeom g, const T* __restrict__ xc, double* partial, unsigned* counter,
-                double* mean_out, Epi epi) {
+    v_stream_up(SView<T> L, StreamGeom g, const T* __restrict__ xc, const T* __restrict__ bp_in, double* partial,
+                unsigned* counter, double* mean_out, Epi epi) {
     pdl_entry();
     constexpr int S = ROWS + 6, D = kStreamDepth;
     __shared__ T se[kStreamWarps][D][32];
@@ -209,7 +198,7 @@ __global__ void __launch_bounds__(kStreamWarps * 32, stream_ctas_per_sm<T>())
             const int c = st_cell(g, gx, gy);
             st_cp_async<sizeof(T)>(&se[wid][k % D][lane], xc + st_coarse(g, gx, gy));
             st_cp_async<sizeof(P2<T>)>(&sy[wid][k % D][lane], L.y + c);
-            st_cp_async<sizeof(P2<T>)>(&sb[wid][k % D][lane], L.bp + c);
+            st_cp_async<sizeof(P2<T>)>(&sb[wid][k % D][lane], bp_in + c);
         };
 #pragma unroll
         for (int k = 0; k < D - 1; ++k) {

@@ -115,12 +115,13 @@ __device__ __forceinline__ int short4_at(short4 v, int q) {
 }
 
 // b: this level's raw right-hand side (the FP64 residual on the finest level);
-// level_sum: its sum (projection, may be null); bc: the coarse right-hand side;
-// coarse_sum (may be null): receives the sum of bc, folded by the last CTA.
+// level_sum: its sum (projection; null below the finest level); bc: the coarse
+// right-hand side; bp_out (null: not written, the cycle reads b itself): the
+// projected right-hand side for k_tile_up.
 template <typename T, typename TB, int NT>
 __global__ void __launch_bounds__(NT)
     k_tile_down(LevelView<T> L, TileView<T> V, const TB* __restrict__ b, const double* level_sum,
-                T* __restrict__ bc, double* partial, unsigned* counter, double* coarse_sum) {
+                T* __restrict__ bc, T* bp_out) {
     pdl_launch();
     extern __shared__ __align__(16) unsigned char tile_smem[];
     T* bp = reinterpret_cast<T*>(tile_smem);
@@ -143,11 +144,12 @@ __global__ void __launch_bounds__(NT)
         const int k = threadIdx.x + u * NT;
         g[u] = k < R.w ? cell[k] : -1;
     }
+    const bool project = L.singular && level_sum;
     T vv[CU], dd[CU], tt[CU];
 #pragma unroll
     for (int u = 0; u < CU; ++u) {
         if (g[u] >= 0) {
-            vv[u] = L.singular ? L.vol[g[u]] : T(0);
+            vv[u] = project ? L.vol[g[u]] : T(0);
             dd[u] = L.dinv[g[u]];
             tt[u] = L.tinv[g[u]];
         }
@@ -164,7 +166,7 @@ __global__ void __launch_bounds__(NT)
     }
     tile_stage_csr<T, NT>(V, t, R.z, val, lrp, lc);
     pdl_wait();
-    const double mean = (L.singular && level_sum) ? *level_sum * L.cvol_inv : 0.0;
+    const double mean = project ? *level_sum * L.cvol_inv : 0.0;
     TB bb[CU];
 #pragma unroll
     for (int u = 0; u < CU; ++u)
@@ -175,7 +177,7 @@ __global__ void __launch_bounds__(NT)
         if (g[u] >= 0) {
             // the projected RHS as proj_b forms it
             double v = double(bb[u]);
-            if (L.singular) v -= double(vv[u]) * mean;
+            if (project) v -= double(vv[u]) * mean;
             const T bk = T(v);
             bp[k] = bk;
             dv[k] = dd[u];
@@ -199,13 +201,12 @@ __global__ void __launch_bounds__(NT)
         const int k = threadIdx.x + u * NT;
         if (k < R.x) {
             L.y[g[u]] = xb[k];  // the pre-smoothed iterate, read by k_tile_up
-            L.bp[g[u]] = bp[k];
+            if (bp_out) bp_out[g[u]] = bp[k];
         }
     }
     __syncthreads();
     // four lanes per coarse cell, lane q takes child q; whole warps (shuffles)
     const int quads = (4 * nco + 31) & ~31;
-    double part = 0;
     for (int gq = threadIdx.x; gq < quads; gq += blockDim.x) {
         const int J = gq >> 2, q = gq & 3;
         T acc = T(0);
@@ -217,25 +218,16 @@ __global__ void __launch_bounds__(NT)
         acc += __shfl_xor_sync(0xffffffffu, acc, 2);
         if (q == 0 && J < nco) {
             bc[J == J0 ? co0 : V.co[c0 + J]] = acc;
-            part += double(acc);
-        }
-    }
-    if (coarse_sum) {
-        if (publish_partial(part, partial, counter)) {
-            const double s = fold_partials(partial, gridDim.x);
-            if (threadIdx.x == 0) {
-                *coarse_sum = s;
-                *counter = 0;
-            }
         }
     }
 }
 
-// xc: the coarse level's correction; mean_out (may be null): the volume mean
-// of the result, folded by the last CTA, which then runs `epi`.
+// xc: the coarse level's correction; bp_in: the projected right-hand side (the
+// level's own below the finest); mean_out (may be null): the volume mean of the
+// result, folded by the last CTA, which then runs `epi`.
 template <typename T, typename Epi, int NT>
 __global__ void __launch_bounds__(NT)
-    k_tile_up(LevelView<T> L, TileView<T> V, const T* __restrict__ xc, double* partial, unsigned* counter,
+    k_tile_up(LevelView<T> L, TileView<T> V, const T* __restrict__ xc, const T* __restrict__ bp_in, double* partial, unsigned* counter,
               double* mean_out, Epi epi) {
     pdl_launch();
     extern __shared__ __align__(16) unsigned char tile_smem[];
@@ -279,7 +271,7 @@ __global__ void __launch_bounds__(NT)
         if (g[u] >= 0) {
             ee[u] = xc[o[u]];
             if (k < R.z) yy[u] = L.y[g[u]];
-            if (k < R.y) bb[u] = L.bp[g[u]];
+            if (k < R.y) bb[u] = bp_in[g[u]];
             if constexpr (Epi::kRz)
                 if (mean_out && k < R.x) rv[u] = epi.r[g[u]];
         }
@@ -387,18 +379,19 @@ __device__ __forceinline__ T vt_apply(const SView<T>& L, const T* v, const unsig
 
 template <typename T, typename TB>
 __global__ void __launch_bounds__(kTileThreads)
-    v_tile_down(SView<T> L, const TB* __restrict__ bin, const double* level_sum, T* __restrict__ bc, double* partial,
-                unsigned* counter, double* coarse_sum) {
-    pdl_entry();
+    v_tile_down(SView<T> L, const TB* __restrict__ bin, const double* level_sum, T* __restrict__ bc, T* bp_out) {
+    pdl_launch();
     constexpr int N = vt::R * vt::R;
     __shared__ T sb[N], sd[N], sx[N], sy[N], sr[N], ss[N];
     __shared__ unsigned char ex[N];
     __shared__ int nb9[9];
     const int b = blockIdx.x;
     vt_blocks(L, b, nb9);
-    const double mean = (L.singular && level_sum) ? *level_sum * L.cvol_inv : 0.0;
+    const bool project = L.singular && level_sum;
+    const int4 mp = *reinterpret_cast<const int4*>(L.map + 4 * b);
     __syncthreads();
-    // the region's loads, all issued before any is used
+    // the region's loads, all issued before any is used; the volumes and
+    // diagonals before the wait
     constexpr int QU = (N + kTileThreads - 1) / kTileThreads;
     int c[QU];
     TB a[QU];
@@ -411,11 +404,15 @@ __global__ void __launch_bounds__(kTileThreads)
 #pragma unroll
     for (int u = 0; u < QU; ++u) {
         if (c[u] >= 0) {
-            a[u] = bin[c[u]];
-            vo[u] = (mean != 0.0 && !L.const_vol) ? L.vol[c[u]] : L.vol0;
+            vo[u] = (project && !L.const_vol) ? L.vol[c[u]] : L.vol0;
             dd[u] = L.dinv ? L.dinv[c[u]] : L.dinv0;
         }
     }
+    pdl_wait();
+    const double mean = project ? *level_sum * L.cvol_inv : 0.0;
+#pragma unroll
+    for (int u = 0; u < QU; ++u)
+        if (c[u] >= 0) a[u] = bin[c[u]];
 #pragma unroll
     for (int u = 0; u < QU; ++u) {
         const int q = threadIdx.x + u * kTileThreads;
@@ -451,17 +448,14 @@ __global__ void __launch_bounds__(kTileThreads)
         const int k = vt::at(q & 15, q >> 4);
         sx[k] = sr[k] - L.tw * vt_apply(L, ss, ex, k);
         L.y[b * 256 + q] = sy[k];
-        L.bp[b * 256 + q] = sb[k];
+        if (bp_out) bp_out[b * 256 + q] = sb[k];
     }
     __syncthreads();
-    const int4 mp = *reinterpret_cast<const int4*>(L.map + 4 * b);
-    double part = 0;
     if (mp.w == 1) {
         for (int q = threadIdx.x; q < 256; q += blockDim.x) {
             const int i = q & 15, j = q >> 4;
             const T t = sx[vt::at(i, j)];
             bc[mp.x * 256 + (mp.z + j) * 16 + mp.y + i] = t;
-            part += double(t);
         }
     } else {
         // 2 x 2 aggregation in the order of v_restrict: row pairs, then the row above
@@ -471,16 +465,6 @@ __global__ void __launch_bounds__(kTileThreads)
             const T d0 = sx[vt::at(i, j + 1)] + sx[vt::at(i + 1, j + 1)];
             const T t = h0 + d0;
             bc[mp.x * 256 + (mp.z + (j >> 1)) * 16 + mp.y + (i >> 1)] = t;
-            part += double(t);
-        }
-    }
-    if (coarse_sum) {
-        if (publish_partial(part, partial, counter)) {
-            const double s = fold_partials(partial, gridDim.x);
-            if (threadIdx.x == 0) {
-                *coarse_sum = s;
-                *counter = 0;
-            }
         }
     }
 }
@@ -495,8 +479,9 @@ __device__ __forceinline__ T vt_coarse(const SView<T>& L, const T* xc, int B, in
 
 template <typename T, typename Epi>
 __global__ void __launch_bounds__(kTileThreads)
-    v_tile_up(SView<T> L, const T* __restrict__ xc, double* partial, unsigned* counter, double* mean_out, Epi epi) {
-    pdl_entry();
+    v_tile_up(SView<T> L, const T* __restrict__ xc, const T* __restrict__ bp_in, double* partial, unsigned* counter,
+              double* mean_out, Epi epi) {
+    pdl_launch();
     constexpr int N = vt::R * vt::R;
     __shared__ T se[N], sp[N], sq[N], sd[N], sb[N];
     __shared__ unsigned char ex[N];
@@ -530,14 +515,18 @@ __global__ void __launch_bounds__(kTileThreads)
 #pragma unroll
     for (int u = 0; u < QU; ++u) {
         e[u] = x[u] = d[u] = bp[u] = T(0);
+        if (c[u] >= 0 && ring[u] <= 2) d[u] = L.dinv ? L.dinv[c[u]] : L.dinv0;
+    }
+    pdl_wait();
+#pragma unroll
+    for (int u = 0; u < QU; ++u) {
         if (c[u] >= 0) {
             const int4 m = mp[u];
             e[u] = m.w == 1 ? xc[m.x * 256 + (m.z + lj[u]) * 16 + m.y + li[u]]
                             : xc[m.x * 256 + (m.z + (lj[u] >> 1)) * 16 + m.y + (li[u] >> 1)];
             if (ring[u] <= 2) {
                 x[u] = L.y[c[u]];
-                d[u] = L.dinv ? L.dinv[c[u]] : L.dinv0;
-                if (ring[u] <= 1) bp[u] = L.bp[c[u]];
+                if (ring[u] <= 1) bp[u] = bp_in[c[u]];
             }
         }
     }
