@@ -248,7 +248,7 @@ tpa_status tpa_batch_solve_device(tpa_batch* batch, const double* rhs, double* x
  * recomputed inside the restriction (one launch instead of two); persistent:
  * when every multi-CTA level is a CSR level, the whole V-cycle runs as one
  * cooperative launch with grid barriers (bounded waits; a barrier that gives up
- * makes the solve return TPA_ERR_TIMEOUT); tiles: 1 (the default) runs each
+ * makes the solve return TPA_ERR_TIMEOUT); tiles: 1 runs each
  * CSR level of the multi-CTA part as two launches on haloed block tiles (both
  * pre-sweeps, the residual and the restriction in one, the prolongation and
  * both post-sweeps in the other; the halo is recomputed in each tile), 2 also
@@ -257,8 +257,8 @@ tpa_status tpa_batch_solve_device(tpa_batch* batch, const double* rhs, double* x
  * the vectorized kernels), 4 as 3 with the larger levels of a periodic block
  * lattice (one tree level of 16x16 blocks filling the domain, constant
  * diagonal and volumes) on row-streaming kernels (two launches per level: a
- * warp walks a strip 26 cells wide up the level with the phases one row
- * apart), 5 every periodic lattice level on row-streaming kernels and the
+ * warp walks a strip 56 cells wide up the level with the phases one row
+ * apart), 5 (the default) every periodic lattice level on row-streaming kernels and the
  * other constant-coefficient levels as 3, 0 none.
  * Every layout gives the same V-cycle to rounding. */
 typedef struct {

@@ -707,16 +707,18 @@ TuneConfig DeviceSolver::effective_tuning() const {
     if (tune_.fuse_restrict >= 0) c.fuse_restrict = tune_.fuse_restrict;
     c.persistent = std::getenv("TPAGMG_PERSISTENT") ? 1 : 0;
     if (tune_.persistent >= 0) c.persistent = tune_.persistent ? 1 : 0;
-    // 1: CSR levels on tiles (the default: measured faster on the droplet),
-    // 2: the constant-coefficient 16x16 levels on stencil tiles as well
-    // (measured slower than the vectorized kernels on uniform 2048^2, whose
-    // finest level makes the tile kernel instruction-bound), 3: stencil tiles
-    // on the constant-coefficient levels of at most kStencilTileCells cells
-    // only, where the six vectorized launches are latency-bound, 4: as 3, with
-    // the larger periodic lattice levels on the row-streaming kernels
-    // (stream.cuh), 5: every periodic lattice level on the row-streaming
-    // kernels, the other constant-coefficient levels as 3, 0: none
-    c.tiles = 1;
+    // 0: no tiles, 1: CSR levels on tiles, 2: the constant-coefficient 16x16
+    // levels on stencil tiles as well, 3: stencil tiles on the constant-coefficient
+    // levels of at most kStencilTileCells cells only, 4: as 3, with the larger
+    // periodic lattice levels on the row-streaming kernels (stream.cuh), 5 (the
+    // default): every periodic lattice level on the row-streaming kernels, the other
+    // constant-coefficient levels as 3.  Two launches per level against the six of
+    // the vectorized kernels, 5 against 1 per solve: periodic 128^2 FP64 699 -> 558
+    // us, 1024 x 512 refinement 1243 -> 914, 2048^2 mixed 3073 -> 1852 (start
+    // against here), droplet 1371 -> 1363.  Above kStencilTileCells the stencil
+    // tiles' index arithmetic is slower than the vectorized kernels (2 on 2048^2),
+    // which keep the large levels that do not stream.
+    c.tiles = 5;
     if (const char* e = std::getenv("TPAGMG_TILES")) c.tiles = std::min(5, std::max(0, std::atoi(e)));
     if (tune_.tiles >= 0) c.tiles = std::min(5, tune_.tiles);
     if (rb_) {  // the red-black sweeps exist for the CSR levels and the tail only
