@@ -24,6 +24,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "cg_state.cuh"
 #include "device.cuh"
 
 namespace tpa {
@@ -431,6 +432,9 @@ DeviceSolver::DeviceSolver(int device) : device_(device) {
     stream_ = own_stream_;
     TPA_CUDA(cudaMallocHost(&host_sc_, sizeof(CgScalars)));
     TPA_CUDA(cudaMallocHost(&host_d_, 64 * sizeof(double)));
+    TPA_CUDA(cudaMallocHost(&host_solve_, sizeof(SolveState)));
+    TPA_CUDA(cudaEventCreate(&ev0_));
+    TPA_CUDA(cudaEventCreate(&ev1_));
     partial_.alloc(static_cast<size_t>(4 * kReduceBlocks));
     sc_.alloc(1);
     sums_.alloc(64);
@@ -443,6 +447,9 @@ DeviceSolver::~DeviceSolver() {
     levels_.clear();
     if (host_sc_) cudaFreeHost(host_sc_);
     if (host_d_) cudaFreeHost(host_d_);
+    if (host_solve_) cudaFreeHost(host_solve_);
+    if (ev0_) cudaEventDestroy(ev0_);
+    if (ev1_) cudaEventDestroy(ev1_);
     if (rstage_) cudaFreeHost(rstage_);
     if (own_stream_) cudaStreamDestroy(own_stream_);
 }

@@ -139,6 +139,8 @@ int fold_grid(K kernel, int block, int64_t want, int cap, size_t smem = 0) {
 std::vector<unsigned char> red_black_colours(const Mesh& m);
 double red_black_weight(const Csr& A, const std::vector<unsigned char>& colours);
 
+struct SolveState;
+
 class DeviceSolver {
 public:
     explicit DeviceSolver(int device);
@@ -218,6 +220,9 @@ private:
     bool rz_foldable() const;
     // CG from the current xw_/b_: returns iterations and flags (Krylov.jl cg! loop)
     void cg_fused(int precision, double target, int itmax, int& niter, int& flags);
+    void cg_loop(int precision);
+    void count_cg_bodies(int precision, int iter, int flags);
+    void ensure_ir();
     void vcycle_fused(const double* r, double* z, int precision);
     void destroy_graphs();
     cudaGraphExec_t cg_graph(int precision);
@@ -242,7 +247,10 @@ private:
     // `solve!` with the set-up and checks fused into two passes (solve_fast.cu)
     void solve_fast(const double* rhs, double* x, double rtol, double atol, int max_cycles, int compatibility,
                     int precision, SolveStats& st);
-    DevArray<double> spartial_, spres_;
+    DevArray<double> spartial_;
+    DevArray<char> sstate_;          // SolveState (cg_state.cuh)
+    SolveState* host_solve_ = nullptr;  // its pinned host copy
+    cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;  // around a solve (its device time)
     double vol_total_ = 0;  // finest-level volume of cells with V > 0
 
     bool fused_ok_ = false;

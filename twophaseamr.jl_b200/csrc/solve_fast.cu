@@ -1,5 +1,5 @@
 // `solve!` around the graph-captured CG loop, with its set-up and checks fused
-// into two finest-level passes (default cycle, at most one ungauged component).
+// into finest-level passes (default cycle, at most one ungauged component).
 //
 // The steps are those of src/solvers/multigrid/elliptic_solver.jl:628-675
 // (ronaldremmerswaal/TwoPhaseAMR.jl): b = V f with covered cells zeroed, the
@@ -7,14 +7,25 @@
 // the initial guess, the initial norms and target (`_solve_krylov_with_stats!`,
 // :550-612, with the roundoff floor of cycles.jl:108-206), Krylov runs with
 // restarts from the true residual (`_run_krylov_reliably!`, :487-526) and the
-// final gauge.  `k_prep` folds the three sums the projection and the gauge need;
-// `k_pres` applies them and evaluates the residual, its two norms and both
-// inputs of the roundoff floor in the same pass.
+// final gauge.
+//
+// `k_prep` folds the three sums the projection and the gauge need; `k_pres`
+// applies them and evaluates the residual, its norms and both inputs of the
+// roundoff floor in one pass.  The CTA that folds them also takes the decision
+// that follows (means, target, whether there is anything to solve, the state of
+// the run), so a solve is one chain of launches that the host reads once, at
+// the end of the first run: prep, pres, the CG graph, the iterate's mean, pres.
+// Reading every decision on the host took six synchronizations of 8-15 us each,
+// and the run started with a residual pass of its own.
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstdlib>
+#include <type_traits>
 
+#include "cg_state.cuh"
 #include "device.cuh"
+#include "launch.cuh"
 
 namespace tpa {
 namespace {
@@ -44,10 +55,10 @@ __device__ __forceinline__ double block_max_all(double v) {
 }
 
 // Publish N block values (sums where max_mask bit k is 0, maxima where it is 1)
-// and fold them in the last block in block order into out[0..N).
-template <int N>
+// and fold them in the last block in block order; its thread 0 calls done(out[N]).
+template <int N, typename F>
 __device__ __forceinline__ void publish_fold(const double (&v)[N], unsigned max_mask, double* partial,
-                                             unsigned* counter, double* out) {
+                                             unsigned* counter, F done) {
     __shared__ bool last;
     double b[N];
     for (int k = 0; k < N; ++k) b[k] = (max_mask >> k) & 1 ? block_max_all(v[k]) : block_sum_all(v[k]);
@@ -60,98 +71,188 @@ __device__ __forceinline__ void publish_fold(const double (&v)[N], unsigned max_
     __syncthreads();
     if (!last) return;
     __threadfence();
+    double out[N];
     for (int k = 0; k < N; ++k) {
-        const double r = (max_mask >> k) & 1 ? fold_partials_max(partial + k * gridDim.x, gridDim.x)
-                                             : fold_partials(partial + k * gridDim.x, gridDim.x);
-        if (threadIdx.x == 0) out[k] = r;
+        out[k] = (max_mask >> k) & 1 ? fold_partials_max(partial + k * gridDim.x, gridDim.x)
+                                     : fold_partials(partial + k * gridDim.x, gridDim.x);
         __syncthreads();
     }
-    if (threadIdx.x == 0) *counter = 0;
+    if (threadIdx.x == 0) {
+        *counter = 0;
+        done(out);
+    }
 }
 
-// b = V f (0 where V = 0), x0 = x_in (0 where V = 0); out = {sum b, sum |b|, sum V x0}.
+constexpr double kEps = 2.220446049250313e-16;
+
+// std::max's choice, a NaN in second place included
+__device__ __forceinline__ double std_max(double a, double b) { return a < b ? b : a; }
+
+// roundoff floor of a residual from max |A||x| / V and max |b| / V
+__host__ __device__ inline double roundoff_floor(double ax, double b) {
+    const double m = ax < b ? b : ax;
+    return 128 * kEps * (1.0 < m ? m : 1.0);
+}
+
+// What the solve was asked for (kernel parameters).
+struct SolveAsk {
+    double rtol, atol, cvol;  // cvol: volume of the ungauged component (0: none)
+    double eta;               // refinement solve: reduction per run (0: one run to the target)
+    int max_cycles, strict;   // strict: an incompatible right-hand side is an error
+};
+
+// target of a run from a residual of strong maximum linf
+__device__ __forceinline__ double run_target(const SolveAsk& q, double target, double linf) {
+    return q.eta > 0 ? std_max(target, q.eta * linf) : target;
+}
+
+__device__ __forceinline__ void start_run(CgState* c, double target, double rsum, int itmax, bool go) {
+    c->target = target;
+    c->rsum = rsum;
+    c->itmax = itmax;
+    c->iter = 0;
+    c->fresh = 1;
+    c->flags = go ? 0 : 8;
+}
+
+// sums of b = V f, |b| and V x0 over cells with V > 0; the means to remove.
 // vol null: every cell's volume is vol0.
 __global__ void k_prep(int n, const double* __restrict__ rhs, const double* __restrict__ xin,
-                       const double* __restrict__ vol, double vol0, double* __restrict__ b, double* __restrict__ x0,
-                       double* partial, unsigned* counter, double* out) {
+                       const double* __restrict__ vol, double vol0, SolveAsk q, double* partial, unsigned* counter,
+                       SolveState* S) {
+    pdl_entry();
     double v[3] = {0, 0, 0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const double V = vol ? vol[i] : vol0;
         const double bi = V > 0 ? rhs[i] * V : 0.0;
         const double xi = V > 0 ? xin[i] : 0.0;
-        b[i] = bi;
-        x0[i] = xi;
         v[0] += bi;
         v[1] += fabs(bi);
         v[2] += V * xi;
     }
-    publish_fold<3>(v, 0u, partial, counter, out);
+    publish_fold<3>(v, 0u, partial, counter, [&](const double (&t)[3]) {
+        S->sum_b = t[0];
+        S->abs_b = t[1];
+        const bool comp = q.cvol != 0;
+        S->mb = comp ? t[0] / q.cvol : 0.0;
+        S->mx = comp ? t[2] / q.cvol : 0.0;
+        S->xm = 0;
+        // a non-finite right-hand side value makes sum |b| non-finite
+        S->ok = isfinite(t[1]) && !(q.strict && comp && fabs(t[0]) > 256 * kEps * std_max(1.0, t[1]));
+    });
 }
 
-// b -= V mb, x = x0 - mx (0 where V = 0), r = b - A x; out = {sum_V r^2 / V,
-// max |r| / V, max (|A| |x|) / V, max |b| / V} over cells with V > 0.  A x is
-// summed as sum_j a_ij (x_j - x_i) (+ bdiag_i x_i at open sides): the rows
-// sum to that conductance (the area-weighted jump maps constants to zero), and
-// this form rounds at
+// After the first residual: the target, and the first run unless there is
+// nothing to solve.  v: {sum_V r^2 / V, max |r| / V, max |A||x| / V, max |b| / V, sum r}.
+__device__ __forceinline__ void after_first(const double (&v)[5], const SolveAsk& q, SolveState* S, CgState* c) {
+    for (int k = 0; k < 4; ++k) S->init[k] = S->fin[k] = v[k];
+    const double floor = roundoff_floor(v[2], v[3]);
+    const double target = std_max(q.atol, std_max(q.rtol * std_max(v[1], kEps), floor));
+    const bool go = S->ok && v[1] > target && q.max_cycles > 0;
+    S->target = target;
+    S->skip = go ? 0 : 1;
+    S->niter = S->flags = S->total = 0;
+    start_run(c, run_target(q, target, v[1]), v[4], q.max_cycles, go);
+}
+
+// After a run's true residual: its counts, and the state of a further run
+// (which the host decides on).
+__device__ __forceinline__ void after_run(const double (&v)[5], const SolveAsk& q, SolveState* S, CgState* c) {
+    for (int k = 0; k < 4; ++k) S->fin[k] = v[k];
+    S->niter = c->iter;
+    S->flags = c->flags;
+    S->total += c->iter;
+    start_run(c, run_target(q, S->target, v[1]), v[4], q.max_cycles - S->total, true);
+}
+
+// Vectors of a residual pass.  First: b = V f - V mb and x = x_in - mx (0 where
+// V = 0) are formed from the caller's rhs and guess and stored; else b and x
+// are the solve's and x - xm goes to the caller's array.
+struct PresIo {
+    const double* rhs;  // the caller's (first pass)
+    const double* xin;  // the guess (first) or the iterate
+    double* b;
+    double* xout;       // the solve's iterate (first) or the caller's solution
+    double* r;
+};
+
+// r = b - A x with the norms.  A x is summed as sum_j a_ij (x_j - x_i) (+ bdiag_i
+// x_i at open sides): the rows sum to that conductance (the area-weighted jump
+// maps constants to zero), and this form rounds at
 // the level of the face fluxes, as the factorized action of elliptic.jl:
 // 1125-1180 does, not at the level of a_ii x_i.  The projection step relies on
 // it: dt max |div u| after the update equals the final residual over 1/dt^2 to
 // a few ulps only when both are evaluated from face differences.
-__global__ void k_pres(LevelView<double> A, double* __restrict__ b, const double* __restrict__ x0,
-                       double* __restrict__ x, double* __restrict__ r, double mb, double mx, int masked,
-                       double* partial, unsigned* counter, double* out) {
-    double v[4] = {0, 0, 0, 0};
+template <bool First>
+__global__ void k_pres(LevelView<double> A, PresIo io, int masked, SolveAsk q, double* partial, unsigned* counter,
+                       SolveState* S, CgState* c) {
+    pdl_entry();
+    const double m = First ? S->mx : S->xm, mb = First ? S->mb : 0.0;
+    const bool store = First || S->ok;
+    const double* __restrict__ x0 = io.xin;
+    double v[5] = {0, 0, 0, 0, 0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < A.n; i += gridDim.x * blockDim.x) {
         const double V = A.vol[i];
-        double bi = b[i];
-        if (mb != 0.0 && V > 0) {
-            bi -= V * mb;
-            b[i] = bi;
+        double bi;
+        if (First) {
+            bi = V > 0 ? io.rhs[i] * V : 0.0;
+            if (mb != 0.0 && V > 0) bi -= V * mb;
+            io.b[i] = bi;
+        } else {
+            bi = io.b[i];
         }
-        const double xi = V > 0 ? x0[i] - mx : 0.0;
+        const double xi = V > 0 ? x0[i] - m : 0.0;
         double acc = 0, aacc = 0;
         for (int k = A.rp[i]; k < A.rp[i + 1]; ++k) {
             const int j = A.ci[k];
-            const double xj = (!masked || A.vol[j] > 0) ? x0[j] - mx : 0.0;
+            const double xj = (!masked || A.vol[j] > 0) ? x0[j] - m : 0.0;
             acc += A.val[k] * (xj - xi);
             aacc += fabs(A.val[k]) * fabs(xj);
         }
         if (A.bdiag) acc += A.bdiag[i] * xi;  // rows at open sides do not sum to zero
-        x[i] = xi;
+        if (store) io.xout[i] = xi;
         const double ri = bi - acc;
-        r[i] = ri;
+        io.r[i] = ri;
+        v[4] += ri;
         if (V > 0) {
             v[0] += ri * ri / V;
-            const double q = fabs(ri) / V;
-            v[1] = (q != q || v[1] != v[1]) ? NAN : fmax(v[1], q);
+            const double s = fabs(ri) / V;
+            v[1] = (s != s || v[1] != v[1]) ? NAN : fmax(v[1], s);
             v[2] = fmax(v[2], aacc / V);
             v[3] = fmax(v[3], fabs(bi) / V);
         }
     }
-    publish_fold<4>(v, 0xEu, partial, counter, out);
+    publish_fold<5>(v, 0xEu, partial, counter, [&](const double (&t)[5]) {
+        if (First) after_first(t, q, S, c);
+        else after_run(t, q, S, c);
+    });
 }
 
 // k_pres on a constant-coefficient 16x16 finest level (vectorized quads,
 // stencil4.cuh): the row is c0 (count x_c - sum of neighbours), evaluated as
 // c0 sum (x_c - x_nb) like k_pres; |A| |x| = |c0| (count |x_c| + sum |neighbours|).
-__global__ void __launch_bounds__(256) v_pres(SView<double> S, double* __restrict__ b, const double* __restrict__ x0,
-                                              double* __restrict__ x, double* __restrict__ r, double mb, double mx,
-                                              double* partial, unsigned* counter, double* out) {
-    double v[4] = {0, 0, 0, 0};
-    const int groups = (S.nblocks + 3) / 4;
-    const double* vol = S.vol;
-    const double ac0 = fabs(S.c0);
+// Every array is 16-byte aligned but the caller's solution, which `wide` says.
+template <bool First>
+__global__ void __launch_bounds__(256) v_pres(SView<double> L, PresIo io, int wide, SolveAsk q, double* partial,
+                                              unsigned* counter, SolveState* S, CgState* c) {
+    pdl_entry();
+    const double mx = First ? S->mx : S->xm, mb = First ? S->mb : 0.0;
+    const bool store = First || S->ok;
+    double v[5] = {0, 0, 0, 0, 0};
+    const int groups = (L.nblocks + 3) / 4;
+    const double* vol = L.vol;
+    const double ac0 = fabs(L.c0);
     for (int grp = blockIdx.x; grp < groups; grp += gridDim.x) {
         const QPos p = q_pos(grp);
-        const bool valid = p.b < S.nblocks;
+        const bool valid = p.b < L.nblocks;
         // a level of equal positive volumes needs no per-cell volume loads
-        const bool uniform = S.const_vol && S.vol0 > 0;
+        const bool uniform = L.const_vol && L.vol0 > 0;
         const QNb<double> g = q_gather<double>(
-            S, p, valid, [&](int c) { return q_ldv(x0 + c); },
-            [&](double xv, int c) { return (uniform || vol[c] > 0) ? xv - mx : 0.0; });
+            L, p, valid, [&](int k) { return q_ldv(io.xin + k); },
+            [&](double xv, int k) { return (uniform || vol[k] > 0) ? xv - mx : 0.0; });
         if (!valid) continue;
-        const Quad<double> vq = uniform ? Quad<double>{{S.vol0, S.vol0, S.vol0, S.vol0}} : q_ld(vol + p.c);
-        Quad<double> bq = q_ldv(b + p.c), rq;
+        const Quad<double> vq = uniform ? Quad<double>{{L.vol0, L.vol0, L.vol0, L.vol0}} : q_ld(vol + p.c);
+        Quad<double> bq = q_ldv((First ? io.rhs : io.b) + p.c), rq;
         for (int m = 0; m < 4; ++m) {
             const bool hw = m > 0 || g.hw, he = m < 3 || g.he;
             const double xc = g.x.v[m];
@@ -168,155 +269,156 @@ __global__ void __launch_bounds__(256) v_pres(SView<double> S, double* __restric
             if (g.hs) nb += fabs(g.s.v[m]), diff += xc - g.s.v[m], ++cnt;
             if (g.hn) nb += fabs(g.n.v[m]), diff += xc - g.n.v[m], ++cnt;
             const double aacc = ac0 * (double(cnt) * fabs(xc) + nb);
-            const double axm = S.c0 * diff;
+            const double axm = L.c0 * diff;
             const double V = vq.v[m];
             double bi = bq.v[m];
-            if (mb != 0.0 && V > 0) bi -= V * mb;
-            bq.v[m] = bi;
+            if (First) {
+                bi = V > 0 ? bi * V : 0.0;
+                if (mb != 0.0 && V > 0) bi -= V * mb;
+                bq.v[m] = bi;
+            }
             const double ri = bi - axm;
             rq.v[m] = ri;
+            v[4] += ri;
             if (V > 0) {
                 v[0] += ri * ri / V;
-                const double q = fabs(ri) / V;
-                v[1] = (q != q || v[1] != v[1]) ? NAN : fmax(v[1], q);
+                const double s = fabs(ri) / V;
+                v[1] = (s != s || v[1] != v[1]) ? NAN : fmax(v[1], s);
                 v[2] = fmax(v[2], aacc / V);
                 v[3] = fmax(v[3], fabs(bi) / V);
             }
         }
-        if (mb != 0.0) q_st(b + p.c, bq);
-        q_st(x + p.c, g.x);
-        q_st(r + p.c, rq);
+        if (First) q_st(io.b + p.c, bq);
+        if (store) {
+            if (wide) q_st(io.xout + p.c, g.x);
+            else
+                for (int m = 0; m < 4; ++m) io.xout[p.c + m] = g.x.v[m];
+        }
+        q_st(io.r + p.c, rq);
     }
-    publish_fold<4>(v, 0xEu, partial, counter, out);
+    publish_fold<5>(v, 0xEu, partial, counter, [&](const double (&t)[5]) {
+        if (First) after_first(t, q, S, c);
+        else after_run(t, q, S, c);
+    });
 }
 
-// out = sum V x; x0 = x (the next k_pres reads x0 and writes x).  vol null:
-// every cell's volume is vol0.
-__global__ void k_xmean(int n, const double* __restrict__ x, const double* __restrict__ vol, double vol0,
-                        double* __restrict__ x0, double* partial, unsigned* counter, double* out) {
+// the iterate's mean sum V x / cvol, taken off by the next residual pass (none
+// when no run was made).  vol null: every cell's volume is vol0.
+__global__ void k_xmean(int n, const double* __restrict__ x, const double* __restrict__ vol, double vol0, double cvol,
+                        double* partial, unsigned* counter, SolveState* S) {
+    pdl_entry();
     double v[1] = {0};
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const double xi = x[i];
-        x0[i] = xi;
-        v[0] += (vol ? vol[i] : vol0) * xi;
-    }
-    publish_fold<1>(v, 0u, partial, counter, out);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        v[0] += (vol ? vol[i] : vol0) * x[i];
+    publish_fold<1>(v, 0u, partial, counter, [&](const double (&t)[1]) { S->xm = S->skip ? 0.0 : t[0] / cvol; });
 }
 
 }  // namespace
 
 void DeviceSolver::solve_fast(const double* rhs, double* x_user, double rtol, double atol, int max_cycles,
                               int compatibility, int precision, SolveStats& st) {
-    const double eps = 2.220446049250313e-16;
     DevLevel& L = levels_[0];
     const int n = L.n;
     const LevelView<double>& A = vd_[0];
+    // programmatic launch only behind a kernel of this solve (not behind the
+    // caller's work or a graph)
+    const Launch go{stream_, pdl_}, plain{stream_, false};
     const int64_t want = (int64_t(n) + kThreads - 1) / kThreads;
-    double* out = spres_.p;
-    const double cvol = L.ncomp == 1 ? L.comp_volume[0] : 0.0;
+    const double* vol = L.const_vol ? nullptr : A.vol;
+    SolveState* S = reinterpret_cast<SolveState*>(sstate_.p);
+    CgState* cg = reinterpret_cast<CgState*>(cgs_.p);
+    const SolveState& hs = *host_solve_;
+    SolveAsk ask;
+    ask.rtol = rtol;
+    ask.atol = atol;
+    ask.cvol = L.ncomp == 1 ? L.comp_volume[0] : 0.0;
+    // precision 2, FP64 iterative refinement: each run is a CG on the correction
+    // with FP32 r, directions and Ap (x and every inner product stay FP64),
+    // started from the FP32 rounding of the true residual and stopped at a fixed
+    // reduction of it or at the target; its recurrence residual follows the true
+    // one to about the FP32 unit roundoff per iteration
+    ask.eta = precision == 2 ? ir_eta_ : 0.0;
+    ask.max_cycles = max_cycles;
+    ask.strict = compatibility == 1 ? 1 : 0;
     double vt = 0;  // total volume of cells with V > 0
     for (double v : L.comp_volume) vt += v;
     if (L.ncomp == 0) vt = vol_total_;
-    auto read = [&](int count) {
-        TPA_CUDA(cudaMemcpyAsync(host_d_, out, size_t(count) * sizeof(double), cudaMemcpyDeviceToHost, stream_));
-        TPA_CUDA(cudaStreamSynchronize(stream_));
-    };
-    cudaEvent_t e0, e1;
-    TPA_CUDA(cudaEventCreate(&e0));
-    TPA_CUDA(cudaEventCreate(&e1));
-    TPA_CUDA(cudaEventRecord(e0, stream_));
+    if (precision == 2) ensure_ir();
+    TPA_CUDA(cudaEventRecord(ev0_, stream_));
     st = SolveStats();
 
-    k_prep<<<fold_grid(k_prep, kThreads, want, kGrid), kThreads, 0, stream_>>>(n, rhs, x_user, L.const_vol ? nullptr : A.vol, L.vol0, b_.p, tmp_.p, spartial_.p, counters_.p + kCPrep,
-                                           out);
-    ++launches_;
-    read(3);
-    // a non-finite right-hand side value makes sum |b| non-finite
-    if (!std::isfinite(host_d_[1])) throw Error(4, "right-hand side must be finite");
-    double mb = 0, mx = 0;
-    if (L.ncomp == 1) {
-        if (compatibility == 1 && std::fabs(host_d_[0]) > 256 * eps * std::max(1.0, host_d_[1]))
-            throw Error(1, "Poisson right-hand side has nonzero volume mean");
-        mb = host_d_[0] / cvol;
-        mx = host_d_[2] / cvol;
-        st.removed_rhs_mean = mb;
-        st.removed_max_component_mean = std::fabs(mb);
+    plain(k_prep, fold_grid(k_prep, kThreads, want, kGrid), kThreads, 0, n, rhs, (const double*)x_user, vol, L.vol0, ask,
+       spartial_.p, counters_.p + kCPrep, S);
+    auto aligned = [](const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+    const bool vec = sdev_[0].vec;
+    PresIo first{rhs, x_user, b_.p, xw_.p, r_.p};
+    if (vec && !(aligned(rhs) && aligned(x_user))) {
+        // the vectorized pass reads 16 bytes at a time
+        TPA_CUDA(cudaMemcpyAsync(b_.p, rhs, sizeof(double) * size_t(n), cudaMemcpyDeviceToDevice, stream_));
+        TPA_CUDA(cudaMemcpyAsync(tmp_.p, x_user, sizeof(double) * size_t(n), cudaMemcpyDeviceToDevice, stream_));
+        first.rhs = b_.p;
+        first.xin = tmp_.p;
     }
-    struct Norms {
-        double l2, linf, floor;
+    auto pres = [&](auto is_first, const PresIo& io, const Launch& launch) {
+        constexpr bool F = decltype(is_first)::value;
+        if (vec)
+            launch(v_pres<F>, fold_grid(v_pres<F>, 256, (sd_[0].nblocks + 3) / 4, kGrid), 256, 0, sd_[0], io,
+               aligned(io.xout) ? 1 : 0, ask, spartial_.p, counters_.p + kCPres, S, cg);
+        else
+            launch(k_pres<F>, fold_grid(k_pres<F>, kThreads, want, kGrid), kThreads, 0, A, io, L.any_void ? 1 : 0, ask,
+               spartial_.p, counters_.p + kCPres, S, cg);
     };
-    auto pres = [&](double b_mean, double x_mean) {
-        if (sdev_[0].vec) {
-            const int groups = (sd_[0].nblocks + 3) / 4;
-            v_pres<<<fold_grid(v_pres, 256, groups, kGrid), 256, 0, stream_>>>(
-                sd_[0], b_.p, tmp_.p, xw_.p, r_.p, b_mean, x_mean, spartial_.p, counters_.p + kCPres, out);
-        } else {
-            k_pres<<<fold_grid(k_pres, kThreads, want, kGrid), kThreads, 0, stream_>>>(
-                A, b_.p, tmp_.p, xw_.p, r_.p, b_mean, x_mean, L.any_void ? 1 : 0, spartial_.p, counters_.p + kCPres,
-                out);
-        }
-        ++launches_;
-        read(4);
-        Norms nm;
-        nm.l2 = vt > 0 ? std::sqrt(host_d_[0] / vt) : 0.0;
-        nm.linf = host_d_[1];
-        nm.floor = 128 * eps * std::max(1.0, std::max(host_d_[2], host_d_[3]));
-        return nm;
-    };
-    const Norms init = pres(mb, mx);
-    const double target = std::max(atol, std::max(rtol * std::max(init.linf, eps), init.floor));
+    pres(std::true_type(), first, first.rhs == rhs ? go : plain);
+    launches_ += 2;
+    double target = 0, init_linf = 0;
     auto guarded = [&](double cur, double fl) {
-        if (!(std::isfinite(init.linf) && std::isfinite(cur) && target < cur && cur < init.linf)) return target;
-        return (std::isfinite(fl) && fl < init.linf / 100) ? std::max(target, fl) : target;
+        if (!(std::isfinite(init_linf) && std::isfinite(cur) && target < cur && cur < init_linf)) return target;
+        return (std::isfinite(fl) && fl < init_linf / 100) ? std::max(target, fl) : target;
     };
-    Norms fin = init;
-    int total = 0;
-    if (init.linf > target) {
-        while (total < max_cycles) {
-            int niter = 0, flags = 0;
-            // precision 2, FP64 iterative refinement: each run is a CG on the
-            // correction with FP32 r, directions and Ap (x and every inner
-            // product stay FP64), started from the FP32 rounding of the true
-            // residual and stopped at a fixed reduction of it or at the target;
-            // its recurrence residual follows the true one to about the FP32
-            // unit roundoff per iteration
-            const double inner = precision == 2 ? std::max(target, ir_eta_ * fin.linf) : target;
-            cg_fused(precision, inner, max_cycles - total, niter, flags);
-            total += niter;
-            // gauge of the iterate, then the true residual and its norms
-            k_xmean<<<fold_grid(k_xmean, kThreads, want, kGrid), kThreads, 0, stream_>>>(n, xw_.p, L.const_vol ? nullptr : A.vol, L.vol0, tmp_.p, spartial_.p, counters_.p + kCMean,
-                                                    out);
+    for (bool first_run = true;; first_run = false) {
+        if (max_cycles > 0) cg_loop(precision);
+        // gauge of the iterate, then the true residual and its norms
+        if (L.ncomp == 1) {
+            plain(k_xmean, fold_grid(k_xmean, kThreads, want, kGrid), kThreads, 0, n, (const double*)xw_.p, vol, L.vol0,
+               ask.cvol, spartial_.p, counters_.p + kCMean, S);
             ++launches_;
-            double xm = 0;
-            if (L.ncomp == 1) {
-                read(1);
-                xm = host_d_[0] / cvol;
-            }
-            fin = pres(0.0, xm);
-            ++st.restarts;
-            const double eff = guarded(fin.linf, fin.floor);
-            if (fin.linf <= eff) break;
-            if (!std::isfinite(fin.linf) || niter == 0) break;
         }
+        pres(std::false_type(), PresIo{nullptr, xw_.p, b_.p, x_user, r_.p}, L.ncomp == 1 ? go : plain);
+        ++launches_;
+        TPA_CUDA(cudaMemcpyAsync(host_solve_, S, sizeof(SolveState), cudaMemcpyDeviceToHost, stream_));
+        TPA_CUDA(cudaEventRecord(ev1_, stream_));
+        TPA_CUDA(cudaStreamSynchronize(stream_));
+        TPA_CUDA(cudaGetLastError());
+        if (first_run) {
+            if (!std::isfinite(hs.abs_b)) throw Error(4, "right-hand side must be finite");
+            if (!hs.ok) throw Error(1, "Poisson right-hand side has nonzero volume mean");
+            target = hs.target;
+            init_linf = hs.init[1];
+            if (hs.skip) break;
+        }
+        count_cg_bodies(precision, hs.niter, hs.flags);
+        ++st.restarts;
+        const double linf = hs.fin[1];
+        if (linf <= guarded(linf, roundoff_floor(hs.fin[2], hs.fin[3]))) break;
+        if (!std::isfinite(linf) || hs.niter == 0 || hs.total >= max_cycles) break;
     }
-    check_barrier();
-    const double tfinal = guarded(fin.linf, fin.floor);
-    TPA_CUDA(cudaMemcpyAsync(x_user, xw_.p, sizeof(double) * size_t(n), cudaMemcpyDeviceToDevice, stream_));
-    TPA_CUDA(cudaEventRecord(e1, stream_));
-    TPA_CUDA(cudaEventSynchronize(e1));
-    TPA_CUDA(cudaGetLastError());
+    if (coop_grid_ > 0) check_barrier();
+    auto l2 = [&](double s) { return vt > 0 ? std::sqrt(s / vt) : 0.0; };
+    const double tfinal = guarded(hs.fin[1], roundoff_floor(hs.fin[2], hs.fin[3]));
     float ms = 0;
-    cudaEventElapsedTime(&ms, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
-    st.cycles = total;
-    st.converged = std::isfinite(fin.linf) && std::isfinite(tfinal) && fin.linf <= tfinal;
-    st.initial_l2 = init.l2;
-    st.initial_linf = init.linf;
-    st.final_l2 = fin.l2;
-    st.final_linf = fin.linf;
+    cudaEventElapsedTime(&ms, ev0_, ev1_);
+    if (L.ncomp == 1) {
+        st.removed_rhs_mean = hs.mb;
+        st.removed_max_component_mean = std::fabs(hs.mb);
+    }
+    st.cycles = hs.total;
+    st.converged = std::isfinite(hs.fin[1]) && std::isfinite(tfinal) && hs.fin[1] <= tfinal;
+    st.initial_l2 = l2(hs.init[0]);
+    st.initial_linf = hs.init[1];
+    st.final_l2 = l2(hs.fin[0]);
+    st.final_linf = hs.fin[1];
     st.target_linf = tfinal;
-    st.residual_scale = std::max(init.linf, eps);
+    st.residual_scale = std::max(hs.init[1], kEps);
     st.ms_total = ms;
 }
 

@@ -13,7 +13,9 @@
 #include <cstring>
 #include <type_traits>
 
+#include "cg_state.cuh"
 #include "device.cuh"
+#include "launch.cuh"
 #include "persistent.cuh"
 #include "stream.cuh"
 #include "tail_dense.cuh"
@@ -61,17 +63,6 @@ static void with_cg_rows(int rows, F f) {
 
 namespace {
 
-struct CgState {
-    double gamma, pAp, alpha, beta, pnorm2, strong_max, target, rsum, rnorm;
-    int flags;  // 1 user exit, 2 zero curvature, 4 machine stop, 8 zero initial residual
-    int iter, itmax;
-    int fresh;  // the next r'z starts the run (gamma = r'z, p = z)
-};
-
-// flags that end a run in the middle of a loop body: the direction and the
-// update of that body do nothing
-constexpr int kCgHalt = 2 | 4 | 8;
-
 enum Counter { kPostMean = 1, kCgAp = 2, kCgUpdate = 3, kCgZ = 4, kCgRes = 5, kRsum = 6 };
 
 inline int blocks_for(int64_t n) {
@@ -86,48 +77,6 @@ constexpr int kMaxGrid = 1184;
 // keep.
 constexpr int kStencilTileCells = 1 << 19;  // 8 CTAs on each of 148 SMs: bounds the partials every fold reads
 #define TPA_GRID_STRIDE(i, n) for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += gridDim.x * blockDim.x)
-
-// Kernel launch on `s`, with programmatic dependent launch when `pdl`: the
-// next kernel of the cycle is scheduled while this one drains and waits in
-// pdl_entry() for its results, which hides the launch gap between the short,
-// dependent kernels of a V-cycle.
-struct Launch {
-    cudaStream_t s;
-    bool pdl;
-    int cluster = 1;     // CTAs per thread-block cluster (grid must be a multiple)
-    bool coop = false;   // cooperative launch (every CTA resident at once)
-    template <typename... KArgs, typename... Args>
-    void operator()(void (*kernel)(KArgs...), int grid, int block, size_t smem, Args... args) const {
-        cudaLaunchConfig_t cfg;
-        std::memset(&cfg, 0, sizeof(cfg));
-        cfg.gridDim = dim3(unsigned(grid));
-        cfg.blockDim = dim3(unsigned(block));
-        cfg.dynamicSmemBytes = smem;
-        cfg.stream = s;
-        cudaLaunchAttribute at[3];
-        unsigned na = 0;
-        if (coop) {
-            at[na].id = cudaLaunchAttributeCooperative;
-            at[na].val.cooperative = 1;
-            ++na;
-        }
-        if (pdl) {
-            at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            at[na].val.programmaticStreamSerializationAllowed = 1;
-            ++na;
-        }
-        if (cluster > 1) {
-            at[na].id = cudaLaunchAttributeClusterDimension;
-            at[na].val.clusterDim.x = unsigned(cluster);
-            at[na].val.clusterDim.y = 1;
-            at[na].val.clusterDim.z = 1;
-            ++na;
-        }
-        cfg.attrs = at;
-        cfg.numAttrs = na;
-        TPA_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...));
-    }
-};
 
 // r = b - A x, folds sum(r) into s->rsum
 __global__ void k_cg_residual(LevelView<double> A, const double* __restrict__ b, const double* __restrict__ x,
@@ -665,6 +614,11 @@ __global__ void k_ir_start(int n, const double* __restrict__ r, float* __restric
     }
 }
 
+// the loop is entered unless the set-up found nothing to solve
+__global__ void k_cg_gate(const CgState* s, cudaGraphConditionalHandle handle) {
+    cudaGraphSetConditional(handle, (s->flags & kCgHalt) ? 0u : 1u);
+}
+
 __global__ void k_cg_set(CgState* s, double target, int itmax) {
     pdl_entry();
     s->target = target;
@@ -815,8 +769,9 @@ void DeviceSolver::build_views() {
     TPA_CUDA(cudaMemsetAsync(lsum_.p, 0, size_t(nl + 2) * sizeof(double), stream_));
     cgs_.alloc(sizeof(CgState));
     TPA_CUDA(cudaMemsetAsync(cgs_.p, 0, sizeof(CgState), stream_));
-    spartial_.alloc(size_t(4) * size_t(kMaxGrid));
-    spres_.alloc(8);
+    spartial_.alloc(size_t(5) * size_t(kMaxGrid));
+    sstate_.alloc(sizeof(SolveState));
+    TPA_CUDA(cudaMemsetAsync(sstate_.p, 0, sizeof(SolveState), stream_));
     build_dense_tail();
     bar_.alloc(2);
     err_.alloc(1);
@@ -1230,8 +1185,16 @@ cudaGraphExec_t DeviceSolver::cg_graph(int precision) {
     cp.conditional.handle = handle;
     cp.conditional.type = cudaGraphCondTypeWhile;
     cp.conditional.size = 1;
-    cudaGraphNode_t node;
-    TPA_CUDA(cudaGraphAddNode(&node, g, nullptr, 0, &cp));
+    CgState* state = reinterpret_cast<CgState*>(cgs_.p);
+    void* gate_args[] = {&state, &handle};
+    cudaKernelNodeParams gate;
+    std::memset(&gate, 0, sizeof(gate));
+    gate.func = reinterpret_cast<void*>(k_cg_gate);
+    gate.gridDim = gate.blockDim = dim3(1);
+    gate.kernelParams = gate_args;
+    cudaGraphNode_t gate_node, node;
+    TPA_CUDA(cudaGraphAddKernelNode(&gate_node, g, nullptr, 0, &gate));
+    TPA_CUDA(cudaGraphAddNode(&node, g, &gate_node, 1, &cp));
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     cudaStream_t saved = stream_;
     stream_ = own_stream_;
@@ -1256,26 +1219,64 @@ cudaGraphExec_t DeviceSolver::cg_graph(int precision) {
     return exec;
 }
 
+// FP32 vectors of the refinement solve, allocated by its first run
+void DeviceSolver::ensure_ir() {
+    if (coop_grid_ > 0) throw Error(5, "the refinement solve runs the multi-launch V-cycle, not the cooperative one");
+    if (ir_.n == 4 * ir_stride()) return;
+    destroy_graphs();  // a captured body holds the old addresses
+    ir_.alloc(4 * ir_stride());
+    TPA_CUDA(cudaMemsetAsync(ir_.p, 0, ir_.n * sizeof(float), stream_));
+}
+
+// The loop bodies of one Krylov run whose state and residual are set; nothing
+// is read back.  With TPAGMG_NO_GRAPH the same iteration is launched kernel by
+// kernel and the stopping rules are read on the host (profiling and diagnosis).
+void DeviceSolver::cg_loop(int precision) {
+    const int n = levels_[0].n;
+    const Launch go{stream_, pdl_};
+    CgState* s = reinterpret_cast<CgState*>(cgs_.p);
+    cudaGraphExec_t exec = cg_graph(precision);
+    if (precision == 2) {
+        // an inner run of the refinement solve starts from the true residual
+        go(k_ir_start, fold_grid(k_ir_start, kThreads, blocks_for(n), kMaxGrid), kThreads, 0, n, (const double*)r_.p,
+           ir_.p, fpartial_.p, counters_.p + kCgRes, s);
+        ++launches_;
+    }
+    if (!std::getenv("TPAGMG_NO_GRAPH")) {
+        TPA_CUDA(cudaGraphLaunch(exec, stream_));
+        return;
+    }
+    CgState hs;
+    auto read = [&] {
+        TPA_CUDA(cudaMemcpyAsync(&hs, s, sizeof(CgState), cudaMemcpyDeviceToHost, stream_));
+        TPA_CUDA(cudaStreamSynchronize(stream_));
+    };
+    read();
+    bool stop = (hs.flags & kCgHalt) != 0;
+    while (!stop) {
+        const int before = launches_;
+        enqueue_cg_body(precision, cudaGraphConditionalHandle(), 0);
+        launches_ = before;  // counted from the iterations (count_cg_bodies)
+        read();
+        stop = (hs.flags & (kCgHalt | 1)) || hs.iter >= hs.itmax;
+    }
+}
+
+// Kernels of a finished run: every body ran all of its kernels; a body that
+// halted is not counted as an iteration.
+void DeviceSolver::count_cg_bodies(int precision, int iter, int flags) {
+    launches_ += (iter + ((flags & kCgHalt) ? 1 : 0)) * graph_body_launches_[precision];
+}
+
+// A run from the current xw_ and b_ (the plain solve's): the state, r = b - A x
+// and sum(r), then the loop.
 void DeviceSolver::cg_fused(int precision, double target, int itmax, int& niter, int& flags) {
     const int n = levels_[0].n;
     const Launch go{stream_, pdl_};
     CgState* s = reinterpret_cast<CgState*>(cgs_.p);
-    if (precision == 2) {
-        if (coop_grid_ > 0) throw Error(5, "the refinement solve runs the multi-launch V-cycle, not the cooperative one");
-        if (ir_.n != 4 * ir_stride()) {
-            destroy_graphs();  // a captured body holds the old addresses
-            ir_.alloc(4 * ir_stride());
-            TPA_CUDA(cudaMemsetAsync(ir_.p, 0, ir_.n * sizeof(float), stream_));
-        }
-    }
-    cudaGraphExec_t exec = cg_graph(precision);
-    // a run: the state, r = b - A x and sum(r); the loop bodies follow
+    if (precision == 2) ensure_ir();
     go(k_cg_set, 1, 1, 0, s, target, itmax);
-    if (precision == 2)
-        // an inner run of the refinement solve starts from the true residual
-        go(k_ir_start, fold_grid(k_ir_start, kThreads, blocks_for(n), kMaxGrid), kThreads, 0, n, (const double*)r_.p,
-           ir_.p, fpartial_.p, counters_.p + kCgRes, s);
-    else if (sdev_[0].vec)
+    if (sdev_[0].vec)
         go(v_cg_residual, fold_grid(v_cg_residual, 256, (sd_[0].nblocks + 3) / 4, kMaxGrid), 256, 0, sd_[0], b_.p, xw_.p, r_.p,
            fpartial_.p, counters_.p + kCgRes, s);
     else if (sdev_[0].on)
@@ -1290,25 +1291,11 @@ void DeviceSolver::cg_fused(int precision, double target, int itmax, int& niter,
     launches_ += 2;
     CgState hs;
     std::memset(&hs, 0, sizeof(hs));
-    if (itmax > 0 && std::getenv("TPAGMG_NO_GRAPH")) {
-        // the same iteration launched kernel by kernel, stopping rules read on
-        // the host after each one (profiling and diagnosis)
-        bool stop = false;
-        while (!stop) {
-            const int before = launches_;
-            enqueue_cg_body(precision, cudaGraphConditionalHandle(), 0);
-            launches_ = before + graph_body_launches_[precision];
-            TPA_CUDA(cudaMemcpyAsync(&hs, s, sizeof(CgState), cudaMemcpyDeviceToHost, stream_));
-            TPA_CUDA(cudaStreamSynchronize(stream_));
-            stop = (hs.flags & (kCgHalt | 1)) || hs.iter >= hs.itmax;
-        }
-    } else if (itmax > 0) {
-        TPA_CUDA(cudaGraphLaunch(exec, stream_));
+    if (itmax > 0) {
+        cg_loop(precision);
         TPA_CUDA(cudaMemcpyAsync(&hs, s, sizeof(CgState), cudaMemcpyDeviceToHost, stream_));
         TPA_CUDA(cudaStreamSynchronize(stream_));
-        // every body ran its kernels; a body that halted is not counted
-        const int bodies = hs.iter + ((hs.flags & kCgHalt) ? 1 : 0);
-        launches_ += bodies * graph_body_launches_[precision];
+        count_cg_bodies(precision, hs.iter, hs.flags);
     }
     TPA_CUDA(cudaGetLastError());
     niter = hs.iter;
