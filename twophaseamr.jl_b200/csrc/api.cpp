@@ -594,10 +594,8 @@ tpa_status tpa_refresh_device(tpa_context* ctx, const double* face_coefficient) 
         const size_t nf = kappa.size();
         cudaStream_t s = ctx->dev->stream();
         if (!std::getenv("TPAGMG_HOST_REFRESH") && ctx->dev->refresh_applicable(ctx->hier) &&
-            ctx->dev->refresh_from_device(ctx->hier, face_coefficient) == 0) {
             // the host keeps the finest coefficients (the rest is recomputed on demand)
-            TPA_CUDA(cudaMemcpyAsync(kappa.data(), face_coefficient, nf * sizeof(double), cudaMemcpyDeviceToHost, s));
-            TPA_CUDA(cudaStreamSynchronize(s));
+            ctx->dev->refresh_from_device(ctx->hier, face_coefficient, kappa) == 0) {
             ctx->host_stale = true;
             stamp(2);
             return;

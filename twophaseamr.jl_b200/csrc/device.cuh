@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <cstdint>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -277,6 +278,7 @@ private:
     std::vector<LevelView<float>> vf_;
     DevArray<LevelView<double>> vd_dev_;
     DevArray<LevelView<float>> vf_dev_;
+    DevArray<double> wts_;  // w, tw and rbw of every level (LevelView::wt)
     DevArray<double> fpartial_, fpartial2_, lsum_, xw_;
     DevArray<unsigned> counters_;
     DevArray<char> cgs_;  // CgState
@@ -351,7 +353,8 @@ public:
     // The same from a device array: 0 when refreshed, 1 when the set of zero
     // coefficients differs from the current one (nothing changed; the host
     // path must rebuild); throws on a non-finite or negative coefficient.
-    int refresh_from_device(const Hierarchy& h, const double* kappa_dev);
+    // `kappa_host` receives the coefficients.
+    int refresh_from_device(const Hierarchy& h, const double* kappa_dev, std::vector<double>& kappa_host);
     // smoother and transfer weight per level, as uploaded or refreshed
     std::vector<double> level_weights();
 
@@ -367,13 +370,21 @@ private:
         DevArray<int> sx, sy, sex;
     };
     void prepare_refresh(const Hierarchy& h);
-    void refresh_levels();  // from the finest coefficients in rl_[0].kappa
+    // from the finest coefficients in rl_[0].kappa
+    void refresh_levels(const std::function<void()>& meanwhile);
+    std::vector<double> kappa_next_;  // the host's next finest coefficients
     std::vector<RefreshLevel> rl_;
     bool rl_ready_ = false;
     int coarse_N_ = 0, coarse_ncomp_ = 0;
     bool lu_cluster_ = false;  // coarse LU on a cluster with the rows in shared memory
     double* rstage_ = nullptr; // pinned staging of the finest-level coefficients
-    DevArray<double> coarse_M_, coarse_MT_, rwtw_, rpart_;
+    void coarse_inverse_lu();
+    void finish_refresh(const std::function<void()>& meanwhile);
+    bool refresh_lu_ = false;  // the coarse inverse by the pivoted LU at once
+    DevArray<double> coarse_shift_;
+    double* host_wtw_ = nullptr;  // in rstage_'s allocation: the weights and the error word read back
+    int* host_rerr_ = nullptr;
+    DevArray<double> coarse_M_, coarse_MT_, rpart_;
     DevArray<int> coarse_piv_, rerr_;
     DevArray<unsigned> rcnt_;
 

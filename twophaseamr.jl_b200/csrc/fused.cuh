@@ -70,7 +70,8 @@ struct LevelView {
     const int* owner;
     const int* cptr;
     const int* child;
-    T w, tw;
+    T w, tw;           // smoother and transfer weight: with_weights fills them in
+    const double* wt;  // the level's weights on the device (w, tw, rbw), rewritten by a refresh
     int singular;      // ungauged component present (one)
     double cvol_inv;   // 1 / component volume
     T* b;              // restricted right-hand side (raw)
@@ -87,6 +88,16 @@ struct LevelView {
     // sum rows as a_ij (x_j - x_i), add it back as bdiag_i x_i.
     const double* bdiag;
 };
+
+// The view with its weights loaded.  They live in device memory so that a
+// coefficient refresh, which recomputes them, leaves captured graphs valid.
+template <typename T>
+__device__ __forceinline__ LevelView<T> with_weights(LevelView<T> L) {
+    L.w = T(__ldg(L.wt));
+    L.tw = T(__ldg(L.wt + 1));
+    L.rbw = T(__ldg(L.wt + 2));
+    return L;
+}
 
 // fold partial[0..count) in fixed order by one block; returns the sum in thread 0
 __device__ __forceinline__ double fold_partials(const double* partial, int count) {
@@ -338,6 +349,7 @@ __device__ __forceinline__ void rb_pair_cell(const LevelView<T>& L, const T* in,
 template <typename T, typename TB>
 __global__ void k_pre2(LevelView<T> L, const TB* __restrict__ b, const double* level_sum) {
     pdl_entry();
+    L = with_weights(L);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     double mean = (L.singular && level_sum) ? *level_sum * L.cvol_inv : 0.0;
     if (i < L.n) pre2_cell<T, TB>(L, b, mean, i);
@@ -349,6 +361,7 @@ template <typename T>
 __global__ void k_rb_half(LevelView<T> L, const T* __restrict__ in, T* __restrict__ out, int c, double* partial,
                           unsigned* counter, double* mean_out) {
     pdl_entry();
+    L = with_weights(L);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     double v = 0;
     if (i < L.n) {
@@ -370,6 +383,7 @@ __global__ void k_rb_half(LevelView<T> L, const T* __restrict__ in, T* __restric
 template <typename T, typename TB>
 __global__ void k_rb_pre(LevelView<T> L, const TB* __restrict__ b, const double* level_sum, T* out) {
     pdl_entry();
+    L = with_weights(L);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     double mean = (L.singular && level_sum) ? *level_sum * L.cvol_inv : 0.0;
     if (i < L.n) rb_first_cell<T, TB>(L, b, mean, out, i);
@@ -381,6 +395,7 @@ template <typename T>
 __global__ void k_rb_pair(LevelView<T> L, const T* __restrict__ in, T* __restrict__ out, int c, double* partial,
                           unsigned* counter, double* mean_out) {
     pdl_entry();
+    L = with_weights(L);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     double v = 0;
     if (i < L.n) {
@@ -409,6 +424,7 @@ __global__ void k_residual(LevelView<T> L) {
 template <typename T>
 __global__ void k_restrict(LevelView<T> L, T* __restrict__ bc) {
     pdl_entry();
+    L = with_weights(L);
     // grid-stride over whole warps (the shuffles need every lane of a warp)
     const int quads = (4 * L.nc + 31) & ~31;
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < quads; g += gridDim.x * blockDim.x) {
@@ -427,6 +443,7 @@ __global__ void k_restrict(LevelView<T> L, T* __restrict__ bc) {
 template <typename T>
 __global__ void k_resrest(LevelView<T> L, T* __restrict__ bc) {
     pdl_entry();
+    L = with_weights(L);
     const int quads = (4 * L.nc + 31) & ~31;
     for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < quads; g += gridDim.x * blockDim.x) {
         const int J = g >> 2, q = g & 3;
@@ -454,6 +471,7 @@ __global__ void k_resrest(LevelView<T> L, T* __restrict__ bc) {
 template <typename T>
 __global__ void k_prolong(LevelView<T> L, const T* __restrict__ xc) {
     pdl_entry();
+    L = with_weights(L);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < L.n) prolong_cell(L, xc, i);
 }
@@ -462,6 +480,7 @@ __global__ void k_prolong(LevelView<T> L, const T* __restrict__ xc) {
 template <typename T>
 __global__ void k_post1(LevelView<T> L) {
     pdl_entry();
+    L = with_weights(L);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < L.n) sweep_cell(L, L.x, L.y, i);
 }
@@ -470,6 +489,7 @@ __global__ void k_post1(LevelView<T> L) {
 template <typename T, typename Epi = MeanOnly>
 __global__ void k_post2(LevelView<T> L, double* partial, unsigned* counter, double* mean_out, Epi epi = Epi()) {
     pdl_entry();
+    L = with_weights(L);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     double v = 0, w = 0;
     if (i < L.n) {
@@ -528,7 +548,7 @@ __device__ void tail_run(const LevelView<T>* __restrict__ levels, int first, int
     const int rank = int(cl.block_rank()), nb = int(cl.num_blocks());
     const int gt = rank * blockDim.x + threadIdx.x, gs = nb * blockDim.x;
     for (int l = first; l < nl; ++l) {
-        LevelView<T> L = levels[l];
+        const LevelView<T> L = with_weights(levels[l]);
         const bool top = (l == 0);  // only the finest level reads the caller's RHS
         double mean = 0;
         if (L.singular) {
@@ -580,7 +600,7 @@ __device__ void tail_run(const LevelView<T>* __restrict__ levels, int first, int
         cl.sync();
     }
     for (int l = nl - 2; l >= first; --l) {
-        LevelView<T> L = levels[l];
+        const LevelView<T> L = with_weights(levels[l]);
         const T* xc = levels[l + 1].x;
         for (int i = gt; i < L.n; i += gs) prolong_cell(L, xc, i);
         cl.sync();

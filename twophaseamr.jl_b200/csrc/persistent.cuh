@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(kTailThreads, 1)
     pdl_entry();
     const int gt = blockIdx.x * blockDim.x + threadIdx.x, gs = gridDim.x * blockDim.x;
     for (int l = 0; l < t; ++l) {
-        const LevelView<T> L = levels[l];
+        const LevelView<T> L = with_weights(levels[l]);
         double mean = 0;
         if (L.singular) mean = (l == 0 ? *rsum : __ldcg(lsum + l)) * L.cvol_inv;
         if (l == 0)
@@ -102,7 +102,7 @@ __global__ void __launch_bounds__(kTailThreads, 1)
                             t == 0 && levels[0].singular ? mean_out : nullptr);
     grid_barrier(bar, err, spins);
     for (int l = t - 1; l >= 0; --l) {
-        const LevelView<T> L = levels[l];
+        const LevelView<T> L = with_weights(levels[l]);
         const T* xc = levels[l + 1].x;
         for (int i = gt; i < L.n; i += gs) prolong_cell(L, xc, i);
         grid_barrier(bar, err, spins);

@@ -141,13 +141,33 @@ __global__ void kr_weights(int n, const int* __restrict__ rp, const int* __restr
         last = atomicAdd(counter, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (last && threadIdx.x == 0) {
-        __threadfence();
-        double ms = 0.0, mt = 0.0, mr = 0.0;
-        for (unsigned b = 0; b < gridDim.x; ++b) {
-            ms = fmax(ms, ((volatile double*)partial)[b]);
-            mt = fmax(mt, ((volatile double*)partial)[gridDim.x + b]);
-            mr = fmax(mr, ((volatile double*)partial)[2 * gridDim.x + b]);
+    if (!last) return;
+    __threadfence();
+    // every thread takes its share of the block maxima, then the block's tree
+    // (one thread reading them in turn took 50 us behind 430 blocks)
+    double ms = 0.0, mt = 0.0, mr = 0.0;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) {
+        ms = fmax(ms, ((volatile double*)partial)[b]);
+        mt = fmax(mt, ((volatile double*)partial)[gridDim.x + b]);
+        mr = fmax(mr, ((volatile double*)partial)[2 * gridDim.x + b]);
+    }
+    for (int o = 16; o; o >>= 1) {
+        ms = fmax(ms, __shfl_down_sync(0xffffffffu, ms, o));
+        mt = fmax(mt, __shfl_down_sync(0xffffffffu, mt, o));
+        mr = fmax(mr, __shfl_down_sync(0xffffffffu, mr, o));
+    }
+    if (!lane) {
+        sh[0][wid] = ms;
+        sh[1][wid] = mt;
+        sh[2][wid] = mr;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        ms = mt = mr = 0.0;
+        for (int w = 0; w < int(blockDim.x >> 5); ++w) {
+            ms = fmax(ms, sh[0][w]);
+            mt = fmax(mt, sh[1][w]);
+            mr = fmax(mr, sh[2][w]);
         }
         wtw[0] = ms == 0.0 ? 1.0 : fmin(1.0, 4.0 / (3.0 * ms));
         wtw[1] = mt == 0.0 ? 0.0 : 4.0 / (3.0 * mt);
@@ -195,6 +215,135 @@ __global__ void kr_coarse_fill(int n, int N, const int* __restrict__ rp, const i
         }
     }
 }
+
+// ---- the coarse inverse by block elimination ------------------------------------
+//
+// The coarse solve needs the n x n block G of [A v; v' 0]^-1 (v: the volumes, one
+// column per ungauged component).  A is symmetric, its null space is the
+// components' constants, so B = A + sum_s c_s v_s v_s' is positive definite and
+//   G = B^-1 - sum_s 1_s 1_s' / (c_s (1'v_s)^2)
+// (B 1_s = c_s (1'v_s) v_s, and the multiplier of the augmented system is
+// 1'b / 1'v).  c_s = d n_s / (1'v_s)^2, d the component's mean diagonal, puts the
+// added eigenvalue among A's.  B^-1 is formed in place by Gauss-Jordan
+// elimination over blocks of 32 rows, which needs no pivoting for a positive
+// definite matrix: ceil(n / 32) launches, each over all 32 x 32 tiles.
+// Measured at n = 256: 8 launches in place of 257 dependent pivot steps in one
+// cluster (724 us) and the triangular solves (132 us).  A block whose pivots are
+// not positive (B singular to working precision) sets err 3, and the refresh
+// takes the pivoted LU of the augmented matrix below instead.
+
+constexpr int kGj = 32;
+
+// B (row-major n x n) and shift[s] = 1 / (c_s (1'v_s)^2); a warp per row
+__global__ void kr_coarse_spd(int n, const int* __restrict__ rp, const int* __restrict__ ci,
+                              const double* __restrict__ val, const int* __restrict__ slot,
+                              const double* __restrict__ vol, int ncomp, double* __restrict__ B,
+                              double* __restrict__ shift) {
+    __shared__ double c[kMaxComponents];
+    for (int s = 0; s < ncomp; ++s) {
+        double tr = 0, cells = 0, vs = 0;
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            if (slot[i] != s) continue;
+            cells += 1;
+            vs += vol[i];
+            for (int k = rp[i]; k < rp[i + 1]; ++k)
+                if (ci[k] == i) tr += val[k];
+        }
+        tr = block_sum_all(tr);
+        cells = block_sum_all(cells);
+        vs = block_sum_all(vs);
+        if (threadIdx.x == 0) {
+            // an isolated component (no couplings) takes a unit diagonal
+            const double d = tr > 0 ? tr : cells;  // mean diagonal times cells
+            c[s] = d / (vs * vs);
+            if (blockIdx.x == 0) shift[s] = 1.0 / d;
+        }
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += (gridDim.x * blockDim.x) >> 5) {
+        double* row = B + size_t(r) * n;
+        const int s = ncomp ? slot[r] : -1;
+        const double cv = s >= 0 ? c[s] * vol[r] : 0.0;
+        for (int j = lane; j < n; j += 32) row[j] = (s >= 0 && slot[j] == s) ? cv * vol[j] : 0.0;
+        __syncwarp();
+        for (int k = rp[r] + lane; k < rp[r + 1]; k += 32) row[ci[k]] += val[k];
+    }
+}
+
+// One block step: with D the diagonal block kb of `in`, C its block column and
+// R its block row,  out = D^-1 at (kb, kb), D^-1 R in row kb, -C D^-1 in column
+// kb, in - C D^-1 R elsewhere.  One CTA per tile of `out`; each inverts D in
+// shared memory (rows beyond n: the identity).  On the last step the tiles are
+// stored as G, less the components' shift.
+__global__ void __launch_bounds__(256) kr_gj_step(int n, int kb, const double* __restrict__ in,
+                                                  double* __restrict__ out, int last, const int* __restrict__ slot,
+                                                  int ncomp, const double* __restrict__ shift, int* err) {
+    __shared__ double D[kGj][kGj + 1], C[kGj][kGj + 1], R[kGj][kGj + 1];
+    const int ti = blockIdx.y, tj = blockIdx.x;
+    const int r = threadIdx.x >> 3, q = threadIdx.x & 7;  // this thread's row and columns q, q + 8, q + 16, q + 24
+    auto load = [&](int bi, int bj, int u) {
+        const int i = bi * kGj + r, j = bj * kGj + q + 8 * u;
+        return i < n && j < n ? in[size_t(i) * n + j] : (bi == bj && i == j ? 1.0 : 0.0);
+    };
+    double own[4];
+    for (int u = 0; u < 4; ++u) {
+        D[r][q + 8 * u] = load(kb, kb, u);
+        C[r][q + 8 * u] = load(ti, kb, u);
+        R[r][q + 8 * u] = load(kb, tj, u);
+        own[u] = load(ti, tj, u);
+    }
+    // D^-1 in place, pivot by pivot: row p scaled by 1 / d_pp, the rest updated
+    // with the old column p, which becomes -d_ip / d_pp
+    bool bad = false;
+    for (int p = 0; p < kGj; ++p) {
+        __syncthreads();
+        const double piv = D[p][p], f = D[r][p];
+        double row[4];
+        for (int u = 0; u < 4; ++u) row[u] = D[p][q + 8 * u];
+        bad = bad || !(piv > 0.0);
+        const double inv = 1.0 / piv;
+        __syncthreads();
+        for (int u = 0; u < 4; ++u) {
+            const int j = q + 8 * u;
+            if (r == p) D[r][j] = j == p ? inv : row[u] * inv;
+            else D[r][j] = j == p ? -f * inv : D[r][j] - f * inv * row[u];
+        }
+    }
+    __syncthreads();
+    if (bad && threadIdx.x == 0 && ti == kb && tj == kb) atomicCAS(err, 0, 3);
+    double o[4];
+    if (ti == kb && tj == kb) {
+        for (int u = 0; u < 4; ++u) o[u] = D[r][q + 8 * u];
+    } else if (tj == kb) {
+        for (int u = 0; u < 4; ++u) o[u] = 0;
+        for (int k = 0; k < kGj; ++k)
+            for (int u = 0; u < 4; ++u) o[u] -= C[r][k] * D[k][q + 8 * u];
+    } else {
+        double w[4] = {0, 0, 0, 0};
+        for (int k = 0; k < kGj; ++k)
+            for (int u = 0; u < 4; ++u) w[u] += D[r][k] * R[k][q + 8 * u];
+        if (ti == kb) {
+            for (int u = 0; u < 4; ++u) o[u] = w[u];
+        } else {
+            __syncthreads();
+            for (int u = 0; u < 4; ++u) R[r][q + 8 * u] = w[u];
+            __syncthreads();
+            for (int u = 0; u < 4; ++u) o[u] = own[u];
+            for (int k = 0; k < kGj; ++k)
+                for (int u = 0; u < 4; ++u) o[u] -= C[r][k] * R[k][q + 8 * u];
+        }
+    }
+    const int i = ti * kGj + r;
+    for (int u = 0; u < 4; ++u) {
+        const int j = tj * kGj + q + 8 * u;
+        if (i >= n || j >= n) continue;
+        if (last && ncomp && slot[i] >= 0 && slot[i] == slot[j]) o[u] -= shift[slot[i]];
+        out[size_t(i) * n + j] = o[u];
+    }
+}
+
+// ---- the pivoted LU of the augmented matrix --------------------------------------
 
 // (value, row) pairs: the larger value wins, ties go to the smaller row (the
 // first maximum of a sequential scan)
@@ -635,10 +784,15 @@ void DeviceSolver::prepare_refresh(const Hierarchy& h) {
         TPA_CUDA(cudaFuncSetAttribute(kr_coarse_inv, cudaFuncAttributeMaxDynamicSharedMemorySize, int(inv_bytes)));
     }
     coarse_piv_.alloc(size_t(coarse_N_));
+    // pinned: the staged coefficients, the weights read back, an error word
     if (rstage_) cudaFreeHost(rstage_);
     rstage_ = nullptr;
-    TPA_CUDA(cudaMallocHost(&rstage_, sizeof(double) * std::max<size_t>(1, size_t(rl_[0].nf))));
-    rwtw_.alloc(size_t(3 * nl));
+    const size_t stage = std::max<size_t>(1, size_t(rl_[0].nf)) + size_t(3 * nl);
+    TPA_CUDA(cudaMallocHost(&rstage_, sizeof(double) * (stage + 1)));
+    host_wtw_ = rstage_ + std::max<size_t>(1, size_t(rl_[0].nf));
+    host_rerr_ = reinterpret_cast<int*>(rstage_ + stage);
+    coarse_shift_.alloc(size_t(kMaxComponents));
+    refresh_lu_ = std::getenv("TPAGMG_REFRESH_LU") != nullptr;  // the pivoted LU at once (diagnosis)
     rpart_.alloc(size_t(3 * 1184));
     rcnt_.alloc(1);
     rerr_.alloc(1);
@@ -668,27 +822,36 @@ void DeviceSolver::refresh_on_device(const Hierarchy& h, const double* kappa_hos
     std::memcpy(rstage_, kappa_host, sizeof(double) * size_t(rl_[0].nf));  // no copy is in flight here
     TPA_CUDA(cudaMemcpyAsync(rl_[0].kappa.p, rstage_, sizeof(double) * size_t(rl_[0].nf), cudaMemcpyHostToDevice,
                              stream_));
-    refresh_levels();
+    refresh_levels({});
 }
 
-int DeviceSolver::refresh_from_device(const Hierarchy& h, const double* kappa_dev) {
+int DeviceSolver::refresh_from_device(const Hierarchy& h, const double* kappa_dev, std::vector<double>& kappa_host) {
     TPA_CUDA(cudaSetDevice(device_));
     if (!rl_ready_) prepare_refresh(h);
     const int nf = rl_[0].nf;
-    int flags = 0;
     TPA_CUDA(cudaMemsetAsync(rerr_.p, 0, sizeof(int), stream_));
     if (nf > 0) kr_check<<<rgrid(nf), kRThreads, 0, stream_>>>(nf, kappa_dev, rl_[0].kappa.p, rerr_.p);
-    TPA_CUDA(cudaMemcpyAsync(&flags, rerr_.p, sizeof(int), cudaMemcpyDeviceToHost, stream_));
+    TPA_CUDA(cudaMemcpyAsync(host_rerr_, rerr_.p, sizeof(int), cudaMemcpyDeviceToHost, stream_));
     TPA_CUDA(cudaStreamSynchronize(stream_));
+    const int flags = *host_rerr_;
     if (flags & 1) throw Error(1, "face coefficients must be finite and nonnegative");
     if (flags & 2) return 1;
+    // the host's copy goes through the pinned stage, emptied while the refresh runs
+    TPA_CUDA(cudaMemcpyAsync(rstage_, kappa_dev, sizeof(double) * size_t(nf), cudaMemcpyDeviceToHost, stream_));
+    TPA_CUDA(cudaEventRecord(ev0_, stream_));
     TPA_CUDA(cudaMemcpyAsync(rl_[0].kappa.p, kappa_dev, sizeof(double) * size_t(nf), cudaMemcpyDeviceToDevice,
                              stream_));
-    refresh_levels();
+    kappa_next_.resize(size_t(nf));
+    refresh_levels([&] {
+        TPA_CUDA(cudaEventSynchronize(ev0_));
+        std::memcpy(kappa_next_.data(), rstage_, sizeof(double) * size_t(nf));
+    });
+    kappa_host.swap(kappa_next_);
     return 0;
 }
 
-void DeviceSolver::refresh_levels() {
+// `meanwhile` (may be empty): host work for the time the kernels take
+void DeviceSolver::refresh_levels(const std::function<void()>& meanwhile) {
     const int nl = int(levels_.size());
     cudaStream_t s = stream_;
     TPA_CUDA(cudaMemsetAsync(rerr_.p, 0, sizeof(int), s));
@@ -714,8 +877,59 @@ void DeviceSolver::refresh_levels() {
                                                    rb_ ? L.colour.p : nullptr,
                                                    L.d.dinv.p, L.f.dinv.p, l + 1 < nl ? L.d.tinv.p : nullptr,
                                                    l + 1 < nl ? L.f.tinv.p : nullptr, rpart_.p, rcnt_.p,
-                                                   rwtw_.p + 3 * l, rerr_.p);
+                                                   wts_.p + 3 * l, rerr_.p);
     }
+    const DevLevel& C = levels_.back();
+    if (refresh_lu_) {
+        coarse_inverse_lu();
+    } else {
+        const int nb = (C.n + kGj - 1) / kGj;
+        kr_coarse_spd<<<std::min(148, (C.n + 7) / 8), 256, 0, s>>>(C.n, C.rowptr.p, C.col.p, C.d.val.p, C.slot.p,
+                                                                   C.d.vol.p, coarse_ncomp_, coarse_M_.p,
+                                                                   coarse_shift_.p);
+        const double* in = coarse_M_.p;
+        for (int kb = 0; kb < nb; ++kb) {
+            const bool last = kb == nb - 1;
+            double* out = last ? coarse_inv_.p : in == coarse_M_.p ? coarse_MT_.p : coarse_M_.p;
+            kr_gj_step<<<dim3(nb, nb), 256, 0, s>>>(C.n, kb, in, out, last ? 1 : 0, C.slot.p, coarse_ncomp_,
+                                                    coarse_shift_.p, rerr_.p);
+            in = out;
+        }
+    }
+    finish_refresh(meanwhile);
+    if (*host_rerr_ == 3) {  // the elimination met a pivot that is not positive
+        TPA_CUDA(cudaMemsetAsync(rerr_.p, 0, sizeof(int), s));
+        coarse_inverse_lu();
+        finish_refresh({});
+    }
+    if (*host_rerr_ == 1) throw Error(1, "elliptic matrix has a non-positive diagonal");
+    if (*host_rerr_ == 2) throw Error(1, "coarsest multigrid matrix is singular");
+    for (int l = 0; l < nl; ++l) {
+        DevLevel& L = levels_[size_t(l)];
+        const double* w = host_wtw_ + 3 * l;
+        L.d.w = w[0];
+        L.f.w = float(w[0]);
+        if (l + 1 < nl) {
+            L.d.tw = w[1];
+            L.f.tw = float(w[1]);
+        }
+        if (rb_) L.rbw = w[2];
+        if (size_t(l) < sd_.size()) {
+            sd_[size_t(l)].w = L.d.w;
+            sf_[size_t(l)].w = L.f.w;
+            sd_[size_t(l)].tw = L.d.tw;
+            sf_[size_t(l)].tw = L.f.tw;
+        }
+    }
+    // the captured graphs read every refreshed value from device memory (the
+    // level weights too, LevelView::wt); only stencil levels hold weights in
+    // their kernels' arguments
+    if (structured_levels() > 0) destroy_graphs();
+}
+
+// G from the pivoted LU of the augmented coarsest matrix
+void DeviceSolver::coarse_inverse_lu() {
+    cudaStream_t s = stream_;
     const DevLevel& C = levels_.back();
     TPA_CUDA(cudaMemsetAsync(coarse_M_.p, 0, sizeof(double) * coarse_M_.n, s));
     kr_coarse_fill<<<rgrid(C.n), kRThreads, 0, s>>>(C.n, coarse_N_, C.rowptr.p, C.col.p, C.d.val.p,
@@ -746,49 +960,24 @@ void DeviceSolver::refresh_levels() {
     }
     kr_coarse_inv<<<(C.n + kInvWarps - 1) / kInvWarps, 32 * kInvWarps, inv_smem(N), s>>>(
         N, C.n, coarse_MT_.p, coarse_piv_.p, coarse_inv_.p, rerr_.p);
-    TPA_CUDA(cudaGetLastError());
-    std::vector<double> wtw(size_t(3 * nl));
-    int err = 0;
-    TPA_CUDA(cudaMemcpyAsync(wtw.data(), rwtw_.p, sizeof(double) * wtw.size(), cudaMemcpyDeviceToHost, s));
-    TPA_CUDA(cudaMemcpyAsync(&err, rerr_.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-    TPA_CUDA(cudaStreamSynchronize(s));
-    if (err == 1) throw Error(1, "elliptic matrix has a non-positive diagonal");
-    if (err == 2) throw Error(1, "coarsest multigrid matrix is singular");
-    for (int l = 0; l < nl; ++l) {
-        DevLevel& L = levels_[size_t(l)];
-        L.d.w = wtw[size_t(3 * l)];
-        L.f.w = float(L.d.w);
-        if (l + 1 < nl) {
-            L.d.tw = wtw[size_t(3 * l + 1)];
-            L.f.tw = float(L.d.tw);
-        }
-        if (rb_) {
-            L.rbw = wtw[size_t(3 * l + 2)];
-            vd_[size_t(l)].rbw = L.rbw;
-            vf_[size_t(l)].rbw = float(L.rbw);
-        }
-        vd_[size_t(l)].w = L.d.w;
-        vf_[size_t(l)].w = L.f.w;
-        vd_[size_t(l)].tw = L.d.tw;
-        vf_[size_t(l)].tw = L.f.tw;
-        if (size_t(l) < sd_.size()) {
-            sd_[size_t(l)].w = L.d.w;
-            sf_[size_t(l)].w = L.f.w;
-            sd_[size_t(l)].tw = L.d.tw;
-            sf_[size_t(l)].tw = L.f.tw;
-        }
-    }
-    // the level views (and the captured graphs, which hold them by value) change
-    vd_dev_.upload(vd_.data(), vd_.size(), s);
-    vf_dev_.upload(vf_.data(), vf_.size(), s);
+}
+
+// What follows the coarse inverse -- the tail's map, the tile copies, the face
+// kernels' sqrt(kappa) -- and the weights and error flag read back, under one
+// synchronization.
+void DeviceSolver::finish_refresh(const std::function<void()>& meanwhile) {
+    cudaStream_t s = stream_;
     build_dense_tail();
-    // the face kernels' sqrt(kappa) (same faces, same zero set)
+    gather_tile_values();
+    // same faces, same zero set
     if (nfaces_ >= 0 && rl_[0].nf > 0)
         TPA_CUDA(cudaMemcpyAsync(f_sqrtk_.p, rl_[0].sk.p, sizeof(double) * size_t(rl_[0].nf), cudaMemcpyDeviceToDevice,
                                  s));
+    TPA_CUDA(cudaMemcpyAsync(host_wtw_, wts_.p, sizeof(double) * wts_.n, cudaMemcpyDeviceToHost, s));
+    TPA_CUDA(cudaMemcpyAsync(host_rerr_, rerr_.p, sizeof(int), cudaMemcpyDeviceToHost, s));
+    TPA_CUDA(cudaGetLastError());
+    if (meanwhile) meanwhile();
     TPA_CUDA(cudaStreamSynchronize(s));
-    gather_tile_values();  // the tile copies of the refreshed level values
-    destroy_graphs();
 }
 
 std::vector<double> DeviceSolver::level_weights() {

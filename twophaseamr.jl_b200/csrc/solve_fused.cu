@@ -720,6 +720,10 @@ void DeviceSolver::build_views() {
     for (int l = nl - 1; l >= 0; --l)
         if (levels_[size_t(l)].n <= tail_cells) tail_first_ = l;
         else break;
+    std::vector<double> wts;
+    for (const DevLevel& L : levels_) wts.insert(wts.end(), {L.d.w, L.d.tw, L.rbw});
+    if (wts_.n != wts.size()) wts_.alloc(wts.size());
+    TPA_CUDA(cudaMemcpyAsync(wts_.p, wts.data(), wts.size() * sizeof(double), cudaMemcpyHostToDevice, stream_));
     int64_t maxgrid = 1;
     for (int l = 0; l < nl; ++l) {
         DevLevel& L = levels_[size_t(l)];
@@ -738,8 +742,7 @@ void DeviceSolver::build_views() {
             v.owner = L.owner.p;
             v.cptr = L.child_ptr.p;
             v.child = L.child.p;
-            v.w = D.w;
-            v.tw = D.tw;
+            v.wt = wts_.p + 3 * l;
             v.singular = L.ncomp == 1;
             v.cvol_inv = L.ncomp == 1 ? 1.0 / L.comp_volume[0] : 0.0;
             v.b = D.b.p;
@@ -750,7 +753,6 @@ void DeviceSolver::build_views() {
             v.s = D.s.p;
             v.colour = L.colour.p;
             v.rb = rb_ ? 1 : 0;
-            v.rbw = static_cast<decltype(v.w)>(L.rbw);
             v.bdiag = nullptr;
         };
         fill(vd_[size_t(l)], L.d);
@@ -1582,6 +1584,7 @@ void DeviceSolver::upload_tiles(const Hierarchy& h) {
     allow_tile_up_smem<double, CgRz>(up_d);
     allow_tile_up_smem<float, CgRz>(up_d);
     gather_tile_values();
+    TPA_CUDA(cudaStreamSynchronize(stream_));
     destroy_graphs();
 }
 
@@ -1595,7 +1598,6 @@ void DeviceSolver::gather_tile_values() {
         k_tile_gather<float><<<g, kThreads, 0, stream_>>>(D.nent, D.pos.p, L.f.val.p, D.val_f.p);
     }
     TPA_CUDA(cudaGetLastError());
-    TPA_CUDA(cudaStreamSynchronize(stream_));
 }
 
 int DeviceSolver::streamed_levels() const {

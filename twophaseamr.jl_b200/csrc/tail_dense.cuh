@@ -79,7 +79,7 @@ __global__ void __launch_bounds__(kDenseBuildThreads)
     for (int e = tid; e < n0 * C; e += nt) bp[e] = (e / C == col0 + e % C) ? 1.0 : 0.0;
     __syncthreads();
     for (int l = first;; ++l) {
-        const LevelView<double> L = levels[l];
+        const LevelView<double> L = with_weights(levels[l]);
         double* x = bp + size_t(L.n) * C;
         if (L.singular) {
             means(bp, nullptr, L.n, L.cvol_inv);
@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(kDenseBuildThreads)
         bp = bc;
     }
     for (int l = nl - 2; l >= first; --l) {
-        const LevelView<double> L = levels[l];
+        const LevelView<double> L = with_weights(levels[l]);
         const double* xc = bp + size_t(levels[l + 1].n) * C;
         bp -= 2 * size_t(L.n) * C;
         double* x = bp + size_t(L.n) * C;

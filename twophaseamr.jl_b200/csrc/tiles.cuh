@@ -123,6 +123,7 @@ __global__ void __launch_bounds__(NT)
     k_tile_down(LevelView<T> L, TileView<T> V, const TB* __restrict__ b, const double* level_sum,
                 T* __restrict__ bc, T* bp_out) {
     pdl_launch();
+    L = with_weights(L);
     extern __shared__ __align__(16) unsigned char tile_smem[];
     T* bp = reinterpret_cast<T*>(tile_smem);
     T* dv = bp + V.n3max;
@@ -230,6 +231,7 @@ __global__ void __launch_bounds__(NT)
     k_tile_up(LevelView<T> L, TileView<T> V, const T* __restrict__ xc, const T* __restrict__ bp_in, double* partial, unsigned* counter,
               double* mean_out, Epi epi) {
     pdl_launch();
+    L = with_weights(L);
     extern __shared__ __align__(16) unsigned char tile_smem[];
     T* e = reinterpret_cast<T*>(tile_smem);
     T* xp = e + V.n3max;

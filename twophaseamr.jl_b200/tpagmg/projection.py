@@ -199,9 +199,14 @@ def project_device(u_interior, u_boundary, pressure, solver, dt, *, tolerance=DE
 
 def refresh_device(solver, kappa):
     """`_refresh_geometric_multigrid!` from device face coefficients."""
+    torch = _torch()
     _sync_stream(solver)
+    # the operator's host copy: into page-locked memory on the same stream, so
+    # that the refresh's own synchronization completes it
+    host = torch.empty(kappa.shape, dtype=kappa.dtype, pin_memory=True)
+    host.copy_(kappa.detach(), non_blocking=True)
     solver.ctx.call("tpa_refresh_device", _ptr(kappa))
-    solver.operator.face_coefficient = kappa.detach().cpu().numpy()
+    solver.operator.face_coefficient = host.numpy()
 
 
 class TwoPhaseStep:
