@@ -58,3 +58,23 @@ def test_solves_around_refreshes():
             st, sf = solve(x, s, rhs, rtol=rtol, precision=precision), solve(y, fresh, rhs, rtol=rtol)
             assert st.converged and sf.converged
             assert np.max(np.abs(x - y)) <= tol * np.max(np.abs(y))
+
+
+@pytest.mark.parametrize("shape", [(12, 8, 8), (10, 20, 10), (16, 16, 16)])
+def test_first_cycle_after_every_refresh(shape):
+    """A V-cycle depends on its own residual and the current coefficients only,
+    from the first one behind a refresh: its kernels start under one another and
+    read their lists early.  Equal inputs give equal bits, whatever ran before."""
+    m, s, k0, k1, r = make(*shape, walls=True)
+    rs = [r, r[::-1].copy(), 3.0 * np.roll(r, 7)]
+    seen = {}
+    for trial in range(24):
+        s.refresh((k0, k1)[trial & 1])
+        for precision in ("fp64", "mixed"):
+            for n, v in enumerate(rs):
+                z = s.vcycle(v, precision=precision)
+                first = seen.setdefault((trial & 1, precision, n), z)
+                assert np.array_equal(z, first), (trial, precision, n)
+    for n, v in enumerate(rs):  # and it is not the previous call's result
+        assert np.array_equal(s.vcycle(v), s.vcycle(v))
+        assert not np.array_equal(seen[1, "fp64", n], seen[1, "fp64", (n + 1) % 3])

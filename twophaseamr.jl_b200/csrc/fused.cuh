@@ -53,9 +53,17 @@ __device__ __forceinline__ void pdl_entry() {
 // the cycle writes: the lists and operator values of its level, which only
 // set-up and refresh write, and the host waits for those before it launches a
 // cycle.  Such loads may run while the kernels before this one drain; anything a
-// kernel of the cycle writes is read after pdl_wait.
+// kernel of the cycle writes is read after pdl_wait.  Two rules keep the halves
+// apart.  What is read after the wait comes through plain pointers: a const
+// __restrict__ parameter marks its loads as invariant, and the compiler then
+// moves them across the wait.  What is read before it comes through ld_static,
+// past the L1, whose lines may be older than the kernel's predecessor.
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename V>
+__device__ __forceinline__ V ld_static(const V* p) {
+    return __ldcg(p);
+}
 
 // Pointers of one level in precision T, read by the fused kernels.
 template <typename T>
@@ -93,9 +101,9 @@ struct LevelView {
 // coefficient refresh, which recomputes them, leaves captured graphs valid.
 template <typename T>
 __device__ __forceinline__ LevelView<T> with_weights(LevelView<T> L) {
-    L.w = T(__ldg(L.wt));
-    L.tw = T(__ldg(L.wt + 1));
-    L.rbw = T(__ldg(L.wt + 2));
+    L.w = T(ld_static(L.wt));
+    L.tw = T(ld_static(L.wt + 1));
+    L.rbw = T(ld_static(L.wt + 2));
     return L;
 }
 

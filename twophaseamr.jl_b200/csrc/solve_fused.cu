@@ -312,14 +312,15 @@ __global__ void __launch_bounds__(256) v_cg_residual(SView<double> L, const doub
     }
 }
 
-// CTA size of a level's CSR tiles: every tile resident in one wave with as
-// many warps per tile as that allows (a tile's phases are dependent chains,
-// so its latency falls with the warps that share them)
+// Kernel forms of a level's CSR tiles by the threads a tile takes (a thread per
+// row, rounded to warps): launch bounds that leave FP64 rows their registers on
+// 8 x 8 and 16 x 16 blocks, and two rows per thread beyond 1024.
 template <typename F>
-void with_tile_threads(int nt, F f) {
-    if (nt == 1024) f(std::integral_constant<int, 1024>());
-    else if (nt == 512) f(std::integral_constant<int, 512>());
-    else f(std::integral_constant<int, 256>());
+void with_tile_threads(int threads, int rows, F f) {
+    if (rows == 2) f(std::integral_constant<int, 1024>(), std::integral_constant<int, 2>());
+    else if (threads <= 256) f(std::integral_constant<int, 256>(), std::integral_constant<int, 1>());
+    else if (threads <= 640) f(std::integral_constant<int, 640>(), std::integral_constant<int, 1>());
+    else f(std::integral_constant<int, 1024>(), std::integral_constant<int, 1>());
 }
 
 template <typename T, typename F>
@@ -410,8 +411,8 @@ struct CgRz {
 // (the x update adds the stored one).
 template <typename T, typename P>
 struct NextDir {
-    const T* __restrict__ x;
-    const P* __restrict__ pold;
+    const T* x;
+    const P* pold;
     double mean, beta;
     bool first;
     __device__ __forceinline__ double operator()(int j) const {
@@ -429,8 +430,8 @@ __device__ __forceinline__ NextDir<T, P> next_dir(const T* xv, const double* mea
 
 // p = z + beta p_old, Ap and alpha = gamma / p'Ap (CSR finest level)
 template <typename T, typename P>
-__global__ void k_cg_dir_ap(LevelView<double> A, const T* __restrict__ xv, const double* mean, P* pa, P* pb,
-                            P* __restrict__ ap, double* partial, unsigned* counter, CgState* s) {
+__global__ void k_cg_dir_ap(LevelView<double> A, const T* xv, const double* mean, P* pa, P* pb, P* ap,
+                            double* partial, unsigned* counter, CgState* s) {
     pdl_launch();
     // the first row's operator entries, which no kernel of the loop writes: up to
     // kPre of them before the wait
@@ -439,19 +440,19 @@ __global__ void k_cg_dir_ap(LevelView<double> A, const T* __restrict__ xv, const
     int b0 = 0, e0 = 0, c0[kPre];
     double a0[kPre];
     if (i0 < A.n) {
-        b0 = A.rp[i0];
-        e0 = A.rp[i0 + 1];
+        b0 = ld_static(A.rp + i0);
+        e0 = ld_static(A.rp + i0 + 1);
     }
 #pragma unroll
     for (int u = 0; u < kPre; ++u)
         if (b0 + u < e0) {
-            c0[u] = A.ci[b0 + u];
-            a0[u] = A.val[b0 + u];
+            c0[u] = ld_static(A.ci + b0 + u);
+            a0[u] = ld_static(A.val + b0 + u);
         }
     pdl_wait();
     if (s->flags & kCgHalt) return;  // the run ended at this body's r'z
     const NextDir<T, P> d = next_dir(xv, mean, pa, pb, s);
-    P* __restrict__ pn = dir_new(pa, pb, s->iter);
+    P* pn = dir_new(pa, pb, s->iter);
     double v = 0;
     TPA_GRID_STRIDE(i, A.n) {
         double y = 0;
@@ -922,14 +923,15 @@ void DeviceSolver::enqueue_vcycle_epi(const R* r, const double* rsum, double* me
             // both pre-sweeps, the residual and the restriction in one launch
             const TileDev& D = tdev_[size_t(l)];
             const TileView<T>& TV = tile_view<T>(l);
-            const size_t sm = tile_down_smem<T>(D.n3max, D.n2max, D.n1max, D.emax);
-            with_tile_threads(D.nt, [&](auto nt) {
-                constexpr int NT = decltype(nt)::value;
+            const size_t sm = tile_smem<T>(D.n3max, D.n2max, D.n1max);
+            with_tile_threads(D.nt, D.rows, [&](auto nt, auto rows) {
+                constexpr int NT = decltype(nt)::value, RW = decltype(rows)::value;
                 if (l == 0)
-                    go(k_tile_down<T, R, NT>, D.ntiles, NT, sm, L, TV, r, rsum, V[size_t(l + 1)].b, L.bp);
+                    go(k_tile_down<T, R, NT, RW>, D.ntiles, D.nt, sm, L, TV, TileRhs<R>{r, rsum}, V[size_t(l + 1)].b,
+                       L.bp);
                 else
-                    go(k_tile_down<T, T, NT>, D.ntiles, NT, sm, L, TV, (const T*)L.b, no_sum, V[size_t(l + 1)].b,
-                       (T*)nullptr);
+                    go(k_tile_down<T, T, NT, RW>, D.ntiles, D.nt, sm, L, TV, TileRhs<T>{L.b, nullptr},
+                       V[size_t(l + 1)].b, (T*)nullptr);
             });
             ++launches_;
             continue;
@@ -1035,9 +1037,9 @@ void DeviceSolver::enqueue_vcycle_epi(const R* r, const double* rsum, double* me
             // prolongation and both post-sweeps in one launch
             const TileDev& D = tdev_[size_t(l)];
             const bool want_mean = (l == 0) && L.singular;
-            with_tile_threads(D.nt, [&](auto nt) {
-                constexpr int NT = decltype(nt)::value;
-                go(k_tile_up<T, Epi, NT>, D.ntiles, NT, tile_up_smem<T>(D.n3max, D.n2max, D.n1max, D.emax), L,
+            with_tile_threads(D.nt, D.rows, [&](auto nt, auto rows) {
+                constexpr int NT = decltype(nt)::value, RW = decltype(rows)::value;
+                go(k_tile_up<T, Epi, NT, RW>, D.ntiles, D.nt, tile_smem<T>(D.n3max, D.n2max, D.n1max), L,
                    tile_view<T>(l), (const T*)V[size_t(l + 1)].x, (const T*)(l == 0 ? L.bp : L.b), fpartial_.p, counters_.p + kPostMean,
                    want_mean ? mean_out : nullptr, epi);
             });
@@ -1359,20 +1361,19 @@ double DeviceSolver::time_fused(int which, int level, int precision, int iters) 
         const TileDev& D = tdev_[size_t(level)];
         const LevelView<T>& L = V[size_t(level)];
         const TileView<T>& TV = tile_view<T>(level);
-        with_tile_threads(D.nt, [&](auto nt) {
-            constexpr int NT = decltype(nt)::value;
-            const size_t sm = tile_down_smem<T>(D.n3max, D.n2max, D.n1max, D.emax);
+        with_tile_threads(D.nt, D.rows, [&](auto nt, auto rows) {
+            constexpr int NT = decltype(nt)::value, RW = decltype(rows)::value;
+            const size_t sm = tile_smem<T>(D.n3max, D.n2max, D.n1max);
             if (which == 6 && level == 0)  // the finest level reads the FP64 residual, as in the cycle
-                k_tile_down<T, double, NT><<<D.ntiles, NT, sm, stream_>>>(
-                    L, TV, (const double*)r_.p, nullptr, V[size_t(level + 1)].b, L.bp);
+                k_tile_down<T, double, NT, RW><<<D.ntiles, D.nt, sm, stream_>>>(
+                    L, TV, TileRhs<double>{r_.p, nullptr}, V[size_t(level + 1)].b, L.bp);
             else if (which == 6)
-                k_tile_down<T, T, NT><<<D.ntiles, NT, sm, stream_>>>(L, TV, (const T*)L.b, nullptr,
-                                                                     V[size_t(level + 1)].b, (T*)nullptr);
+                k_tile_down<T, T, NT, RW><<<D.ntiles, D.nt, sm, stream_>>>(L, TV, TileRhs<T>{L.b, nullptr},
+                                                                           V[size_t(level + 1)].b, (T*)nullptr);
             else
-                k_tile_up<T, MeanOnly, NT><<<D.ntiles, NT, tile_up_smem<T>(D.n3max, D.n2max, D.n1max, D.emax),
-                                            stream_>>>(L, TV, (const T*)V[size_t(level + 1)].x,
-                                                       (const T*)(level == 0 ? L.bp : L.b), fpartial_.p,
-                                                       counters_.p, nullptr, MeanOnly());
+                k_tile_up<T, MeanOnly, NT, RW><<<D.ntiles, D.nt, sm, stream_>>>(
+                    L, TV, (const T*)V[size_t(level + 1)].x, (const T*)(level == 0 ? L.bp : L.b), fpartial_.p,
+                    counters_.p, nullptr, MeanOnly());
         });
     };
     // 8 / 9: the down / up row-streaming kernel of a streamed lattice level
@@ -1459,19 +1460,6 @@ const TileView<T>& DeviceSolver::tile_view(int l) const {
     else return tf_[size_t(l)];
 }
 
-template <typename T, typename TB>
-static void allow_tile_down_smem(size_t bytes) {
-    TPA_CUDA(cudaFuncSetAttribute(k_tile_down<T, TB, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
-    TPA_CUDA(cudaFuncSetAttribute(k_tile_down<T, TB, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
-    TPA_CUDA(cudaFuncSetAttribute(k_tile_down<T, TB, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
-}
-template <typename T, typename Epi>
-static void allow_tile_up_smem(size_t bytes) {
-    TPA_CUDA(cudaFuncSetAttribute(k_tile_up<T, Epi, 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
-    TPA_CUDA(cudaFuncSetAttribute(k_tile_up<T, Epi, 512>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
-    TPA_CUDA(cudaFuncSetAttribute(k_tile_up<T, Epi, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
-}
-
 // Tiles of every CSR level of the multi-CTA part of the default cycle (not the
 // stencil levels, the tail, the red-black smoother or the cooperative cycle).
 void DeviceSolver::upload_tiles(const Hierarchy& h) {
@@ -1485,7 +1473,7 @@ void DeviceSolver::upload_tiles(const Hierarchy& h) {
     // a tile's arrays live in shared memory: at most this many cells (rings <= 3)
     int sms = 148;
     TPA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
-    size_t down_d = 0, up_d = 0;
+    size_t most = 0;  // tiles of a level: one partial sum each in the folds of the tile kernels
     for (int l = 0; l < tail_first_ && l + 1 < nl; ++l) {
         if (sdev_[size_t(l)].vec) {  // stencil tiles and row streaming need no lists
             const bool small = levels_[size_t(l)].n <= kStencilTileCells;
@@ -1518,71 +1506,44 @@ void DeviceSolver::upload_tiles(const Hierarchy& h) {
         D.n3max = T.n3max;
         D.n2max = T.n2max;
         D.n1max = T.n1max;
-        D.emax = T.emax;
-        // 2 CTAs of 1024 threads, 4 of 512 fit an SM (by threads)
-        D.nt = T.ntiles <= 2 * sms ? 1024 : T.ntiles <= 4 * sms ? 512 : 256;
+        D.rows = T.n2max > 1024 ? 2 : 1;
+        // a thread per ROWS rows and per ROWS + 1 cells
+        D.nt = (std::max((T.n2max + D.rows - 1) / D.rows, (T.n3max + D.rows) / (D.rows + 1)) + 31) & ~31;
         D.nent = int(T.pos.size());
+        D.info.upload(T.info.data(), T.info.size(), stream_);
         D.cell.upload(T.cell.data(), T.cell.size(), stream_);
         D.own.upload(T.own.data(), T.own.size(), stream_);
-        D.cell_off.upload(T.cell_off.data(), T.cell_off.size(), stream_);
-        D.ring.upload(T.ring.data(), T.ring.size(), stream_);
-        D.lrp.upload(T.lrp.data(), T.lrp.size(), stream_);
-        D.lrp_off.upload(T.lrp_off.data(), T.lrp_off.size(), stream_);
-        D.ent_off.upload(T.ent_off.data(), T.ent_off.size(), stream_);
+        D.slice.upload(T.slice.data(), T.slice.size(), stream_);
         D.pos.upload(T.pos.data(), T.pos.size(), stream_);
-        D.lcol.upload(T.lcol.data(), T.lcol.size(), stream_);
+        D.col.upload(T.col.data(), T.col.size(), stream_);
         D.co.upload(T.co.data(), T.co.size(), stream_);
-        D.co_off.upload(T.co_off.data(), T.co_off.size(), stream_);
         D.ch.upload(T.ch.data(), T.ch.size(), stream_);
         D.val_d.alloc(T.pos.size());
         D.val_f.alloc(T.pos.size());
         TPA_CUDA(cudaStreamSynchronize(stream_));  // the host arrays go out of scope
         auto fill = [&](auto& v, auto* val) {
-            v.ntiles = D.ntiles;
             v.n3max = D.n3max;
             v.n2max = D.n2max;
             v.n1max = D.n1max;
-            v.emax = D.emax;
+            v.info = D.info.p;
             v.cell = D.cell.p;
             v.own = D.own.p;
-            v.cell_off = D.cell_off.p;
-            v.ring = reinterpret_cast<const int4*>(D.ring.p);
-            v.lrp = D.lrp.p;
-            v.lrp_off = D.lrp_off.p;
-            v.ent_off = D.ent_off.p;
+            v.slice = reinterpret_cast<const int2*>(D.slice.p);
             v.val = val;
-            v.lcol = reinterpret_cast<const short*>(D.lcol.p);
+            v.col = reinterpret_cast<const short*>(D.col.p);
             v.co = D.co.p;
-            v.co_off = D.co_off.p;
             v.ch = reinterpret_cast<const short4*>(D.ch.p);
         };
         fill(td_[size_t(l)], D.val_d.p);
         fill(tf_[size_t(l)], D.val_f.p);
-        down_d = std::max(down_d, tile_down_smem<double>(D.n3max, D.n2max, D.n1max, D.emax));
-        up_d = std::max(up_d, tile_up_smem<double>(D.n3max, D.n2max, D.n1max, D.emax));
+        most = std::max(most, size_t(D.ntiles));
         D.on = true;
     }
-    if (down_d == 0) return;
-    // one partial sum per tile in the folds of the tile kernels
-    size_t ntiles = 0;
-    for (const auto& D : tdev_) ntiles = std::max(ntiles, size_t(D.on ? D.ntiles : 0));
-    if (ntiles > fpartial_.n) {
-        fpartial_.alloc(ntiles);
-        fpartial2_.alloc(ntiles);
+    if (most == 0) return;
+    if (most > fpartial_.n) {
+        fpartial_.alloc(most);
+        fpartial2_.alloc(most);
     }
-    int optin = 0;
-    TPA_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
-    if (down_d > size_t(optin) || up_d > size_t(optin)) {
-        for (auto& D : tdev_) D.on = false;
-        return;
-    }
-    allow_tile_down_smem<double, double>(down_d);
-    allow_tile_down_smem<float, double>(down_d);
-    allow_tile_down_smem<float, float>(down_d);
-    allow_tile_up_smem<double, MeanOnly>(up_d);
-    allow_tile_up_smem<float, MeanOnly>(up_d);
-    allow_tile_up_smem<double, CgRz>(up_d);
-    allow_tile_up_smem<float, CgRz>(up_d);
     gather_tile_values();
     TPA_CUDA(cudaStreamSynchronize(stream_));
     destroy_graphs();

@@ -174,8 +174,7 @@ __global__ void __launch_bounds__(kDenseBuildThreads)
 // Bound by the latency of one launch, the load of b and the warp sum.
 template <typename T, typename TB>
 __global__ void __launch_bounds__(32 * kDenseRows)
-    k_tail_dense(int n, int ld, const double* __restrict__ M, const TB* __restrict__ b, T* __restrict__ x,
-                 double* mean_out) {
+    k_tail_dense(int n, int ld, const double* __restrict__ M, const TB* b, T* x, double* mean_out) {
     pdl_launch();
     constexpr int kChunk = 2048;
     __shared__ __align__(16) double sb[kChunk];
@@ -186,7 +185,7 @@ __global__ void __launch_bounds__(32 * kDenseRows)
 #pragma unroll
         for (int q = 0; q < 16; ++q) {
             const int k = k0 + 64 * q + 2 * lane;
-            t[q] = k < n ? __ldg(reinterpret_cast<const double2*>(m + k)) : make_double2(0.0, 0.0);
+            t[q] = k < n ? ld_static(reinterpret_cast<const double2*>(m + k)) : make_double2(0.0, 0.0);
         }
     };
     load(0);

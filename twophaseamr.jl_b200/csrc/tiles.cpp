@@ -31,10 +31,6 @@ TileLevelHost build_tiles(const Csr& A, int64_t nblocks, int64_t cpb, const std:
     std::vector<int32_t> loc(size_t(n), -1);
     std::vector<char> seen(size_t(nc), 0);
     T.ntiles = int(nblocks);
-    T.cell_off.push_back(0);
-    T.lrp_off.push_back(0);
-    T.ent_off.push_back(0);
-    T.co_off.push_back(0);
     std::vector<int32_t> cells;
     for (int64_t t = 0; t < nblocks; ++t) {
         cells.clear();
@@ -61,22 +57,41 @@ TileLevelHost build_tiles(const Csr& A, int64_t nblocks, int64_t cpb, const std:
             ring[r] = int(end);
         }
         bool fits = ring[3] <= max_cells;
-        // local rows of rings <= 2: every column is a local cell by construction
+        // slices of the rows of rings <= 2: every column is a local cell by construction
         const int n2 = ring[2];
-        const size_t e_begin = T.pos.size();
-        for (int k = 0; k < n2 && fits; ++k) {
-            const int32_t g = cells[size_t(k)];
-            T.lrp.push_back(int32_t(T.pos.size() - e_begin));
-            for (int64_t e = A.ptr[size_t(g)]; e < A.ptr[size_t(g) + 1]; ++e) {
-                const int32_t lc = loc[size_t(A.col[size_t(e)])];
-                if (lc < 0 || lc >= ring[3]) fits = false;
-                T.pos.push_back(int32_t(e));
-                T.lcol.push_back(int16_t(lc));
+        TileInfo info;
+        info.cell = int32_t(T.cell.size());
+        info.slice = int32_t(T.slice.size() / 2);
+        info.co = int32_t(T.co.size());
+        for (int k0 = 0; k0 < n2 && fits; k0 += kTileSlice) {
+            int width = 0;
+            const int rows = std::min(kTileSlice, n2 - k0);
+            for (int k = 0; k < rows; ++k) {
+                const int32_t g = cells[size_t(k0 + k)];
+                width = std::max<int>(width, int(A.ptr[size_t(g) + 1] - A.ptr[size_t(g)]));
+            }
+            if (width > kTileMaxRow) fits = false;
+            const size_t first = T.pos.size();
+            T.slice.push_back(int32_t(first));
+            T.slice.push_back(width);
+            T.pos.resize(first + size_t(kTileSlice) * size_t(width), -1);
+            T.col.resize(T.pos.size(), 0);
+            for (int k = 0; k < rows && fits; ++k) {
+                const int32_t g = cells[size_t(k0 + k)];
+                for (int u = 0; u < width; ++u) {
+                    const size_t at = first + size_t(kTileSlice) * size_t(u) + size_t(k);
+                    const int64_t e = A.ptr[size_t(g)] + u;
+                    if (e >= A.ptr[size_t(g) + 1]) {
+                        T.col[at] = int16_t(k0 + k);
+                        continue;
+                    }
+                    const int32_t lc = loc[size_t(A.col[size_t(e)])];
+                    if (lc < 0 || lc >= ring[3]) fits = false;
+                    T.pos[at] = int32_t(e);
+                    T.col[at] = int16_t(lc);
+                }
             }
         }
-        T.lrp.push_back(int32_t(T.pos.size() - e_begin));
-        const int64_t ne = int64_t(T.pos.size() - e_begin);
-        if (ne > 32767) fits = false;
         // coarse cells of the block, in order of their first child
         int nco = 0;
         for (int64_t k = 0; k < cpb && fits; ++k) {
@@ -97,16 +112,15 @@ TileLevelHost build_tiles(const Csr& A, int64_t nblocks, int64_t cpb, const std:
         if (!fits) return TileLevelHost();
         T.cell.insert(T.cell.end(), cells.begin(), cells.end());
         for (int32_t g : cells) T.own.push_back(owner[size_t(g)]);
-        for (int r = 0; r < 4; ++r) T.ring.push_back(ring[r]);
-        T.cell_off.push_back(int32_t(T.cell.size()));
-        T.lrp_off.push_back(int32_t(T.lrp.size()));
-        T.ent_off.push_back(int32_t(T.pos.size()));
-        T.co_off.push_back(int32_t(T.co.size()));
+        info.nco = nco;
+        info.n0 = ring[0];
+        info.n1 = ring[1];
+        info.n2 = ring[2];
+        info.n3 = ring[3];
+        T.info.push_back(info);
         T.n3max = std::max(T.n3max, ring[3]);
         T.n2max = std::max(T.n2max, ring[2]);
         T.n1max = std::max(T.n1max, ring[1]);
-        T.emax = std::max<int>(T.emax, int(ne));
-        T.comax = std::max(T.comax, nco);
     }
     // every coarse cell belongs to exactly one tile
     if (int64_t(T.co.size()) != nc) return TileLevelHost();

@@ -19,306 +19,330 @@
 // Every row is summed in CSR order with the arithmetic of the unfused kernels
 // (pre2_cell, residual_cell, restrict_quad, prolong_cell, sweep_cell), so the
 // two paths give the same V-cycle up to the order of the coarse RHS sum.
+//
+// A thread owns one row of the tile (two on tiles of more than 1024 rows): it
+// holds the row's entries, right-hand side, diagonals and iterate in registers
+// through all phases, and only the vector that a phase reads at other rows
+// goes through shared memory.  A row's products load independent shared-memory
+// words, where walking a staged CSR row was a chain of dependent loads; per
+// tile of a 16 x 16 block this is about 2.4 k warp instructions in place of 14 k.
 #pragma once
 
 #include <cuda_runtime.h>
 
 #include "fused.cuh"
 #include "stencil.cuh"
+#include "tiles.hpp"
 
 namespace tpa {
 
-constexpr int kTileThreads = 256;  // stencil tiles; CSR tiles take NT = 256, 512 or 1024
+constexpr int kTileThreads = 256;  // stencil tiles
 constexpr int kTileMaxCells = 1536;  // cells of a CSR tile (rings <= 3) at most
 
 // One level's tiles in precision T (device pointers).
 template <typename T>
 struct TileView {
-    int ntiles;
-    int n3max, n2max, n1max, emax;
+    const TileInfo* info;
     const int* cell;
-    const int* own;    // parallel to cell: tentative owner on the coarse level
-    const int* cell_off;
-    const int4* ring;  // per tile: cells of rings <= 0, 1, 2, 3
-    const int* lrp;
-    const int* lrp_off;
-    const int* ent_off;
-    const T* val;      // the level's CSR values in tile entry order
-    const short* lcol;
+    const int* own;     // parallel to cell: tentative owner on the coarse level
+    const int2* slice;  // {first entry, width}
+    const T* val;       // the level's operator values in entry order (0: padding)
+    const short* col;
     const int* co;
-    const int* co_off;
-    const short4* ch;  // per coarse cell: local indices of its children (-1: none)
+    const short4* ch;   // per coarse cell: local indices of its children (-1: none)
+    int n3max, n2max, n1max;
 };
 
-// Shared memory of a tile: the cell arrays in precision T, the tile's CSR
-// values (T), its local row pointers (int) and local columns (short), so that
-// every phase after the prologue reads shared memory only.
+// Shared memory of a tile: the three vectors that rows read from one another.
 template <typename T>
-__host__ __device__ inline size_t tile_down_smem(int n3, int n2, int n1, int e) {
-    return sizeof(T) * (3 * size_t(n3) + size_t(n2) + 3 * size_t(n1) + size_t(e)) + sizeof(int) * (size_t(n2) + 1) +
-           sizeof(short) * size_t(e);
+__host__ __device__ inline size_t tile_smem(int n3, int n2, int n1) {
+    return sizeof(T) * (size_t(n3) + size_t(n2) + size_t(n1));
 }
 
-template <typename T>
-__host__ __device__ inline size_t tile_up_smem(int n3, int n2, int n1, int e) {
-    return sizeof(T) * (size_t(n3) + 3 * size_t(n2) + 2 * size_t(n1) + size_t(e)) + sizeof(int) * (size_t(n2) + 1) +
-           sizeof(short) * size_t(e);
+__device__ __forceinline__ TileInfo tile_info(const TileInfo* p) {
+    const int4* q = reinterpret_cast<const int4*>(p);
+    const int4 a = ld_static(q), b = ld_static(q + 1);
+    return TileInfo{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 }
 
-// Loads in flight per thread in the prologues: a CTA's latency is that of its
-// dependent load chains, so every batch of independent loads is issued before
-// any of them is used.  The lists, operator values, diagonals and volumes are
-// loaded before the programmatic-launch wait (pdl_wait), under the tail of the
-// kernel before; only the vectors the cycle writes are loaded after it.
-constexpr int kTileEntriesPerThread = 8;
-
-// the tile's local CSR into shared memory (coalesced copies, 8 entries in flight)
-template <typename T, int NT>
-__device__ __forceinline__ void tile_stage_csr(const TileView<T>& V, int t, int n2, T* sval, int* slrp, short* slc) {
-    const int* rowp = V.lrp + V.lrp_off[t];
-    const int e0 = V.ent_off[t], ne = V.ent_off[t + 1] - e0;
-    const T* val = V.val + e0;
-    const short* lc = V.lcol + e0;
-    constexpr int U = kTileEntriesPerThread;
-    for (int base = threadIdx.x; base < ne; base += U * NT) {
-        T v[U];
-        short c[U];
+// a row's entries in registers (w: its slice's width, the same over the warp)
+template <typename T>
+struct TileRow {
+    T v[kTileMaxRow];
+    int c[kTileMaxRow];
+    int w;
+    __device__ __forceinline__ void load(const TileView<T>& V, int first, int k, int n2) {
+        w = 0;
+        if (k - (k & 31) >= n2) return;  // a slice beyond the tile's rows (whole warps)
+        const int2 s = ld_static(V.slice + first + (k >> 5));
+        w = s.y;
+        const T* val = V.val + s.x + (k & 31);
+        const short* col = V.col + s.x + (k & 31);
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int e = base + u * NT;
-            if (e < ne) {
-                v[u] = val[e];
-                c[u] = lc[e];
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const int e = base + u * NT;
-            if (e < ne) {
-                sval[e] = v[u];
-                slc[e] = c[u];
+        for (int u = 0; u < kTileMaxRow; ++u) {
+            if (u < w) {
+                v[u] = ld_static(val + 32 * u);
+                c[u] = ld_static(col + 32 * u);
             }
         }
     }
-    for (int k = threadIdx.x; k <= n2; k += blockDim.x) slrp[k] = rowp[k];
-}
+    __device__ __forceinline__ T dot(const T* x) const {
+        T acc = T(0);
+#pragma unroll
+        for (int u = 0; u < kTileMaxRow; ++u)
+            if (u < w) acc += v[u] * x[c[u]];
+        return acc;
+    }
+};
 
-template <typename T>
-__device__ __forceinline__ T tile_rowdot(const T* val, const short* lc, const int* lrp, const T* v, int k) {
-    T acc = T(0);
-    for (int e = lrp[k]; e < lrp[k + 1]; ++e) acc += val[e] * v[lc[e]];
-    return acc;
-}
+// Right-hand side of a level of one solve: the level's own or, on the finest
+// level, the caller's residual (FP64 or FP32), projected by the level's sum.
+template <typename TB>
+struct TileRhs {
+    const TB* b;
+    const double* sum;  // null: not projected
+    template <typename T>
+    __device__ __forceinline__ bool projects(const LevelView<T>& L) const {
+        return L.singular && sum;
+    }
+    template <typename T>
+    __device__ __forceinline__ bool start(const LevelView<T>& L, double& mean) const {
+        mean = projects(L) ? *sum * L.cvol_inv : 0.0;
+        return true;
+    }
+    __device__ __forceinline__ TB load(int g) const { return b[g]; }
+};
 
-__device__ __forceinline__ int short4_at(short4 v, int q) {
-    return q == 0 ? v.x : q == 1 ? v.y : q == 2 ? v.z : v.w;
-}
-
-// b: this level's raw right-hand side (the FP64 residual on the finest level);
-// level_sum: its sum (projection; null below the finest level); bc: the coarse
-// right-hand side; bp_out (null: not written, the cycle reads b itself): the
-// projected right-hand side for k_tile_up.
-template <typename T, typename TB, int NT>
-__global__ void __launch_bounds__(NT)
-    k_tile_down(LevelView<T> L, TileView<T> V, const TB* __restrict__ b, const double* level_sum,
-                T* __restrict__ bc, T* bp_out) {
-    pdl_launch();
-    L = with_weights(L);
-    extern __shared__ __align__(16) unsigned char tile_smem[];
-    T* bp = reinterpret_cast<T*>(tile_smem);
-    T* dv = bp + V.n3max;
-    T* xa = dv + V.n3max;
+// The down half on tile blockIdx.x: src gives the right-hand side; bc receives
+// the coarse one; bp_out (null: not written, the cycle reads b itself) the
+// projected right-hand side for the up half; the pre-smoothed iterate goes to
+// L.y.  ROWS rows and ROWS + 1 cells per thread.
+template <typename T, int ROWS, typename Src>
+__device__ __forceinline__ void tile_down(const LevelView<T>& L, const TileView<T>& V, const Src& src,
+                                          T* bc, T* bp_out) {
+    extern __shared__ __align__(16) unsigned char tile_smem_raw[];
+    T* xa = reinterpret_cast<T*>(tile_smem_raw);
     T* xb = xa + V.n3max;
-    T* ti = xb + V.n2max;
-    T* rr = ti + V.n1max;
-    T* ss = rr + V.n1max;
-    T* val = ss + V.n1max;
-    int* lrp = reinterpret_cast<int*>(val + V.emax);
-    short* lc = reinterpret_cast<short*>(lrp + V.n2max + 1);
-    const int t = blockIdx.x;
-    const int4 R = V.ring[t];
-    const int* cell = V.cell + V.cell_off[t];
-    constexpr int CU = (kTileMaxCells + NT - 1) / NT;
+    T* ss = xb + V.n2max;
+    constexpr int CU = ROWS + 1;
+    const TileInfo I = tile_info(V.info + blockIdx.x);
+    const int nt = blockDim.x;
     int g[CU];
 #pragma unroll
     for (int u = 0; u < CU; ++u) {
-        const int k = threadIdx.x + u * NT;
-        g[u] = k < R.w ? cell[k] : -1;
+        const int k = threadIdx.x + u * nt;
+        g[u] = k < I.n3 ? ld_static(V.cell + I.cell + k) : -1;
     }
-    const bool project = L.singular && level_sum;
-    T vv[CU], dd[CU], tt[CU];
+    TileRow<T> row[ROWS];
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) row[q].load(V, I.slice, threadIdx.x + q * nt, I.n2);
+    const bool project = src.projects(L);
+    T vv[CU], dd[CU], tt[ROWS];
 #pragma unroll
     for (int u = 0; u < CU; ++u) {
+        vv[u] = dd[u] = T(0);
         if (g[u] >= 0) {
-            vv[u] = project ? L.vol[g[u]] : T(0);
-            dd[u] = L.dinv[g[u]];
-            tt[u] = L.tinv[g[u]];
+            if (project) vv[u] = ld_static(L.vol + g[u]);
+            dd[u] = ld_static(L.dinv + g[u]);
         }
     }
-    // the restriction's lists: one lane per child, four per coarse cell
-    const int c0 = V.co_off[t];
-    const int nco = V.co_off[t + 1] - c0;
-    const int J0 = threadIdx.x >> 2;
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) tt[q] = int(threadIdx.x) + q * nt < I.n1 ? ld_static(L.tinv + g[q]) : T(0);
     short4 ch0 = make_short4(-1, -1, -1, -1);
     int co0 = 0;
-    if (J0 < nco) {
-        ch0 = V.ch[c0 + J0];
-        co0 = V.co[c0 + J0];
+    if (int(threadIdx.x) < I.nco) {
+        ch0 = ld_static(V.ch + I.co + threadIdx.x);
+        co0 = ld_static(V.co + I.co + threadIdx.x);
     }
-    tile_stage_csr<T, NT>(V, t, R.z, val, lrp, lc);
     pdl_wait();
-    const double mean = project ? *level_sum * L.cvol_inv : 0.0;
-    TB bb[CU];
+    double mean;
+    if (!src.start(L, mean)) return;  // the same over the tile
+    T bp[CU];
 #pragma unroll
     for (int u = 0; u < CU; ++u)
-        if (g[u] >= 0) bb[u] = b[g[u]];
-#pragma unroll
-    for (int u = 0; u < CU; ++u) {
-        const int k = threadIdx.x + u * NT;
         if (g[u] >= 0) {
-            // the projected RHS as proj_b forms it
-            double v = double(bb[u]);
-            if (project) v -= double(vv[u]) * mean;
-            const T bk = T(v);
-            bp[k] = bk;
-            dv[k] = dd[u];
-            xa[k] = L.w * dd[u] * bk;
-            if (k < R.y) ti[k] = tt[u];
+            double v = double(src.load(g[u]));
+            if (project) v -= double(vv[u]) * mean;  // as proj_b
+            bp[u] = T(v);
+        }
+    T xr[ROWS], rr[ROWS];
+#pragma unroll
+    for (int u = 0; u < CU; ++u)
+        if (g[u] >= 0) {
+            const T x1 = L.w * dd[u] * bp[u];
+            xa[threadIdx.x + u * nt] = x1;
+            if (u < ROWS) xr[u] = x1;
+        }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) {
+        const int k = threadIdx.x + q * nt;
+        if (k < I.n2) {
+            xr[q] = xr[q] + L.w * dd[q] * (bp[q] - row[q].dot(xa));
+            xb[k] = xr[q];
         }
     }
     __syncthreads();
-    for (int k = threadIdx.x; k < R.z; k += blockDim.x) {
-        const T acc = tile_rowdot(val, lc, lrp, xa, k);
-        xb[k] = xa[k] + L.w * dv[k] * (bp[k] - acc);
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) {
+        const int k = threadIdx.x + q * nt;
+        if (k < I.n1) {
+            rr[q] = bp[q] - row[q].dot(xb);
+            ss[k] = tt[q] * rr[q];
+        }
+        if (k < I.n0) {
+            L.y[g[q]] = xr[q];  // the pre-smoothed iterate, read by the up half
+            if (bp_out) bp_out[g[q]] = bp[q];
+        }
     }
     __syncthreads();
-    for (int k = threadIdx.x; k < R.y; k += blockDim.x) {
-        const T rk = bp[k] - tile_rowdot(val, lc, lrp, xb, k);
-        rr[k] = rk;
-        ss[k] = ti[k] * rk;
+    T* t = xa;  // r - wt A s on the block
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) {
+        const int k = threadIdx.x + q * nt;
+        if (k < I.n0) t[k] = rr[q] - L.tw * row[q].dot(ss);
     }
+    __syncthreads();
+    // a coarse cell per thread, its children in the fixed order (c0 + c1) + (c2 + c3)
+    for (int J = threadIdx.x; J < I.nco; J += nt) {
+        const short4 c = J == int(threadIdx.x) ? ch0 : V.ch[I.co + J];
+        const T c0 = c.x >= 0 ? t[c.x] : T(0), c1 = c.y >= 0 ? t[c.y] : T(0);
+        const T c2 = c.z >= 0 ? t[c.z] : T(0), c3 = c.w >= 0 ? t[c.w] : T(0);
+        bc[J == int(threadIdx.x) ? co0 : V.co[I.co + J]] = (c0 + c1) + (c2 + c3);
+    }
+}
+
+// The up half: xc the coarse level's correction, bp_in the projected right-hand
+// side; out(g, x) takes the result of cell g and its value from `pre(g)`, which
+// is called before the wait (static data) and `late(g)` after it.
+template <typename T, int ROWS, typename Out>
+__device__ __forceinline__ void tile_up(const LevelView<T>& L, const TileView<T>& V, const T* xc, const T* bp_in,
+                                        Out& out) {
+    extern __shared__ __align__(16) unsigned char tile_smem_raw[];
+    T* e = reinterpret_cast<T*>(tile_smem_raw);
+    T* xp = e + V.n3max;
+    T* xq = xp + V.n2max;
+    constexpr int CU = ROWS + 1;
+    const TileInfo I = tile_info(V.info + blockIdx.x);
+    const int nt = blockDim.x;
+    int g[CU], o[CU];
 #pragma unroll
     for (int u = 0; u < CU; ++u) {
-        const int k = threadIdx.x + u * NT;
-        if (k < R.x) {
-            L.y[g[u]] = xb[k];  // the pre-smoothed iterate, read by k_tile_up
-            if (bp_out) bp_out[g[u]] = bp[k];
+        const int k = threadIdx.x + u * nt;
+        g[u] = k < I.n3 ? ld_static(V.cell + I.cell + k) : -1;
+        o[u] = k < I.n3 ? ld_static(V.own + I.cell + k) : -1;
+    }
+    TileRow<T> row[ROWS];
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) row[q].load(V, I.slice, threadIdx.x + q * nt, I.n2);
+    T dd[ROWS], tt[ROWS], x[ROWS], bb[ROWS], er[ROWS];
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) {
+        const int k = threadIdx.x + q * nt;
+        if (k < I.n2) {
+            dd[q] = ld_static(L.dinv + g[q]);
+            tt[q] = ld_static(L.tinv + g[q]);
+        }
+        out.before(q, g[q], k < I.n0);
+    }
+    pdl_wait();
+    if (!out.start()) return;  // the same over the tile
+#pragma unroll
+    for (int u = 0; u < CU; ++u) {
+        const int k = threadIdx.x + u * nt;
+        if (g[u] >= 0) {
+            const T ev = xc[o[u]];
+            e[k] = ev;
+            if (u < ROWS) er[u] = ev;
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) {
+        const int k = threadIdx.x + q * nt;
+        if (k < I.n2) x[q] = L.y[g[q]];
+        if (k < I.n1) bb[q] = bp_in[g[q]];
+        out.after(q, g[q], k < I.n0);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) {
+        const int k = threadIdx.x + q * nt;
+        if (k < I.n2) {
+            x[q] += er[q] - L.tw * tt[q] * row[q].dot(e);
+            xp[k] = x[q];
         }
     }
     __syncthreads();
-    // four lanes per coarse cell, lane q takes child q; whole warps (shuffles)
-    const int quads = (4 * nco + 31) & ~31;
-    for (int gq = threadIdx.x; gq < quads; gq += blockDim.x) {
-        const int J = gq >> 2, q = gq & 3;
-        T acc = T(0);
-        if (J < nco) {
-            const int i = short4_at(J == J0 ? ch0 : V.ch[c0 + J], q);
-            if (i >= 0) acc = rr[i] - L.tw * tile_rowdot(val, lc, lrp, ss, i);
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) {
+        const int k = threadIdx.x + q * nt;
+        if (k < I.n1) {
+            x[q] = x[q] + L.w * dd[q] * (bb[q] - row[q].dot(xp));
+            xq[k] = x[q];
         }
-        acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-        acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-        if (q == 0 && J < nco) {
-            bc[J == J0 ? co0 : V.co[c0 + J]] = acc;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < ROWS; ++q) {
+        const int k = threadIdx.x + q * nt;
+        if (k < I.n0) {
+            const T v = x[q] + L.w * dd[q] * (bb[q] - row[q].dot(xq));
+            L.x[g[q]] = v;
+            out.take(q, double(v));
         }
     }
 }
+
+template <typename T, typename TB, int NT, int ROWS>
+__global__ void __launch_bounds__(NT, 1)
+    k_tile_down(LevelView<T> L, TileView<T> V, TileRhs<TB> src, T* bc, T* bp_out) {
+    pdl_launch();
+    tile_down<T, ROWS>(with_weights(L), V, src, bc, bp_out);
+}
+
+// What the up half of one solve's level does with its result: the sums of the
+// finest level's mean (mean_out not null) and of the epilogue's r'x.
+template <typename T, typename Epi, int ROWS>
+struct TileMean {
+    const T* vol;
+    bool on;
+    const Epi& epi;
+    T vv[ROWS];
+    double rv[ROWS];
+    double v = 0, w = 0;
+    __device__ __forceinline__ void before(int q, int g, bool own) {
+        if (on && own) vv[q] = ld_static(vol + g);
+    }
+    __device__ __forceinline__ bool start() const { return true; }
+    __device__ __forceinline__ void after(int q, int g, bool own) {
+        if constexpr (Epi::kRz)
+            if (on && own) rv[q] = epi.r[g];
+    }
+    __device__ __forceinline__ void take(int q, double x) {
+        if (!on) return;
+        v += double(vv[q]) * x;
+        if constexpr (Epi::kRz) w += rv[q] * x;
+    }
+};
 
 // xc: the coarse level's correction; bp_in: the projected right-hand side (the
 // level's own below the finest); mean_out (may be null): the volume mean of the
 // result, folded by the last CTA, which then runs `epi`.
-template <typename T, typename Epi, int NT>
-__global__ void __launch_bounds__(NT)
-    k_tile_up(LevelView<T> L, TileView<T> V, const T* __restrict__ xc, const T* __restrict__ bp_in, double* partial, unsigned* counter,
+template <typename T, typename Epi, int NT, int ROWS>
+__global__ void __launch_bounds__(NT, 1)
+    k_tile_up(LevelView<T> L, TileView<T> V, const T* xc, const T* bp_in, double* partial, unsigned* counter,
               double* mean_out, Epi epi) {
     pdl_launch();
-    L = with_weights(L);
-    extern __shared__ __align__(16) unsigned char tile_smem[];
-    T* e = reinterpret_cast<T*>(tile_smem);
-    T* xp = e + V.n3max;
-    T* dv = xp + V.n2max;
-    T* ti = dv + V.n2max;
-    T* bp = ti + V.n2max;
-    T* xq = bp + V.n1max;
-    T* val = xq + V.n1max;
-    int* lrp = reinterpret_cast<int*>(val + V.emax);
-    short* lc = reinterpret_cast<short*>(lrp + V.n2max + 1);
-    const int t = blockIdx.x;
-    const int4 R = V.ring[t];
-    const int* cell = V.cell + V.cell_off[t];
-    const int* own = V.own + V.cell_off[t];
-    constexpr int CU = (kTileMaxCells + NT - 1) / NT;
-    int g[CU], o[CU];
-#pragma unroll
-    for (int u = 0; u < CU; ++u) {
-        const int k = threadIdx.x + u * NT;
-        g[u] = k < R.w ? cell[k] : -1;
-        o[u] = k < R.w ? own[k] : -1;
-    }
-    T ee[CU], yy[CU], dd[CU], tt[CU], bb[CU], vv[CU];
-    double rv[CU];
-#pragma unroll
-    for (int u = 0; u < CU; ++u) {
-        const int k = threadIdx.x + u * NT;
-        if (k < R.z) {
-            dd[u] = L.dinv[g[u]];
-            tt[u] = L.tinv[g[u]];
-        }
-        if (mean_out && k < R.x) vv[u] = L.vol[g[u]];
-    }
-    tile_stage_csr<T, NT>(V, t, R.z, val, lrp, lc);
-    pdl_wait();
-#pragma unroll
-    for (int u = 0; u < CU; ++u) {
-        const int k = threadIdx.x + u * NT;
-        if (g[u] >= 0) {
-            ee[u] = xc[o[u]];
-            if (k < R.z) yy[u] = L.y[g[u]];
-            if (k < R.y) bb[u] = bp_in[g[u]];
-            if constexpr (Epi::kRz)
-                if (mean_out && k < R.x) rv[u] = epi.r[g[u]];
-        }
-    }
-#pragma unroll
-    for (int u = 0; u < CU; ++u) {
-        const int k = threadIdx.x + u * NT;
-        if (g[u] >= 0) {
-            e[k] = ee[u];
-            if (k < R.z) {
-                xp[k] = yy[u];
-                dv[k] = dd[u];
-                ti[k] = tt[u];
-            }
-            if (k < R.y) bp[k] = bb[u];
-        }
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < R.z; k += blockDim.x) {
-        const T ae = tile_rowdot(val, lc, lrp, e, k);
-        xp[k] += e[k] - L.tw * ti[k] * ae;
-    }
-    __syncthreads();
-    for (int k = threadIdx.x; k < R.y; k += blockDim.x)
-        xq[k] = xp[k] + L.w * dv[k] * (bp[k] - tile_rowdot(val, lc, lrp, xp, k));
-    __syncthreads();
-    double v = 0, w = 0;
-#pragma unroll
-    for (int u = 0; u < CU; ++u) {
-        const int k = threadIdx.x + u * NT;
-        if (k >= R.x) break;
-        const T out = xq[k] + L.w * dv[k] * (bp[k] - tile_rowdot(val, lc, lrp, xq, k));
-        L.x[g[u]] = out;
-        if (mean_out) {
-            v += double(vv[u]) * double(out);
-            if constexpr (Epi::kRz) w += rv[u] * double(out);
-        }
-    }
-    if (mean_out) fold_mean(v, w, partial, counter, mean_out, L.cvol_inv, epi);
+    TileMean<T, Epi, ROWS> out{L.vol, mean_out != nullptr, epi};
+    tile_up<T, ROWS>(with_weights(L), V, xc, bp_in, out);
+    if (mean_out) fold_mean(out.v, out.w, partial, counter, mean_out, L.cvol_inv, epi);
 }
 
-// tile copies of a level's CSR values: out[k] = val[pos[k]]
+// tile copies of a level's CSR values: out[k] = val[pos[k]] (0 for padding)
 template <typename T>
 __global__ void k_tile_gather(int m, const int* __restrict__ pos, const T* __restrict__ val, T* __restrict__ out) {
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x) out[k] = val[pos[k]];
+    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < m; k += gridDim.x * blockDim.x)
+        out[k] = pos[k] >= 0 ? val[pos[k]] : T(0);
 }
 
 // ---------------------------------------------------------------------------------
@@ -341,12 +365,12 @@ __device__ __forceinline__ int at(int i, int j) { return (j + 3) * R + (i + 3); 
 template <typename T>
 __device__ __forceinline__ void vt_blocks(const SView<T>& L, int b, int* nb9) {
     if (threadIdx.x == 0) {
-        const int4 c = *reinterpret_cast<const int4*>(L.nbr + 4 * b);
+        const int4 c = ld_static(reinterpret_cast<const int4*>(L.nbr + 4 * b));
         const int4 none = make_int4(-1, -1, -1, -1);
-        const int4 w = c.x >= 0 ? *reinterpret_cast<const int4*>(L.nbr + 4 * c.x) : none;
-        const int4 e = c.y >= 0 ? *reinterpret_cast<const int4*>(L.nbr + 4 * c.y) : none;
-        const int4 s = c.z >= 0 ? *reinterpret_cast<const int4*>(L.nbr + 4 * c.z) : none;
-        const int4 n = c.w >= 0 ? *reinterpret_cast<const int4*>(L.nbr + 4 * c.w) : none;
+        const int4 w = c.x >= 0 ? ld_static(reinterpret_cast<const int4*>(L.nbr + 4 * c.x)) : none;
+        const int4 e = c.y >= 0 ? ld_static(reinterpret_cast<const int4*>(L.nbr + 4 * c.y)) : none;
+        const int4 s = c.z >= 0 ? ld_static(reinterpret_cast<const int4*>(L.nbr + 4 * c.z)) : none;
+        const int4 n = c.w >= 0 ? ld_static(reinterpret_cast<const int4*>(L.nbr + 4 * c.w)) : none;
         nb9[0] = c.x >= 0 ? w.z : s.x;  // south-west
         nb9[1] = c.z;
         nb9[2] = c.y >= 0 ? e.z : s.y;  // south-east
@@ -381,7 +405,7 @@ __device__ __forceinline__ T vt_apply(const SView<T>& L, const T* v, const unsig
 
 template <typename T, typename TB>
 __global__ void __launch_bounds__(kTileThreads)
-    v_tile_down(SView<T> L, const TB* __restrict__ bin, const double* level_sum, T* __restrict__ bc, T* bp_out) {
+    v_tile_down(SView<T> L, const TB* bin, const double* level_sum, T* bc, T* bp_out) {
     pdl_launch();
     constexpr int N = vt::R * vt::R;
     __shared__ T sb[N], sd[N], sx[N], sy[N], sr[N], ss[N];
@@ -390,7 +414,7 @@ __global__ void __launch_bounds__(kTileThreads)
     const int b = blockIdx.x;
     vt_blocks(L, b, nb9);
     const bool project = L.singular && level_sum;
-    const int4 mp = *reinterpret_cast<const int4*>(L.map + 4 * b);
+    const int4 mp = ld_static(reinterpret_cast<const int4*>(L.map + 4 * b));
     __syncthreads();
     // the region's loads, all issued before any is used; the volumes and
     // diagonals before the wait
@@ -406,8 +430,8 @@ __global__ void __launch_bounds__(kTileThreads)
 #pragma unroll
     for (int u = 0; u < QU; ++u) {
         if (c[u] >= 0) {
-            vo[u] = (project && !L.const_vol) ? L.vol[c[u]] : L.vol0;
-            dd[u] = L.dinv ? L.dinv[c[u]] : L.dinv0;
+            vo[u] = (project && !L.const_vol) ? ld_static(L.vol + c[u]) : L.vol0;
+            dd[u] = L.dinv ? ld_static(L.dinv + c[u]) : L.dinv0;
         }
     }
     pdl_wait();
@@ -481,8 +505,7 @@ __device__ __forceinline__ T vt_coarse(const SView<T>& L, const T* xc, int B, in
 
 template <typename T, typename Epi>
 __global__ void __launch_bounds__(kTileThreads)
-    v_tile_up(SView<T> L, const T* __restrict__ xc, const T* __restrict__ bp_in, double* partial, unsigned* counter,
-              double* mean_out, Epi epi) {
+    v_tile_up(SView<T> L, const T* xc, const T* bp_in, double* partial, unsigned* counter, double* mean_out, Epi epi) {
     pdl_launch();
     constexpr int N = vt::R * vt::R;
     __shared__ T se[N], sp[N], sq[N], sd[N], sb[N];
@@ -509,7 +532,7 @@ __global__ void __launch_bounds__(kTileThreads)
             ring[u] = max(max(-i, i - 15), max(-j, j - 15));
             if (B >= 0) {
                 c[u] = B * 256 + lj[u] * 16 + li[u];
-                mp[u] = *reinterpret_cast<const int4*>(L.map + 4 * B);
+                mp[u] = ld_static(reinterpret_cast<const int4*>(L.map + 4 * B));
             }
         }
     }
@@ -517,7 +540,7 @@ __global__ void __launch_bounds__(kTileThreads)
 #pragma unroll
     for (int u = 0; u < QU; ++u) {
         e[u] = x[u] = d[u] = bp[u] = T(0);
-        if (c[u] >= 0 && ring[u] <= 2) d[u] = L.dinv ? L.dinv[c[u]] : L.dinv0;
+        if (c[u] >= 0 && ring[u] <= 2) d[u] = L.dinv ? ld_static(L.dinv + c[u]) : L.dinv0;
     }
     pdl_wait();
 #pragma unroll

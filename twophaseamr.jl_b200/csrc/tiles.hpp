@@ -20,26 +20,36 @@
 
 namespace tpa {
 
+// A tile's rows (rings <= 2) are cut into slices of 32 rows, one per warp, each
+// as wide as its longest row: entry u of the slice's row k lies at
+// 32 u + k of the slice, so that a warp's loads are consecutive.  Rows of the
+// balanced tree hold at most 11 entries; a level with a longer row than
+// kTileMaxRow is not tiled.
+constexpr int kTileSlice = 32;
+constexpr int kTileMaxRow = 12;
+
+// a tile's parts of the level's lists
+struct alignas(16) TileInfo {
+    int32_t cell, slice, co, nco;  // first cell, first slice, first coarse cell and their number
+    int32_t n0, n1, n2, n3;        // cells of rings <= 0, 1, 2, 3
+};
+
 struct TileLevelHost {
     bool ok = false;
     int ntiles = 0;
     int n3max = 0, n2max = 0, n1max = 0;  // largest ring counts (cumulative) over the tiles
-    int emax = 0;                         // largest number of local CSR entries of a tile
-    int comax = 0;                        // largest number of coarse cells of a tile
-    // per tile t, cells cell[cell_off[t] .. cell_off[t + 1]): the block's cells in
-    // order (n0 of them), then ring 1, ring 2, ring 3; ring[4 t + r] = cells of
-    // rings <= r (ring[4 t] = n0)
-    std::vector<int32_t> cell, cell_off, ring;
-    std::vector<int32_t> own;  // parallel to cell: the tentative owner (coarse cell) of each tile cell
-    // local rows 0 .. n2 - 1 of tile t: entries lrp[lrp_off[t] + k] ..
-    // lrp[lrp_off[t] + k + 1] (relative to ent_off[t]) in CSR order; pos is the
-    // entry's position in the level CSR, lcol its column as a local cell index
-    std::vector<int32_t> lrp, lrp_off, pos, ent_off;
-    std::vector<int16_t> lcol;
-    // coarse cells whose children lie in tile t: co[co_off[t] ..), and for each
-    // the local indices of its first four children (-1: none), in the order of
-    // the level's child lists
-    std::vector<int32_t> co, co_off;
+    std::vector<TileInfo> info;
+    // the tiles' cells: the block's in order, then ring 1, ring 2, ring 3, each
+    // with its tentative owner (coarse cell)
+    std::vector<int32_t> cell, own;
+    // slices {first entry, width}, and per entry its position in the level CSR
+    // (-1: padding) and its column as a local cell index (padding: the row's own)
+    std::vector<int32_t> slice, pos;
+    std::vector<int16_t> col;
+    // the coarse cells whose children lie in a tile and, for each, the local
+    // indices of its first four children (-1: none), in the order of the level's
+    // child lists
+    std::vector<int32_t> co;
     std::vector<int16_t> ch;
 };
 
@@ -47,7 +57,8 @@ struct TileLevelHost {
 // sorted columns) and tentative owners `owner` onto `nc` coarse cells.  ok is
 // false (and the level keeps the unfused kernels) when a coarse cell's
 // children do not all lie in one block, a coarse cell has more than four
-// children, or a tile would exceed `max_cells` cells or 32767 local entries.
+// children, a row has more than kTileMaxRow entries, or a tile would exceed
+// `max_cells` cells.
 TileLevelHost build_tiles(const Csr& A, int64_t nblocks, int64_t cpb, const std::vector<int32_t>& owner, int64_t nc,
                           int max_cells);
 
