@@ -20,10 +20,10 @@ def refine(seed, density):
 
 CASES = {
     # mesh, whether the finest level is tiled
-    "b32": (dict(base_mesh=(128, 96), block_size=(32, 32), periodic=(True, False), max_level=1,
+    "b32": (dict(base_mesh=(128, 64), block_size=(32, 32), periodic=(True, False), max_level=1,
                  refine=refine(1, 0.4)), True),
     "b24": (dict(base_mesh=(48, 48), block_size=(24, 24), max_level=2, refine=refine(2, 0.6)), True),
-    "b16": (dict(base_mesh=(32, 48), block_size=(16, 16), periodic=(False, False), max_level=3,
+    "b16": (dict(base_mesh=(32, 32), block_size=(16, 16), periodic=(False, False), max_level=3,
                  refine=refine(3, 0.6)), True),
     "b16x2": (dict(base_mesh=(64, 16), block_size=(16, 2), extent=(4.0, 1.0), max_level=2,
                    refine=refine(4, 0.5)), True),
