@@ -315,7 +315,7 @@ private:
         bool stream = false;  // periodic lattice level: row-streaming kernels (v_stream_*)
         int srows[2] = {0, 0}, sgrid[2] = {0, 0};  // their strip height and grid (FP64, FP32 kernels)
         int cg_rows = 0, cg_grid = 0;              // the same for the CG direction kernel (finest level)
-        int ntiles = 0, n3max = 0, n2max = 0, n1max = 0, nent = 0;
+        int ntiles = 0, nent = 0;
         int nt = 256, rows = 1;  // threads per tile and rows per thread
         DevArray<TileInfo> info;
         DevArray<int> cell, own, slice, pos, co;

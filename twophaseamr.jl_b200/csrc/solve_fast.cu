@@ -26,33 +26,13 @@
 #include "cg_state.cuh"
 #include "device.cuh"
 #include "launch.cuh"
+#include "solve_state.cuh"
 
 namespace tpa {
 namespace {
 
 constexpr int kGrid = 1184;  // 8 CTAs on each of 148 SMs
 constexpr int kCPrep = 8, kCPres = 9, kCMean = 10;
-
-__device__ __forceinline__ double block_max_all(double v) {
-    __shared__ double sh[32];
-    __shared__ int nan_seen;
-    bool nan = v != v;
-    double m = nan ? 0.0 : v;
-    for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    __syncthreads();
-    if (threadIdx.x == 0) nan_seen = 0;
-    __syncthreads();
-    if (nan) nan_seen = 1;
-    if (!lane) sh[wid] = m;
-    __syncthreads();
-    m = 0;
-    if (threadIdx.x < (blockDim.x >> 5)) m = sh[threadIdx.x];
-    if (wid == 0)
-        for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
-    __syncthreads();
-    return nan_seen ? NAN : m;
-}
 
 // Publish N block values (sums where max_mask bit k is 0, maxima where it is 1)
 // and fold them in the last block in block order; its thread 0 calls done(out[N]).
@@ -83,38 +63,6 @@ __device__ __forceinline__ void publish_fold(const double (&v)[N], unsigned max_
     }
 }
 
-constexpr double kEps = 2.220446049250313e-16;
-
-// std::max's choice, a NaN in second place included
-__device__ __forceinline__ double std_max(double a, double b) { return a < b ? b : a; }
-
-// roundoff floor of a residual from max |A||x| / V and max |b| / V
-__host__ __device__ inline double roundoff_floor(double ax, double b) {
-    const double m = ax < b ? b : ax;
-    return 128 * kEps * (1.0 < m ? m : 1.0);
-}
-
-// What the solve was asked for (kernel parameters).
-struct SolveAsk {
-    double rtol, atol, cvol;  // cvol: volume of the ungauged component (0: none)
-    double eta;               // refinement solve: reduction per run (0: one run to the target)
-    int max_cycles, strict;   // strict: an incompatible right-hand side is an error
-};
-
-// target of a run from a residual of strong maximum linf
-__device__ __forceinline__ double run_target(const SolveAsk& q, double target, double linf) {
-    return q.eta > 0 ? std_max(target, q.eta * linf) : target;
-}
-
-__device__ __forceinline__ void start_run(CgState* c, double target, double rsum, int itmax, bool go) {
-    c->target = target;
-    c->rsum = rsum;
-    c->itmax = itmax;
-    c->iter = 0;
-    c->fresh = 1;
-    c->flags = go ? 0 : 8;
-}
-
 // sums of b = V f, |b| and V x0 over cells with V > 0; the means to remove.
 // vol null: every cell's volume is vol0.
 __global__ void k_prep(int n, const double* __restrict__ rhs, const double* __restrict__ xin,
@@ -140,29 +88,6 @@ __global__ void k_prep(int n, const double* __restrict__ rhs, const double* __re
         // a non-finite right-hand side value makes sum |b| non-finite
         S->ok = isfinite(t[1]) && !(q.strict && comp && fabs(t[0]) > 256 * kEps * std_max(1.0, t[1]));
     });
-}
-
-// After the first residual: the target, and the first run unless there is
-// nothing to solve.  v: {sum_V r^2 / V, max |r| / V, max |A||x| / V, max |b| / V, sum r}.
-__device__ __forceinline__ void after_first(const double (&v)[5], const SolveAsk& q, SolveState* S, CgState* c) {
-    for (int k = 0; k < 4; ++k) S->init[k] = S->fin[k] = v[k];
-    const double floor = roundoff_floor(v[2], v[3]);
-    const double target = std_max(q.atol, std_max(q.rtol * std_max(v[1], kEps), floor));
-    const bool go = S->ok && v[1] > target && q.max_cycles > 0;
-    S->target = target;
-    S->skip = go ? 0 : 1;
-    S->niter = S->flags = S->total = 0;
-    start_run(c, run_target(q, target, v[1]), v[4], q.max_cycles, go);
-}
-
-// After a run's true residual: its counts, and the state of a further run
-// (which the host decides on).
-__device__ __forceinline__ void after_run(const double (&v)[5], const SolveAsk& q, SolveState* S, CgState* c) {
-    for (int k = 0; k < 4; ++k) S->fin[k] = v[k];
-    S->niter = c->iter;
-    S->flags = c->flags;
-    S->total += c->iter;
-    start_run(c, run_target(q, S->target, v[1]), v[4], q.max_cycles - S->total, true);
 }
 
 // Vectors of a residual pass.  First: b = V f - V mb and x = x_in - mx (0 where

@@ -312,17 +312,6 @@ __global__ void __launch_bounds__(256) v_cg_residual(SView<double> L, const doub
     }
 }
 
-// Kernel forms of a level's CSR tiles by the threads a tile takes (a thread per
-// row, rounded to warps): launch bounds that leave FP64 rows their registers on
-// 8 x 8 and 16 x 16 blocks, and two rows per thread beyond 1024.
-template <typename F>
-void with_tile_threads(int threads, int rows, F f) {
-    if (rows == 2) f(std::integral_constant<int, 1024>(), std::integral_constant<int, 2>());
-    else if (threads <= 256) f(std::integral_constant<int, 256>(), std::integral_constant<int, 1>());
-    else if (threads <= 640) f(std::integral_constant<int, 640>(), std::integral_constant<int, 1>());
-    else f(std::integral_constant<int, 1024>(), std::integral_constant<int, 1>());
-}
-
 template <typename T, typename F>
 void with_nxc(const SView<T>& S, F f) {
     if (S.nx == 16 && S.ny == 16) f(std::integral_constant<int, 16>{});
@@ -923,14 +912,13 @@ void DeviceSolver::enqueue_vcycle_epi(const R* r, const double* rsum, double* me
             // both pre-sweeps, the residual and the restriction in one launch
             const TileDev& D = tdev_[size_t(l)];
             const TileView<T>& TV = tile_view<T>(l);
-            const size_t sm = tile_smem<T>(D.n3max, D.n2max, D.n1max);
             with_tile_threads(D.nt, D.rows, [&](auto nt, auto rows) {
                 constexpr int NT = decltype(nt)::value, RW = decltype(rows)::value;
                 if (l == 0)
-                    go(k_tile_down<T, R, NT, RW>, D.ntiles, D.nt, sm, L, TV, TileRhs<R>{r, rsum}, V[size_t(l + 1)].b,
+                    go(k_tile_down<T, R, NT, RW>, D.ntiles, D.nt, 0, L, TV, TileRhs<R>{r, rsum}, V[size_t(l + 1)].b,
                        L.bp);
                 else
-                    go(k_tile_down<T, T, NT, RW>, D.ntiles, D.nt, sm, L, TV, TileRhs<T>{L.b, nullptr},
+                    go(k_tile_down<T, T, NT, RW>, D.ntiles, D.nt, 0, L, TV, TileRhs<T>{L.b, nullptr},
                        V[size_t(l + 1)].b, (T*)nullptr);
             });
             ++launches_;
@@ -1039,7 +1027,7 @@ void DeviceSolver::enqueue_vcycle_epi(const R* r, const double* rsum, double* me
             const bool want_mean = (l == 0) && L.singular;
             with_tile_threads(D.nt, D.rows, [&](auto nt, auto rows) {
                 constexpr int NT = decltype(nt)::value, RW = decltype(rows)::value;
-                go(k_tile_up<T, Epi, NT, RW>, D.ntiles, D.nt, tile_smem<T>(D.n3max, D.n2max, D.n1max), L,
+                go(k_tile_up<T, Epi, NT, RW>, D.ntiles, D.nt, 0, L,
                    tile_view<T>(l), (const T*)V[size_t(l + 1)].x, (const T*)(l == 0 ? L.bp : L.b), fpartial_.p, counters_.p + kPostMean,
                    want_mean ? mean_out : nullptr, epi);
             });
@@ -1363,15 +1351,14 @@ double DeviceSolver::time_fused(int which, int level, int precision, int iters) 
         const TileView<T>& TV = tile_view<T>(level);
         with_tile_threads(D.nt, D.rows, [&](auto nt, auto rows) {
             constexpr int NT = decltype(nt)::value, RW = decltype(rows)::value;
-            const size_t sm = tile_smem<T>(D.n3max, D.n2max, D.n1max);
             if (which == 6 && level == 0)  // the finest level reads the FP64 residual, as in the cycle
-                k_tile_down<T, double, NT, RW><<<D.ntiles, D.nt, sm, stream_>>>(
+                k_tile_down<T, double, NT, RW><<<D.ntiles, D.nt, 0, stream_>>>(
                     L, TV, TileRhs<double>{r_.p, nullptr}, V[size_t(level + 1)].b, L.bp);
             else if (which == 6)
-                k_tile_down<T, T, NT, RW><<<D.ntiles, D.nt, sm, stream_>>>(L, TV, TileRhs<T>{L.b, nullptr},
+                k_tile_down<T, T, NT, RW><<<D.ntiles, D.nt, 0, stream_>>>(L, TV, TileRhs<T>{L.b, nullptr},
                                                                            V[size_t(level + 1)].b, (T*)nullptr);
             else
-                k_tile_up<T, MeanOnly, NT, RW><<<D.ntiles, D.nt, sm, stream_>>>(
+                k_tile_up<T, MeanOnly, NT, RW><<<D.ntiles, D.nt, 0, stream_>>>(
                     L, TV, (const T*)V[size_t(level + 1)].x, (const T*)(level == 0 ? L.bp : L.b), fpartial_.p,
                     counters_.p, nullptr, MeanOnly());
         });
@@ -1503,12 +1490,8 @@ void DeviceSolver::upload_tiles(const Hierarchy& h) {
         if (!T.ok) continue;
         TileDev& D = tdev_[size_t(l)];
         D.ntiles = T.ntiles;
-        D.n3max = T.n3max;
-        D.n2max = T.n2max;
-        D.n1max = T.n1max;
         D.rows = T.n2max > 1024 ? 2 : 1;
-        // a thread per ROWS rows and per ROWS + 1 cells
-        D.nt = (std::max((T.n2max + D.rows - 1) / D.rows, (T.n3max + D.rows) / (D.rows + 1)) + 31) & ~31;
+        D.nt = tile_threads(T.n3max, T.n2max, D.rows);
         D.nent = int(T.pos.size());
         D.info.upload(T.info.data(), T.info.size(), stream_);
         D.cell.upload(T.cell.data(), T.cell.size(), stream_);
@@ -1522,9 +1505,6 @@ void DeviceSolver::upload_tiles(const Hierarchy& h) {
         D.val_f.alloc(T.pos.size());
         TPA_CUDA(cudaStreamSynchronize(stream_));  // the host arrays go out of scope
         auto fill = [&](auto& v, auto* val) {
-            v.n3max = D.n3max;
-            v.n2max = D.n2max;
-            v.n1max = D.n1max;
             v.info = D.info.p;
             v.cell = D.cell.p;
             v.own = D.own.p;

@@ -30,6 +30,8 @@
 
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "fused.cuh"
 #include "stencil.cuh"
 #include "tiles.hpp"
@@ -50,14 +52,33 @@ struct TileView {
     const short* col;
     const int* co;
     const short4* ch;   // per coarse cell: local indices of its children (-1: none)
-    int n3max, n2max, n1max;
 };
 
-// Shared memory of a tile: the three vectors that rows read from one another.
-template <typename T>
-__host__ __device__ inline size_t tile_smem(int n3, int n2, int n1) {
-    return sizeof(T) * (size_t(n3) + size_t(n2) + size_t(n1));
+// threads of a tile: one per `rows` rows and per rows + 1 cells
+inline int tile_threads(int n3max, int n2max, int rows) {
+    const int by_rows = (n2max + rows - 1) / rows, by_cells = (n3max + rows) / (rows + 1);
+    return ((by_rows > by_cells ? by_rows : by_cells) + 31) & ~31;
 }
+
+// Kernel forms of a level's CSR tiles by the threads a tile takes (a thread per
+// row, rounded to warps): launch bounds that leave FP64 rows their registers on
+// 8 x 8 and 16 x 16 blocks, and two rows per thread beyond 1024.
+template <typename F>
+void with_tile_threads(int threads, int rows, F f) {
+    if (rows == 2) f(std::integral_constant<int, 1024>(), std::integral_constant<int, 2>());
+    else if (threads <= 256) f(std::integral_constant<int, 256>(), std::integral_constant<int, 1>());
+    else if (threads <= 640) f(std::integral_constant<int, 640>(), std::integral_constant<int, 1>());
+    else f(std::integral_constant<int, 1024>(), std::integral_constant<int, 1>());
+}
+
+// The three vectors that rows read from one another, at offsets known to the
+// compiler: cells (rings <= 3), then two of the rows.
+template <typename T, int NT, int ROWS>
+struct TileShared {
+    static constexpr int kCells = (ROWS + 1) * NT < kTileMaxCells ? (ROWS + 1) * NT : kTileMaxCells;
+    static constexpr int kRows = ROWS * NT < kTileMaxCells ? ROWS * NT : kTileMaxCells;
+    T a[kCells], b[kRows], c[kRows];
+};
 
 __device__ __forceinline__ TileInfo tile_info(const TileInfo* p) {
     const int4* q = reinterpret_cast<const int4*>(p);
@@ -117,13 +138,11 @@ struct TileRhs {
 // the coarse one; bp_out (null: not written, the cycle reads b itself) the
 // projected right-hand side for the up half; the pre-smoothed iterate goes to
 // L.y.  ROWS rows and ROWS + 1 cells per thread.
-template <typename T, int ROWS, typename Src>
+template <typename T, int NT, int ROWS, typename Src>
 __device__ __forceinline__ void tile_down(const LevelView<T>& L, const TileView<T>& V, const Src& src,
                                           T* bc, T* bp_out) {
-    extern __shared__ __align__(16) unsigned char tile_smem_raw[];
-    T* xa = reinterpret_cast<T*>(tile_smem_raw);
-    T* xb = xa + V.n3max;
-    T* ss = xb + V.n2max;
+    __shared__ TileShared<T, NT, ROWS> sm;
+    T *xa = sm.a, *xb = sm.b, *ss = sm.c;
     constexpr int CU = ROWS + 1;
     const TileInfo I = tile_info(V.info + blockIdx.x);
     const int nt = blockDim.x;
@@ -215,13 +234,11 @@ __device__ __forceinline__ void tile_down(const LevelView<T>& L, const TileView<
 // The up half: xc the coarse level's correction, bp_in the projected right-hand
 // side; out(g, x) takes the result of cell g and its value from `pre(g)`, which
 // is called before the wait (static data) and `late(g)` after it.
-template <typename T, int ROWS, typename Out>
+template <typename T, int NT, int ROWS, typename Out>
 __device__ __forceinline__ void tile_up(const LevelView<T>& L, const TileView<T>& V, const T* xc, const T* bp_in,
                                         Out& out) {
-    extern __shared__ __align__(16) unsigned char tile_smem_raw[];
-    T* e = reinterpret_cast<T*>(tile_smem_raw);
-    T* xp = e + V.n3max;
-    T* xq = xp + V.n2max;
+    __shared__ TileShared<T, NT, ROWS> sm;
+    T *e = sm.a, *xp = sm.b, *xq = sm.c;
     constexpr int CU = ROWS + 1;
     const TileInfo I = tile_info(V.info + blockIdx.x);
     const int nt = blockDim.x;
@@ -297,7 +314,7 @@ template <typename T, typename TB, int NT, int ROWS>
 __global__ void __launch_bounds__(NT, 1)
     k_tile_down(LevelView<T> L, TileView<T> V, TileRhs<TB> src, T* bc, T* bp_out) {
     pdl_launch();
-    tile_down<T, ROWS>(with_weights(L), V, src, bc, bp_out);
+    tile_down<T, NT, ROWS>(with_weights(L), V, src, bc, bp_out);
 }
 
 // What the up half of one solve's level does with its result: the sums of the
@@ -334,7 +351,7 @@ __global__ void __launch_bounds__(NT, 1)
               double* mean_out, Epi epi) {
     pdl_launch();
     TileMean<T, Epi, ROWS> out{L.vol, mean_out != nullptr, epi};
-    tile_up<T, ROWS>(with_weights(L), V, xc, bp_in, out);
+    tile_up<T, NT, ROWS>(with_weights(L), V, xc, bp_in, out);
     if (mean_out) fold_mean(out.v, out.w, partial, counter, mean_out, L.cvol_inv, epi);
 }
 
