@@ -103,34 +103,14 @@ struct BLevel {
 
 using BState = CgState;  // per-problem CG scalars
 
-// Publish N block values of item `blockIdx.x` (sums where max_mask bit k is 0,
-// maxima where it is 1; value k at partial[k * stride + item]); in the CTA that
-// completes the problem's items [first, first + count), thread 0 then calls
-// done(out) with their fixed-order folds.
+// N values folded over a problem's items [first, first + count); this CTA's item
+// is blockIdx.x, value k at partial[k * stride + item]
 template <int N, typename F>
 __device__ __forceinline__ void fold_problem(const double (&v)[N], unsigned max_mask, double* partial, int stride,
                                              unsigned* counter, int first, int count, F done) {
-    __shared__ bool last;
-    double b[N];
-    for (int k = 0; k < N; ++k) b[k] = (max_mask >> k) & 1 ? block_max_all(v[k]) : block_sum_all(v[k]);
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < N; ++k) partial[k * stride + blockIdx.x] = b[k];
-        __threadfence();
-        last = atomicAdd(counter, 1u) == unsigned(count) - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    double out[N];
-    for (int k = 0; k < N; ++k) {
-        out[k] = (max_mask >> k) & 1 ? fold_partials_max(partial + k * stride + first, count)
-                                     : fold_partials(partial + k * stride + first, count);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        *counter = 0;
-        done(out);
-    }
+    double* p[N];
+    for (int k = 0; k < N; ++k) p[k] = partial + k * stride;
+    fold_blocks<N>(v, max_mask, p, counter, blockIdx.x, first, count, done);
 }
 
 // ---- the tiled cycle ----------------------------------------------------------------

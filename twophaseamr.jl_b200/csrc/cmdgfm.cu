@@ -71,13 +71,9 @@ __global__ void k_cm_scatter(int64_t np, const double* __restrict__ src, const d
         v += q;
     }
     if (anchor < 0) return;
-    if (publish_partial(v, partial, counter)) {
-        const double t = fold_partials(partial, gridDim.x);
-        if (threadIdx.x == 0) {
-            full[anchor] = 0.0 - t;
-            *counter = 0;
-        }
-    }
+    fold_sum(v, partial, counter, [&](double t) {
+        full[anchor] = 0.0 - t;
+    });
 }
 
 // one block per anchor: full[anchor] = -(sum of its component's values)

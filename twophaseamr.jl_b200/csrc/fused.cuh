@@ -163,34 +163,88 @@ __device__ __forceinline__ double block_sum_all(double v) {
     return v;
 }
 
-// Write this block's partial, and return true in the block that finishes last.
-__device__ __forceinline__ bool publish_partial(double v, double* partial, unsigned* counter) {
+// the larger one; a NaN wins
+__device__ __forceinline__ double nan_max(double a, double b) { return a > b || a != a ? a : b; }
+
+constexpr int kWarpFold = 320;  // partials that one warp folds (10 loads in flight per lane)
+
+// N block values of item `item` (sums where max_mask bit k is 0, maxima with NaN
+// propagating where it is 1) into p[k][item]; the CTA that completes the items
+// [first, first + count) folds them in a fixed order and its thread 0 calls
+// done(out[N]).  The last statement of a kernel: one shared-memory exchange for
+// all values, then warp 0 alone publishes and (up to kWarpFold items) folds, so
+// that the other warps leave.  A block reduction per value and a CTA barrier
+// behind the atomic took 2 to 3 us of a CTA's time.
+// WARP = 0: the whole CTA folds whatever the count (the order of k_fold_sum).
+template <int N, int WARP = kWarpFold, typename F>
+__device__ __forceinline__ void fold_blocks(const double (&v)[N], unsigned max_mask, double* const* p,
+                                            unsigned* counter, int item, int first, int count, F done) {
+    __shared__ double sh[N][32];
     __shared__ bool last;
-    v = block_sum_all(v);
-    if (threadIdx.x == 0) {
-        partial[blockIdx.x] = v;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = int(blockDim.x >> 5);
+    auto join = [&](int k, double x, double y) { return (max_mask >> k) & 1 ? nan_max(x, y) : x + y; };
+    double b[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) b[k] = v[k];
+    auto warp = [&] {
+#pragma unroll
+        for (int o = 16; o; o >>= 1)
+#pragma unroll
+            for (int k = 0; k < N; ++k) b[k] = join(k, b[k], __shfl_down_sync(0xffffffffu, b[k], o));
+    };
+    auto block = [&] {  // the CTA's value in warp 0's lane 0
+        warp();
+        if (!lane)
+#pragma unroll
+            for (int k = 0; k < N; ++k) sh[k][wid] = b[k];
+        __syncthreads();
+        if (wid) return;
+#pragma unroll
+        for (int k = 0; k < N; ++k) b[k] = lane < nw ? sh[k][lane] : 0.0;
+        warp();
+    };
+    auto publish = [&] {  // thread 0
+#pragma unroll
+        for (int k = 0; k < N; ++k) p[k][item] = b[k];
         __threadfence();
-        unsigned t = atomicAdd(counter, 1u);
-        last = (t == gridDim.x - 1);
+        return atomicAdd(counter, 1u) == unsigned(count) - 1;
+    };
+    auto gather = [&](int from, int step) {
+        __threadfence();
+#pragma unroll
+        for (int k = 0; k < N; ++k) b[k] = 0;
+#pragma unroll 4
+        for (int i = from; i < count; i += step)
+#pragma unroll
+            for (int k = 0; k < N; ++k) b[k] = join(k, b[k], __ldcg(p[k] + first + i));
+    };
+    block();
+    if (count <= WARP) {
+        if (wid) return;
+        int l = 0;
+        if (!lane) l = publish() ? 1 : 0;
+        if (!__shfl_sync(0xffffffffu, l, 0)) return;
+        gather(lane, 32);
+        warp();
+    } else {
+        if (threadIdx.x == 0) last = publish();
+        __syncthreads();
+        if (!last) return;
+        gather(int(threadIdx.x), int(blockDim.x));
+        block();
     }
-    __syncthreads();
-    return last;
+    if (threadIdx.x == 0) {
+        *counter = 0;
+        done(b);
+    }
 }
 
-// publish_partial of two block sums (v into p1, w into p2) under one counter
-__device__ __forceinline__ bool publish_partial2(double v, double w, double* p1, double* p2, unsigned* counter) {
-    __shared__ bool last;
-    v = block_sum_all(v);
-    w = block_sum_all(w);
-    if (threadIdx.x == 0) {
-        p1[blockIdx.x] = v;
-        p2[blockIdx.x] = w;
-        __threadfence();
-        unsigned t = atomicAdd(counter, 1u);
-        last = (t == gridDim.x - 1);
-    }
-    __syncthreads();
-    return last;
+// one sum over the grid
+template <typename F>
+__device__ __forceinline__ void fold_sum(double v, double* partial, unsigned* counter, F done) {
+    const double a[1] = {v};
+    double* const p[1] = {partial};
+    fold_blocks<1>(a, 0u, p, counter, blockIdx.x, 0, gridDim.x, [&](const double (&t)[1]) { done(t[0]); });
 }
 
 // Epilogue of the finest level's last post-smoothing, which folds the volume
@@ -210,22 +264,15 @@ template <typename Epi>
 __device__ __forceinline__ void fold_mean(double v, double w, double* partial, unsigned* counter, double* mean_out,
                                           double cvol_inv, const Epi& epi) {
     if constexpr (Epi::kRz) {
-        if (publish_partial2(v, w, partial, epi.partial, counter)) {
-            const double s = fold_partials(partial, gridDim.x);
-            const double rx = fold_partials(epi.partial, gridDim.x);
-            if (threadIdx.x == 0) {
-                const double mean = s * cvol_inv;
-                *mean_out = mean;
-                epi(mean, rx);
-                *counter = 0;
-            }
-        }
-    } else if (publish_partial(v, partial, counter)) {
-        const double s = fold_partials(partial, gridDim.x);
-        if (threadIdx.x == 0) {
-            *mean_out = s * cvol_inv;
-            *counter = 0;
-        }
+        const double a[2] = {v, w};
+        double* const p[2] = {partial, epi.partial};
+        fold_blocks<2>(a, 0u, p, counter, blockIdx.x, 0, gridDim.x, [&](const double (&t)[2]) {
+            const double mean = t[0] * cvol_inv;
+            *mean_out = mean;
+            epi(mean, t[1]);
+        });
+    } else {
+        fold_sum(v, partial, counter, [&](double t) { *mean_out = t * cvol_inv; });
     }
 }
 
@@ -377,13 +424,9 @@ __global__ void k_rb_half(LevelView<T> L, const T* __restrict__ in, T* __restric
         v = double(L.vol[i]) * double(out[i]);
     }
     if (mean_out) {
-        if (publish_partial(v, partial, counter)) {
-            double s = fold_partials(partial, gridDim.x);
-            if (threadIdx.x == 0) {
-                *mean_out = s * L.cvol_inv;
-                *counter = 0;
-            }
-        }
+        fold_sum(v, partial, counter, [&](double s) {
+            *mean_out = s * L.cvol_inv;
+        });
     }
 }
 
@@ -411,13 +454,9 @@ __global__ void k_rb_pair(LevelView<T> L, const T* __restrict__ in, T* __restric
         v = double(L.vol[i]) * double(out[i]);
     }
     if (mean_out) {
-        if (publish_partial(v, partial, counter)) {
-            double s = fold_partials(partial, gridDim.x);
-            if (threadIdx.x == 0) {
-                *mean_out = s * L.cvol_inv;
-                *counter = 0;
-            }
-        }
+        fold_sum(v, partial, counter, [&](double s) {
+            *mean_out = s * L.cvol_inv;
+        });
     }
 }
 

@@ -34,33 +34,13 @@ namespace {
 constexpr int kGrid = 1184;  // 8 CTAs on each of 148 SMs
 constexpr int kCPrep = 8, kCPres = 9, kCMean = 10;
 
-// Publish N block values (sums where max_mask bit k is 0, maxima where it is 1)
-// and fold them in the last block in block order; its thread 0 calls done(out[N]).
-template <int N, typename F>
+// N values folded over the grid, value k in partial[k gridDim.x ..)
+template <int N, int WARP = kWarpFold, typename F>
 __device__ __forceinline__ void publish_fold(const double (&v)[N], unsigned max_mask, double* partial,
                                              unsigned* counter, F done) {
-    __shared__ bool last;
-    double b[N];
-    for (int k = 0; k < N; ++k) b[k] = (max_mask >> k) & 1 ? block_max_all(v[k]) : block_sum_all(v[k]);
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < N; ++k) partial[k * gridDim.x + blockIdx.x] = b[k];
-        __threadfence();
-        const unsigned t = atomicAdd(counter, 1u);
-        last = (t == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    double out[N];
-    for (int k = 0; k < N; ++k) {
-        out[k] = (max_mask >> k) & 1 ? fold_partials_max(partial + k * gridDim.x, gridDim.x)
-                                     : fold_partials(partial + k * gridDim.x, gridDim.x);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        *counter = 0;
-        done(out);
-    }
+    double* p[N];
+    for (int k = 0; k < N; ++k) p[k] = partial + k * gridDim.x;
+    fold_blocks<N, WARP>(v, max_mask, p, counter, blockIdx.x, 0, gridDim.x, done);
 }
 
 // sums of b = V f, |b| and V x0 over cells with V > 0; the means to remove.
@@ -78,7 +58,8 @@ __global__ void k_prep(int n, const double* __restrict__ rhs, const double* __re
         v[1] += fabs(bi);
         v[2] += V * xi;
     }
-    publish_fold<3>(v, 0u, partial, counter, [&](const double (&t)[3]) {
+    // in the order of the plain solve's sums: the removed mean is often rounding alone
+    publish_fold<3, 0>(v, 0u, partial, counter, [&](const double (&t)[3]) {
         S->sum_b = t[0];
         S->abs_b = t[1];
         const bool comp = q.cvol != 0;

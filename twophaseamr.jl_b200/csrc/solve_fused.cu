@@ -88,26 +88,18 @@ __global__ void k_cg_residual(LevelView<double> A, const double* __restrict__ b,
         r[i] = ri;
         v += ri;
     }
-    if (publish_partial(v, partial, counter)) {
-        double t = fold_partials(partial, gridDim.x);
-        if (threadIdx.x == 0) {
-            s->rsum = t;
-            *counter = 0;
-        }
-    }
+    fold_sum(v, partial, counter, [&](double t) {
+        s->rsum = t;
+    });
 }
 
 __global__ void k_sum_into(int n, const double* __restrict__ v, double* partial, unsigned* counter, double* out) {
     pdl_entry();
     double acc = 0;
     TPA_GRID_STRIDE(i, n) acc += v[i];
-    if (publish_partial(acc, partial, counter)) {
-        double t = fold_partials(partial, gridDim.x);
-        if (threadIdx.x == 0) {
-            *out = t;
-            *counter = 0;
-        }
-    }
+    fold_sum(acc, partial, counter, [&](double t) {
+        *out = t;
+    });
 }
 
 __device__ __forceinline__ void alpha_from(double pAp, CgState* s) {
@@ -149,13 +141,9 @@ __global__ void k_cg_ap(LevelView<double> A, const double* __restrict__ p, doubl
         ap[i] = y;
         v += p[i] * y;
     }
-    if (publish_partial(v, partial, counter)) {
-        double pAp = fold_partials(partial, gridDim.x);
-        if (threadIdx.x == 0) {
-            alpha_from(pAp, s);
-            *counter = 0;
-        }
-    }
+    fold_sum(v, partial, counter, [&](double pAp) {
+        alpha_from(pAp, s);
+    });
 }
 
 // Search directions of iteration `iter` in the ping-pong pair (pa, pb): the
@@ -180,7 +168,6 @@ __global__ void k_cg_update(int n, double* __restrict__ x, P* __restrict__ r, P*
                             unsigned* counter, CgState* s, cudaGraphConditionalHandle handle, int set_cond) {
     pdl_entry();
     const P* __restrict__ p = dir_new(pa, pb, s->iter);
-    __shared__ bool last;
     const bool skip = s->flags & kCgHalt;
     const double alpha = s->alpha;
     double m = 0, sum = 0;
@@ -201,46 +188,13 @@ __global__ void k_cg_update(int n, double* __restrict__ x, P* __restrict__ r, P*
         }
         sum += ri;
     }
-    // block max (NaN propagating) and block sum
-    __shared__ double shm[32], shs[32];
-    __shared__ int nan_seen;
-    if (threadIdx.x == 0) nan_seen = 0;
-    __syncthreads();
-    if (nan) nan_seen = 1;
-    double mm = m, ss = sum;
-    for (int o = 16; o; o >>= 1) {
-        mm = fmax(mm, __shfl_down_sync(0xffffffffu, mm, o));
-        ss += __shfl_down_sync(0xffffffffu, ss, o);
-    }
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (!lane) {
-        shm[wid] = mm;
-        shs[wid] = ss;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double bm = 0, bs = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-            bm = fmax(bm, shm[w]);
-            bs += shs[w];
-        }
-        pmax[blockIdx.x] = nan_seen ? NAN : bm;
-        psum[blockIdx.x] = bs;
-        __threadfence();
-        unsigned t = atomicAdd(counter, 1u);
-        last = (t == gridDim.x - 1);
-    }
-    __syncthreads();
-    if (last) {
-        double mx = fold_partials_max(pmax, gridDim.x);
-        double sm = fold_partials(psum, gridDim.x);
-        if (threadIdx.x == 0) {
-            s->strong_max = mx;
-            s->rsum = sm;
-            *counter = 0;
-            cg_after_update(s, skip, handle, set_cond);
-        }
-    }
+    const double a[2] = {nan ? NAN : m, sum};
+    double* const folds[2] = {pmax, psum};
+    fold_blocks<2>(a, 1u, folds, counter, blockIdx.x, 0, gridDim.x, [&](const double (&t)[2]) {
+        s->strong_max = t[0];
+        s->rsum = t[1];
+        cg_after_update(s, skip, handle, set_cond);
+    });
 }
 
 // block-structured finest level: Ap = A p and alpha
@@ -264,13 +218,9 @@ __global__ void s_cg_residual(SView<double> L, const double* __restrict__ b, con
         r[c] = v;
         part += v;
     }
-    if (publish_partial(part, partial, counter)) {
-        double tt = fold_partials(partial, gridDim.x);
-        if (threadIdx.x == 0) {
-            s->rsum = tt;
-            *counter = 0;
-        }
-    }
+    fold_sum(part, partial, counter, [&](double tt) {
+        s->rsum = tt;
+    });
 }
 
 // constant-coefficient 16x16 finest level: Ap = A p and alpha (vectorized quads)
@@ -303,13 +253,9 @@ __global__ void __launch_bounds__(256) v_cg_residual(SView<double> L, const doub
         }
         q_st(r + p.c, rr);
     }
-    if (publish_partial(part, partial, counter)) {
-        double tt = fold_partials(partial, gridDim.x);
-        if (threadIdx.x == 0) {
-            s->rsum = tt;
-            *counter = 0;
-        }
-    }
+    fold_sum(part, partial, counter, [&](double tt) {
+        s->rsum = tt;
+    });
 }
 
 template <typename T, typename F>
@@ -339,13 +285,9 @@ __global__ void k_cg_z(int n, const T* __restrict__ xv, const double* mean, cons
     }
     for (int i = 4 * nq + blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         v += double(r[i]) * (double(xv[i]) - m);
-    if (publish_partial(v, partial, counter)) {
-        double g = fold_partials(partial, gridDim.x);
-        if (threadIdx.x == 0) {
-            *counter = 0;
-            cg_after_z(s, g);
-        }
-    }
+    fold_sum(v, partial, counter, [&](double g) {
+        cg_after_z(s, g);
+    });
 }
 
 // gamma_next = g = r'z from the V-cycle at the start of a loop body.  The
@@ -458,13 +400,9 @@ __global__ void k_cg_dir_ap(LevelView<double> A, const T* xv, const double* mean
         ap[i] = P(y);
         v += pi * y;
     }
-    if (publish_partial(v, partial, counter)) {
-        double pAp = fold_partials(partial, gridDim.x);
-        if (threadIdx.x == 0) {
-            alpha_from(pAp, s);
-            *counter = 0;
-        }
-    }
+    fold_sum(v, partial, counter, [&](double pAp) {
+        alpha_from(pAp, s);
+    });
 }
 
 // the same on a block-structured finest level
@@ -574,13 +512,9 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCgCtas)
             }
         }
     }
-    if (publish_partial(part, partial, counter)) {
-        const double sum = fold_partials(partial, gridDim.x);
-        if (threadIdx.x == 0) {
-            alpha_from(sum, s);
-            *counter = 0;
-        }
-    }
+    fold_sum(part, partial, counter, [&](double sum) {
+        alpha_from(sum, s);
+    });
 }
 
 // Start of an inner run of the refinement solve: the FP64 true residual
@@ -595,13 +529,9 @@ __global__ void k_ir_start(int n, const double* __restrict__ r, float* __restric
         r32[i] = ri;
         v += double(ri);
     }
-    if (publish_partial(v, partial, counter)) {
-        const double t = fold_partials(partial, gridDim.x);
-        if (threadIdx.x == 0) {
-            s->rsum = t;
-            *counter = 0;
-        }
-    }
+    fold_sum(v, partial, counter, [&](double t) {
+        s->rsum = t;
+    });
 }
 
 // the loop is entered unless the set-up found nothing to solve

@@ -9,27 +9,6 @@
 
 namespace tpa {
 
-__device__ __forceinline__ double block_max_all(double v) {
-    __shared__ double sh[32];
-    __shared__ int nan_seen;
-    bool nan = v != v;
-    double m = nan ? 0.0 : v;
-    for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    __syncthreads();
-    if (threadIdx.x == 0) nan_seen = 0;
-    __syncthreads();
-    if (nan) nan_seen = 1;
-    if (!lane) sh[wid] = m;
-    __syncthreads();
-    m = 0;
-    if (threadIdx.x < (blockDim.x >> 5)) m = sh[threadIdx.x];
-    if (wid == 0)
-        for (int o = 16; o; o >>= 1) m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
-    __syncthreads();
-    return nan_seen ? NAN : m;
-}
-
 constexpr double kEps = 2.220446049250313e-16;
 
 // std::max's choice, a NaN in second place included

@@ -218,13 +218,9 @@ __device__ __forceinline__ void s_apply_dot(const SView<T>& L, const T* x, T* y,
         y[c] = v;
         part += double(x[c]) * double(v);
     }
-    if (publish_partial(part, partial, counter)) {
-        double s = fold_partials(partial, gridDim.x);
-        if (threadIdx.x == 0) {
-            fold(s);
-            *counter = 0;
-        }
-    }
+    fold_sum(part, partial, counter, [&](double s) {
+        fold(s);
+    });
 }
 
 // s_apply_dot with the operand formed where it is read: ld(q) = x_q, and
@@ -242,13 +238,9 @@ __device__ __forceinline__ void s_apply_dot_ld(const SView<T>& L, Ld ld, Keep ke
         y[c] = P(v);
         part += double(xc) * double(v);
     }
-    if (publish_partial(part, partial, counter)) {
-        double s = fold_partials(partial, gridDim.x);
-        if (threadIdx.x == 0) {
-            fold(s);
-            *counter = 0;
-        }
-    }
+    fold_sum(part, partial, counter, [&](double s) {
+        fold(s);
+    });
 }
 
 #undef TPA_S_CELL

@@ -406,13 +406,9 @@ __device__ __forceinline__ void v_apply_dot(const SView<double>& L, const double
         q_st(y + p.c, ax);
         for (int m = 0; m < 4; ++m) part += g.x.v[m] * ax.v[m];
     }
-    if (publish_partial(part, partial, counter)) {
-        const double s = fold_partials(partial, gridDim.x);
-        if (threadIdx.x == 0) {
-            fold(s);
-            *counter = 0;
-        }
-    }
+    fold_sum(part, partial, counter, [&](double s) {
+        fold(s);
+    });
 }
 
 // v_apply_dot with the operand formed where it is read: ld(c) is the quad of
@@ -435,13 +431,9 @@ __device__ __forceinline__ void v_apply_dot_ld(const SView<double>& L, Ld ld, P*
         q_st(y + p.c, ax);
         for (int m = 0; m < 4; ++m) part += g.x.v[m] * ax.v[m];
     }
-    if (publish_partial(part, partial, counter)) {
-        const double s = fold_partials(partial, gridDim.x);
-        if (threadIdx.x == 0) {
-            fold(s);
-            *counter = 0;
-        }
-    }
+    fold_sum(part, partial, counter, [&](double s) {
+        fold(s);
+    });
 }
 
 #undef TPA_Q_LOOP
