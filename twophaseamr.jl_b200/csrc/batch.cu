@@ -20,9 +20,10 @@ namespace {
 
 // ---- fine-space FP64 kernels (one BFItem per CTA) --------------------------------
 
-// the slice of this thread's row (item blockIdx.x, row threadIdx.x of it)
-__device__ __forceinline__ int2 fine_slice(const FineRows& A) {
-    return ld_static(A.slice + size_t(blockIdx.x) * (kItemRows / 32) + (threadIdx.x >> 5));
+// the slice of this thread's q-th row (row q kItemRows + threadIdx.x of item blockIdx.x)
+__device__ __forceinline__ int2 fine_slice(const FineRows& A, int q) {
+    return ld_static(A.slice + size_t(blockIdx.x) * (kFineRows / 32) + size_t(q) * (kItemRows / 32) +
+                     (threadIdx.x >> 5));
 }
 
 __device__ __forceinline__ BFItem fine_item(const BFItem* fi) {
@@ -42,14 +43,16 @@ __global__ void bk_prep(const BFItem* fi, FineFold f, const double* __restrict__
                         const double* __restrict__ xin, const double* __restrict__ comp_vol, SolveAsk q,
                         SolveState* S) {
     const BFItem it = fine_item(fi);
-    const int i = it.begin + int(threadIdx.x);
     double v[3] = {0, 0, 0};
-    if (i < it.end) {
+#pragma unroll
+    for (int q4 = 0; q4 < kFinePer; ++q4) {
+        const int i = it.begin + q4 * kItemRows + int(threadIdx.x);
+        if (i >= it.end) continue;
         const double V = vol[i];
         const double bi = V > 0 ? rhs[i] * V : 0.0, xi = V > 0 ? xin[i] : 0.0;
-        v[0] = bi;
-        v[1] = fabs(bi);
-        v[2] = V * xi;
+        v[0] += bi;
+        v[1] += fabs(bi);
+        v[2] += V * xi;
     }
     fine_fold<3>(f, v, 0u, it.prob, [&](const double (&t)[3]) {
         SolveState& s = S[it.prob];
@@ -74,12 +77,13 @@ template <bool First>
 __global__ void bk_pres(const BFItem* fi, FineFold f, FineRows A, const double* rhs, const double* xin, double* b,
                         double* xout, double* r, SolveAsk q, SolveState* S, BState* st, int* active) {
     const BFItem it = fine_item(fi);
-    const int2 sl = fine_slice(A);
     const SolveState& s = S[it.prob];
     const double m = First ? s.mx : s.xm, mb = First ? s.mb : 0.0;
-    const int i = it.begin + int(threadIdx.x);
     double v[5] = {0, 0, 0, 0, 0};
-    if (i < it.end) {
+    for (int q4 = 0; q4 < kFinePer; ++q4) {
+        const int i = it.begin + q4 * kItemRows + int(threadIdx.x);
+        if (i >= it.end) continue;
+        const int2 sl = fine_slice(A, q4);
         const double V = A.vol[i];
         double bi;
         if (First) {
@@ -93,6 +97,7 @@ __global__ void bk_pres(const BFItem* fi, FineFold f, FineRows A, const double* 
         double acc = 0, aacc = 0;
         const int* ci = A.ci + sl.x + (threadIdx.x & 31);
         const double* val = A.val + sl.x + (threadIdx.x & 31);
+#pragma unroll 4
         for (int u = 0; u < sl.y; ++u) {
             const int j = ci[32 * u];
             const double a = val[32 * u];
@@ -103,12 +108,12 @@ __global__ void bk_pres(const BFItem* fi, FineFold f, FineRows A, const double* 
         xout[i] = xi;
         const double ri = bi - acc;
         r[i] = ri;
-        v[4] = ri;
+        v[4] += ri;
         if (V > 0) {
-            v[0] = ri * ri / V;
-            v[1] = ri != ri ? NAN : fabs(ri) / V;
-            v[2] = aacc / V;
-            v[3] = fabs(bi) / V;
+            v[0] += ri * ri / V;
+            v[1] = nan_max(v[1], fabs(ri) / V);
+            v[2] = nan_max(v[2], aacc / V);
+            v[3] = nan_max(v[3], fabs(bi) / V);
         }
     }
     fine_fold<5>(f, v, 0xEu, it.prob, [&](const double (&t)[5]) {
@@ -128,8 +133,12 @@ __global__ void bk_pres(const BFItem* fi, FineFold f, FineRows A, const double* 
 __global__ void bk_xmean(const BFItem* fi, FineFold f, const double* __restrict__ vol, const double* x,
                          const double* __restrict__ comp_vol, SolveState* S) {
     const BFItem it = fine_item(fi);
-    const int i = it.begin + int(threadIdx.x);
-    const double v[1] = {i < it.end ? vol[i] * x[i] : 0.0};
+    double v[1] = {0};
+#pragma unroll
+    for (int q4 = 0; q4 < kFinePer; ++q4) {
+        const int i = it.begin + q4 * kItemRows + int(threadIdx.x);
+        if (i < it.end) v[0] += vol[i] * x[i];
+    }
     fine_fold<1>(f, v, 0u, it.prob, [&](const double (&t)[1]) {
         const double cv = comp_vol[it.prob];
         S[it.prob].xm = cv > 0 && S[it.prob].ok ? t[0] / cv : 0.0;
@@ -154,59 +163,81 @@ __device__ __forceinline__ void balpha(double pAp, BState* s) {
     }
 }
 
-// Ap = A p and alpha; a row's first 8 entries in flight before the wait
+// Ap = A p and alpha; the first row's entries (up to 8) in flight before the wait
 __global__ void __launch_bounds__(kItemRows)
     bk_cg_ap(const BFItem* fi, FineFold f, FineRows A, const double* p, double* ap, BState* st, const int* active) {
     pdl_launch();
     const BFItem it = fine_item(fi);
-    const int2 sl = fine_slice(A);
-    const int* ci = A.ci + sl.x + (threadIdx.x & 31);
-    const double* val = A.val + sl.x + (threadIdx.x & 31);
     constexpr int kPre = 8;
     int c[kPre];
     double a[kPre];
+    int2 sl;
+    auto load = [&](int q) {
+        sl = fine_slice(A, q);
 #pragma unroll
-    for (int u = 0; u < kPre; ++u)
-        if (u < sl.y) {
-            c[u] = ld_static(ci + 32 * u);
-            a[u] = ld_static(val + 32 * u);
-        }
+        for (int u = 0; u < kPre; ++u)
+            if (u < sl.y) {
+                c[u] = ld_static(A.ci + sl.x + 32 * u + (threadIdx.x & 31));
+                a[u] = ld_static(A.val + sl.x + 32 * u + (threadIdx.x & 31));
+            }
+    };
+    load(0);
     pdl_wait();
     if (!active[it.prob]) return;
-    const int i = it.begin + int(threadIdx.x);
     double v[1] = {0};
-    if (i < it.end) {
+    for (int q = 0; q < kFinePer; ++q) {
+        const int i = it.begin + q * kItemRows + int(threadIdx.x);
+        if (q) load(q);
+        if (i >= it.end) continue;
         double y = 0;
 #pragma unroll
         for (int u = 0; u < kPre; ++u)
             if (u < sl.y) y += a[u] * p[c[u]];
-        for (int u = kPre; u < sl.y; ++u) y += val[32 * u] * p[ci[32 * u]];
+        for (int u = kPre; u < sl.y; ++u)
+            y += A.val[sl.x + 32 * u + (threadIdx.x & 31)] * p[A.ci[sl.x + 32 * u + (threadIdx.x & 31)]];
         ap[i] = y;
-        v[0] = p[i] * y;
+        v[0] += p[i] * y;
     }
     fine_fold<1>(f, v, 0u, it.prob, [&](const double (&t)[1]) { balpha(t[0], st + it.prob); });
 }
 
-__global__ void bk_cg_update(const BFItem* fi, FineFold f, const double* __restrict__ vol, double* x, double* r,
-                             const double* p, const double* ap, BState* st, const int* active) {
+__global__ void __launch_bounds__(kItemRows)
+    bk_cg_update(const BFItem* fi, FineFold f, const double* __restrict__ vol, double* x, double* r, const double* p,
+                 const double* ap, BState* st, const int* active) {
     pdl_launch();
     const BFItem it = fine_item(fi);
-    const int i = it.begin + int(threadIdx.x);
-    const double V = i < it.end ? ld_static(vol + i) : 0.0;
+    double V[kFinePer];
+#pragma unroll
+    for (int q = 0; q < kFinePer; ++q) {
+        const int i = it.begin + q * kItemRows + int(threadIdx.x);
+        V[q] = i < it.end ? ld_static(vol + i) : 0.0;
+    }
     pdl_wait();
     if (!active[it.prob]) return;
     const bool skip = st[it.prob].flags & 2;
     const double alpha = st[it.prob].alpha;
+    double ri[kFinePer], xi[kFinePer], pi[kFinePer], ai[kFinePer];
+#pragma unroll
+    for (int q = 0; q < kFinePer; ++q) {
+        const int i = it.begin + q * kItemRows + int(threadIdx.x);
+        if (i >= it.end) continue;
+        ri[q] = r[i];
+        xi[q] = x[i];
+        pi[q] = p[i];
+        ai[q] = ap[i];
+    }
     double v[2] = {0, 0};
-    if (i < it.end) {
-        double ri = r[i];
+#pragma unroll
+    for (int q = 0; q < kFinePer; ++q) {
+        const int i = it.begin + q * kItemRows + int(threadIdx.x);
+        if (i >= it.end) continue;
         if (!skip) {
-            x[i] += alpha * p[i];
-            ri -= alpha * ap[i];
-            r[i] = ri;
+            x[i] = xi[q] + alpha * pi[q];
+            ri[q] -= alpha * ai[q];
+            r[i] = ri[q];
         }
-        if (V > 0) v[0] = ri != ri ? NAN : fabs(ri) / V;
-        v[1] = ri;
+        if (V[q] > 0) v[0] = nan_max(v[0], fabs(ri[q]) / V[q]);
+        v[1] += ri[q];
     }
     fine_fold<2>(f, v, 1u, it.prob, [&](const double (&t)[2]) {
         st[it.prob].strong_max = t[0];
@@ -216,8 +247,9 @@ __global__ void bk_cg_update(const BFItem* fi, FineFold f, const double* __restr
 
 // p = z + beta p, z = V-cycle output - mean (not stored); a run's first: p = z
 template <typename T>
-__global__ void bk_cg_p(const BFItem* fi, const BLevel<T>* __restrict__ lv, const double* mean, double* p,
-                        const BState* st, const int* active) {
+__global__ void __launch_bounds__(kItemRows)
+    bk_cg_p(const BFItem* fi, const BLevel<T>* __restrict__ lv, const double* mean, double* p, const BState* st,
+            const int* active) {
     pdl_launch();
     const BFItem it = fine_item(fi);
     const T* xv = lv[it.lvl].x;
@@ -225,10 +257,15 @@ __global__ void bk_cg_p(const BFItem* fi, const BLevel<T>* __restrict__ lv, cons
     if (!active[it.prob]) return;
     const BState& s = st[it.prob];
     if (s.flags & 6) return;
-    const int i = it.begin + int(threadIdx.x);
-    if (i >= it.end) return;
-    const double z = double(xv[i + it.off]) - mean[it.prob];
-    p[i] = s.iter == 0 ? z : z + s.beta * p[i];
+    const double m = mean[it.prob], beta = s.beta;
+    const bool fresh = s.iter == 0;
+#pragma unroll
+    for (int q = 0; q < kFinePer; ++q) {
+        const int i = it.begin + q * kItemRows + int(threadIdx.x);
+        if (i >= it.end) continue;
+        const double z = double(xv[i + it.off]) - m;
+        p[i] = fresh ? z : z + beta * p[i];
+    }
 }
 
 // loop condition of the graph: any problem still iterating
@@ -468,8 +505,8 @@ void BatchSolver::build(const std::vector<const Hierarchy*>& hs) {
             const Csr& A = h.levels[0].op.A;
             const int F = int(F_[size_t(k)]);
             pf[size_t(k)] = int(fi.size());
-            for (int64_t b = 0; b < A.n; b += kItemRows)
-                fi.push_back(BFItem{F + int(b), F + int(std::min<int64_t>(A.n, b + kItemRows)), k, j,
+            for (int64_t b = 0; b < A.n; b += kFineRows)
+                fi.push_back(BFItem{F + int(b), F + int(std::min<int64_t>(A.n, b + kFineRows)), k, j,
                                     int(M[size_t(j)][size_t(k)]) - F});
             pc[size_t(k)] = int(fi.size()) - pf[size_t(k)];
             comp_vol_.push_back(h.levels[0].op.singular ? h.levels[0].op.comp.volume[0] : 0.0);
@@ -482,7 +519,7 @@ void BatchSolver::build(const std::vector<const Hierarchy*>& hs) {
         for (const BFItem& it : fi) {
             const Csr& A = hs[size_t(it.prob)]->levels[0].op.A;
             const int F = int(F_[size_t(it.prob)]);
-            for (int b = 0; b < kItemRows; b += 32) {
+            for (int b = 0; b < kFineRows; b += 32) {
                 int width = 0;
                 for (int i = it.begin + b; i < std::min(it.end, it.begin + b + 32); ++i)
                     width = std::max<int>(width, int(A.ptr[size_t(i - F) + 1] - A.ptr[size_t(i - F)]));
@@ -500,8 +537,8 @@ void BatchSolver::build(const std::vector<const Hierarchy*>& hs) {
             const HostLevel& hl = hs[size_t(it.prob)]->levels[0];
             const Csr& A = hl.op.A;
             const int F = int(F_[size_t(it.prob)]);
-            for (int b = 0; b < kItemRows; b += 32) {
-                const size_t sl = 2 * (q * (kItemRows / 32) + size_t(b / 32));
+            for (int b = 0; b < kFineRows; b += 32) {
+                const size_t sl = 2 * (q * (kFineRows / 32) + size_t(b / 32));
                 for (int r = 0; r < 32; ++r) {
                     const int i = it.begin + b + r;
                     const bool in = i < it.end;

@@ -44,7 +44,11 @@ struct BItem {
     int begin, end, prob, delta;
 };
 
-// a finest-level item of the CG (fine-space rows [begin, end); level row = row + off)
+// A finest-level item of the CG (fine-space rows [begin, end); level row = row +
+// off): kFineRows rows, each thread's kFinePer of them kItemRows apart, so that
+// a fold (a fence and an atomic per item) is paid once per 1024 rows.
+constexpr int kFinePer = 4;
+constexpr int kFineRows = kFinePer * kItemRows;
 struct BFItem {
     int begin, end, prob, lvl, off;
 };

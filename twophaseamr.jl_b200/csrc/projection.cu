@@ -247,6 +247,7 @@ void DeviceSolver::upload_projection(const Mesh& mesh, const std::vector<double>
     proj_phi_.alloc(size_t(n));
     proj_in_.alloc(size_t(std::max<int64_t>(nf, 1)));
     perr_.alloc(1);
+    TPA_CUDA(cudaMemsetAsync(perr_.p, 0, sizeof(int), stream_));
     const DevLevel& L = levels_[0];
     if (L.ncomp > 1) {
         proj_part_.alloc(size_t(kMaxComponents) * size_t(kReduceBlocks));
@@ -261,14 +262,16 @@ void DeviceSolver::conditional_fraction(const double* raw, double floor, double*
     if (!(std::isfinite(floor) && floor > 0 && floor < 0.5))
         throw Error(1, "fraction_floor must be finite and in (0, 0.5)");
     const int n = ncells();
-    int err = 0;
-    TPA_CUDA(cudaMemsetAsync(perr_.p, 0, sizeof(int), stream_));
+    // the flag is zero between calls; it comes back through pinned memory
+    int* err = reinterpret_cast<int*>(host_d_);
     kp_conditional<<<pgrid(n), kPThreads, 0, stream_>>>(n, raw, floor, physical, conditional, perr_.p);
     TPA_CUDA(cudaGetLastError());
     ++launches_;
-    TPA_CUDA(cudaMemcpyAsync(&err, perr_.p, sizeof(int), cudaMemcpyDeviceToHost, stream_));
+    TPA_CUDA(cudaMemcpyAsync(err, perr_.p, sizeof(int), cudaMemcpyDeviceToHost, stream_));
     TPA_CUDA(cudaStreamSynchronize(stream_));
-    if (err) throw Error(1, "volume fractions must be finite and lie in [0, 1]");
+    if (!*err) return;
+    TPA_CUDA(cudaMemsetAsync(perr_.p, 0, sizeof(int), stream_));
+    throw Error(1, "volume fractions must be finite and lie in [0, 1]");
 }
 
 void DeviceSolver::face_coefficients(const double* conditional, double rho_l, double rho_g, double* kappa) {

@@ -25,15 +25,13 @@ namespace tpa {
 // the strip height of a row-streamed level: the one whose rounds of resident
 // warps (ctas CTAs per SM) walk the fewest rows, the taller on a tie
 // (strips of `cols` interior columns; `frame` rows walked besides the interior)
-// (`shallow`: the short strips of 8 and 4 rows too, for the small levels,
-// where a strip's walk is the kernel's time)
-static int stream_rows(int nbx, int nby, int sms, int ctas, int cols = kStreamCols, int frame = 6,
-                       bool shallow = true) {
+// (the short strips of 8 and 4 rows serve the small levels, where a strip's walk
+// is the kernel's time)
+static int stream_rows(int nbx, int nby, int sms, int ctas, int cols = kStreamCols, int frame = 6) {
     const int64_t slots = int64_t(ctas) * kStreamWarps * sms;
     int best = 0;
     int64_t cost = 0;
     for (int rows : {36, 24, 16, 8, 4}) {
-        if (!shallow && rows < 16) break;
         const int64_t strips = int64_t((16 * nbx + cols - 1) / cols) * ((16 * nby + rows - 1) / rows);
         const int64_t c = (strips + slots - 1) / slots * (rows + frame);
         if (!best || c < cost) {
@@ -56,7 +54,9 @@ static void with_stream_rows(int rows, F f) {
 // the strip heights of the streamed CG direction kernel (finest level)
 template <typename F>
 static void with_cg_rows(int rows, F f) {
-    if (rows == 16) f(std::integral_constant<int, 16>{});
+    if (rows == 4) f(std::integral_constant<int, 4>{});
+    else if (rows == 8) f(std::integral_constant<int, 8>{});
+    else if (rows == 16) f(std::integral_constant<int, 16>{});
     else if (rows == 24) f(std::integral_constant<int, 24>{});
     else f(std::integral_constant<int, 36>{});
 }
@@ -75,6 +75,7 @@ constexpr int kMaxGrid = 1184;
 // of 2^19 cells is 2048 tiles, under two resident waves of 256-thread CTAs;
 // the next level up streams HBM at a rate the tiles' index arithmetic cannot
 // keep.
+constexpr int kRzCells = 1 << 20;  // rz_foldable
 constexpr int kStencilTileCells = 1 << 19;  // 8 CTAs on each of 148 SMs: bounds the partials every fold reads
 #define TPA_GRID_STRIDE(i, n) for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += gridDim.x * blockDim.x)
 
@@ -171,24 +172,36 @@ __global__ void k_cg_update(int n, double* __restrict__ x, P* __restrict__ r, P*
     const bool skip = s->flags & kCgHalt;
     const double alpha = s->alpha;
     double m = 0, sum = 0;
-    bool nan = false;
-    TPA_GRID_STRIDE(i, n) {
-        double ri = double(r[i]);
+    // two cells' loads in flight per thread
+    const int step = gridDim.x * blockDim.x;
+    for (int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 2 * step) {
+        const int i1 = i0 + step, j1 = i1 < n ? i1 : i0;
+        double ri[2] = {double(r[i0]), double(r[j1])};
+        double V[2] = {vol0, vol0};
+        if (vol) {
+            V[0] = vol[i0];
+            V[1] = vol[j1];
+        }
         if (!skip) {
-            x[i] += alpha * double(p[i]);
-            const P rs = P(ri - alpha * double(ap[i]));
-            r[i] = rs;
-            ri = double(rs);
+            const double p0 = double(p[i0]), p1 = double(p[j1]), a0 = double(ap[i0]), a1 = double(ap[j1]);
+            const double x0 = x[i0], x1 = x[j1];
+            const P r0 = P(ri[0] - alpha * a0), r1 = P(ri[1] - alpha * a1);
+            x[i0] = x0 + alpha * p0;
+            r[i0] = r0;
+            if (i1 < n) {
+                x[i1] = x1 + alpha * p1;
+                r[i1] = r1;
+            }
+            ri[0] = double(r0);
+            ri[1] = double(r1);
         }
-        double V = vol ? vol[i] : vol0;
-        if (V > 0) {
-            double q = fabs(ri) / V;
-            if (q != q) nan = true;
-            m = fmax(m, q);
+        for (int q = 0; q < 2; ++q) {
+            if (q && i1 >= n) break;
+            if (V[q] > 0) m = nan_max(m, fabs(ri[q]) / V[q]);
+            sum += ri[q];
         }
-        sum += ri;
     }
-    const double a[2] = {nan ? NAN : m, sum};
+    const double a[2] = {m, sum};
     double* const folds[2] = {pmax, psum};
     fold_blocks<2>(a, 1u, folds, counter, blockIdx.x, 0, gridDim.x, [&](const double (&t)[2]) {
         s->strong_max = t[0];
@@ -324,9 +337,10 @@ __device__ void cg_after_z(CgState* s, double g) {
 // r'z folded into the finest post-smoothing of the CG loop's V-cycle:
 // r'z = sum r_i (x_i - mean) = sum r_i x_i - mean sum r_i, with sum r_i from
 // the x / r update (s->rsum)
+template <typename R>
 struct CgRz {
     static constexpr bool kRz = true;
-    const double* r;
+    const R* r;
     double* partial;
     CgState* s;
     __device__ void operator()(double mean, double rx) const { cg_after_z(s, rx - mean * s->rsum); }
@@ -889,11 +903,11 @@ void DeviceSolver::enqueue_vcycle_epi(const R* r, const double* rsum, double* me
         // the tail as one dense product (tail_dense.cuh)
         const int grid = (dense_n_ + kDenseRows - 1) / kDenseRows;
         if (t == 0)
-            go(k_tail_dense<T, R>, grid, 32 * kDenseRows, 0, dense_n_, dense_ld_, (const double*)dense_M_.p, r,
-               V[0].x, tail_mean);
+            go(k_tail_dense<T, R, Epi>, grid, 32 * kDenseRows, 0, dense_n_, dense_ld_, (const double*)dense_M_.p, r,
+               V[0].x, tail_mean, counters_.p + kPostMean, epi);
         else
-            go(k_tail_dense<T, T>, grid, 32 * kDenseRows, 0, dense_n_, dense_ld_, (const double*)dense_M_.p,
-               (const T*)V[size_t(t)].b, V[size_t(t)].x, nullptr);
+            go(k_tail_dense<T, T, MeanOnly>, grid, 32 * kDenseRows, 0, dense_n_, dense_ld_,
+               (const double*)dense_M_.p, (const T*)V[size_t(t)].b, V[size_t(t)].x, nullptr, nullptr, MeanOnly());
     } else {
         const Launch gt{stream_, pdl_, tail_ctas_};
         gt(k_tail<T, R>, tail_ctas_, kTailThreads, 0, Vdev, t, nl, t == 0 ? r : nullptr, coarse_inv_.p, coarse_n_,
@@ -1030,10 +1044,10 @@ void DeviceSolver::enqueue_cg_body(int precision, cudaGraphConditionalHandle han
         using T = std::remove_pointer_t<decltype(xv)>;
         using P = std::remove_pointer_t<decltype(r)>;
         // z = M r and r'z (beta, or the start of a run)
-        if (std::is_same<P, double>::value && rz_foldable()) {
+        if (rz_foldable()) {
             // r'z in the V-cycle's last kernel
-            const CgRz epi{r_.p, fpartial2_.p, s};
-            enqueue_vcycle_epi<T>(r_.p, &s->rsum, mean, epi);
+            const CgRz<P> epi{r, fpartial2_.p, s};
+            enqueue_vcycle_epi<T>((const P*)r, &s->rsum, mean, epi);
         } else {
             enqueue_vcycle<T>((const P*)r, &s->rsum, mean);
             go(k_cg_z<T, P>, fold_grid(k_cg_z<T, P>, kThreads, blocks_for((n + 3) / 4), kMaxGrid), kThreads, 0, n,
@@ -1077,21 +1091,21 @@ void DeviceSolver::enqueue_cg_body(int precision, cudaGraphConditionalHandle han
     TPA_CUDA(cudaGetLastError());
 }
 
-// The finest level is a CSR level swept by the multi-CTA kernels (not the tail
-// or the cooperative cycle), with the damped-Jacobi post-smoothing, and is
-// singular (its last post-smoothing folds the mean): r'z can ride on that fold.
-// The structured and vectorized post-smoothings can carry it too (s_post2,
-// v_sweep take the epilogue), but their folding grids are capped and stride
-// over the level.  On the vectorized 2048^2 level the extra r stream cost more
-// than the separate pass it replaces (3.35 -> 3.38 ms), and the structured
-// kernel, with the same capped grid, is left out with it.  The CSR
-// post-smoothing has one thread per cell and gains (droplet: 2.56 -> 2.49 ms).
-// The row-streamed finest level (v_stream_up) takes the epilogue as well, but
-// its r loads raised the kernel from 21.6 to 34-35 µs on 2048^2, plain or
-// staged by cp.async, about what the separate pass costs (12.8 µs); it is left
-// out too.
+// r'z rides on the V-cycle's last kernel, which folds the mean (singular level,
+// damped Jacobi, not the cooperative cycle): the up tiles and the CSR
+// post-smoothing of a CSR finest level, the dense product when the whole
+// hierarchy is the tail, and the streamed or tiled up kernel of a small
+// constant-coefficient level.  Above kRzCells a streamed level's extra r loads
+// cost what the separate pass takes (2048^2: the up kernel 21 -> 34 us, plain or
+// staged by cp.async, the pass 12.8 us); below, the pass is a launch's latency
+// (periodic 128^2 FP64: see kRzCells).  The vectorized and structured
+// post-smoothings (v_sweep, s_post2) have capped grids that stride over the
+// level and lost by it (2048^2: 3.35 -> 3.38 ms).
 bool DeviceSolver::rz_foldable() const {
-    return tail_first_ > 0 && coop_grid_ == 0 && !rb_ && levels_[0].ncomp == 1 && !sdev_.empty() && !sdev_[0].on;
+    if (coop_grid_ > 0 || rb_ || levels_[0].ncomp != 1 || sdev_.empty()) return false;
+    if (tail_first_ == 0) return dense_n_ > 0;
+    if (!sdev_[0].on) return true;
+    return tdev_.size() && (tdev_[0].stream || tdev_[0].vec) && levels_[0].n <= kRzCells;
 }
 
 cudaGraphExec_t DeviceSolver::cg_graph(int precision) {
@@ -1127,7 +1141,7 @@ cudaGraphExec_t DeviceSolver::cg_graph(int precision) {
     cudaError_t ce = cudaStreamEndCapture(stream_, &captured);
     stream_ = saved;
     // + direction/Ap, update and (unless folded) z
-    graph_body_launches_[precision] = launches_ - saved_launches + (precision < 2 && rz_foldable() ? 2 : 3);
+    graph_body_launches_[precision] = launches_ - saved_launches + (rz_foldable() ? 2 : 3);
     launches_ = saved_launches;
     if (ce != cudaSuccess) {
         cudaGraphDestroy(g);
@@ -1406,7 +1420,7 @@ void DeviceSolver::upload_tiles(const Hierarchy& h) {
                                                           int64_t(ctas) * sms));
                 }
             if (D.stream && l == 0) {  // the CG's direction and operator product on the finest level
-                D.cg_rows = stream_rows(sdev_[0].snbx, sdev_[0].snby, sms, kStreamCgCtas, kStreamCgCols, 2, false);
+                D.cg_rows = stream_rows(sdev_[0].snbx, sdev_[0].snby, sms, kStreamCgCtas, kStreamCgCols, 2);
                 const StreamGeom g = stream_cg_geom();
                 D.cg_grid = int(std::min<int64_t>((int64_t(g.nsx) * g.nsy + kStreamWarps - 1) / kStreamWarps,
                                                   int64_t(kStreamCgCtas) * sms));

@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(256) v_sweep(SView<T> L, const T* __restrict__
             const Quad<T> v = L.const_vol ? Quad<T>{{L.vol0, L.vol0, L.vol0, L.vol0}} : q_ld(L.vol + p.c);
             for (int m = 0; m < 4; ++m) part += double(v.v[m]) * double(o.v[m]);
             if constexpr (Epi::kRz) {
-                const Quad<double> rq = q_ldv(epi.r + p.c);
+                const auto rq = q_ldv(epi.r + p.c);
                 for (int m = 0; m < 4; ++m) rx += rq.v[m] * double(o.v[m]);
             }
         }

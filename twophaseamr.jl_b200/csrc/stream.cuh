@@ -28,6 +28,8 @@
 
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "stencil4.cuh"
 
 namespace tpa {
@@ -205,6 +207,17 @@ __global__ void __launch_bounds__(kStreamWarps * 32, stream_ctas_per_sm<T>())
             stage_row(k);
             st_commit();
         }
+        // the rows of r for the epilogue, in flight together on short strips
+        using ER = std::remove_cv_t<std::remove_pointer_t<decltype(epi.r)>>;
+        constexpr int RR = Epi::kRz && ROWS <= 8 ? ROWS : 1;
+        P2<ER> rr[RR];
+        if constexpr (Epi::kRz && ROWS <= 8)
+            if (mean_out) {
+#pragma unroll
+                for (int k = 0; k < ROWS; ++k)
+                    if (out_col && y0 + k < H)
+                        rr[k] = *reinterpret_cast<const P2<ER>*>(epi.r + st_cell(g, gx, y0 + k));
+            }
         P2<T> e[S], y[S], b[S], p[S], q[S];
 #pragma unroll
         for (int k = 0; k < S; ++k) {
@@ -236,8 +249,11 @@ __global__ void __launch_bounds__(kStreamWarps * 32, stream_ctas_per_sm<T>())
                         v += double(L.vol0) * double(o.l);
                         v += double(L.vol0) * double(o.r);
                         if constexpr (Epi::kRz) {
-                            w += epi.r[c] * double(o.l);
-                            w += epi.r[c + 1] * double(o.r);
+                            P2<ER> rq;
+                            if constexpr (ROWS <= 8) rq = rr[j - 3];
+                            else rq = *reinterpret_cast<const P2<ER>*>(epi.r + c);
+                            w += double(rq.l) * double(o.l);
+                            w += double(rq.r) * double(o.r);
                         }
                     }
                 }

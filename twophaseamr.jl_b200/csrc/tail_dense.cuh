@@ -170,11 +170,13 @@ __global__ void __launch_bounds__(kDenseBuildThreads)
 // x = M b: a warp per row, the row's first 1024 entries in flight before the
 // wait (M is written by set-up only, and the host waits for it before any
 // V-cycle is launched), b staged in shared memory once per CTA.  mean_out (may
-// be null): the whole hierarchy is the tail and M removes the mean itself.
+// be null): the whole hierarchy is the tail and M removes the mean itself; the
+// CG's epilogue then takes r'x.
 // Bound by the latency of one launch, the load of b and the warp sum.
-template <typename T, typename TB>
+template <typename T, typename TB, typename Epi>
 __global__ void __launch_bounds__(32 * kDenseRows)
-    k_tail_dense(int n, int ld, const double* __restrict__ M, const TB* b, T* x, double* mean_out) {
+    k_tail_dense(int n, int ld, const double* __restrict__ M, const TB* b, T* x, double* mean_out,
+                 unsigned* counter, Epi epi) {
     pdl_launch();
     constexpr int kChunk = 2048;
     __shared__ __align__(16) double sb[kChunk];
@@ -213,6 +215,10 @@ __global__ void __launch_bounds__(32 * kDenseRows)
     for (int o = 16; o; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
     if (!lane && row < n) x[row] = T(s);
     if (mean_out && blockIdx.x == 0 && threadIdx.x == 0) *mean_out = 0.0;
+    if constexpr (Epi::kRz) {
+        const double rx = !lane && row < n ? double(epi.r[row]) * double(T(s)) : 0.0;
+        fold_sum(rx, epi.partial, counter, [&](double t) { epi(0.0, t); });
+    }
 }
 
 }  // namespace tpa

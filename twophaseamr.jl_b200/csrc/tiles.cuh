@@ -333,7 +333,7 @@ struct TileMean {
     __device__ __forceinline__ bool start() const { return true; }
     __device__ __forceinline__ void after(int q, int g, bool own) {
         if constexpr (Epi::kRz)
-            if (on && own) rv[q] = epi.r[g];
+            if (on && own) rv[q] = double(epi.r[g]);
     }
     __device__ __forceinline__ void take(int q, double x) {
         if (!on) return;
@@ -601,7 +601,7 @@ __global__ void __launch_bounds__(kTileThreads)
         L.x[c] = o;
         if (mean_out) {
             v += (L.const_vol ? double(L.vol0) : double(L.vol[c])) * double(o);
-            if constexpr (Epi::kRz) w += epi.r[c] * double(o);
+            if constexpr (Epi::kRz) w += double(epi.r[c]) * double(o);
         }
     }
     if (mean_out) fold_mean(v, w, partial, counter, mean_out, L.cvol_inv, epi);
