@@ -18,6 +18,8 @@
 #include <cstring>
 
 #include "cmdgfm.cuh"
+#include "fused.cuh"
+#include "launch.cuh"
 
 namespace tpa {
 namespace {
@@ -58,28 +60,51 @@ __device__ __forceinline__ double nan_max(double a, double b) { return (a != a |
 
 // ---------------------------------------------------------------- preconditioner
 
+// The kernels of one BiCGSTAB iteration are short (3-10 us on the 25,000
+// unknowns of a level-6 wave front) and each depends on the one before, so the
+// iteration is bound by launches and load latencies, not by its bytes.  The
+// iteration therefore has as few kernels as its reductions allow: dot products
+// ride on the product that makes their operand, and the scalars they give are
+// folded again by every CTA of the kernel that needs them (in the same order,
+// so each CTA has the same value); one CTA stores them.  Each kernel is a
+// programmatic dependent launch that loads its share of the system (pointers,
+// columns, values, scales: written before the loop) and waits only then.  What
+// the loop writes is read through plain pointers.  With 22 launches per
+// iteration besides the V-cycles' own, a projection of that front took 4.51 ms;
+// with these 11, 4.04 ms.
+
 // full[cell_i] = src_i / rows_i (the reduced right-hand side scattered); with
 // one component (anchor >= 0) the last block also writes full[anchor] = -(the
-// sum of the values), folded from per-block partials in block order
-__global__ void k_cm_scatter(int64_t np, const double* __restrict__ src, const double* __restrict__ rows,
-                             const int32_t* __restrict__ cell, double* __restrict__ full, int anchor,
-                             double* partial, unsigned* counter) {
+// sum of the values), folded from per-block partials in block order, and the
+// sum of the whole, which is then zero unless a value is not finite
+__global__ void k_cm_scatter(int64_t np, const double* src, const double* rows, const int32_t* cell, double* full,
+                             int anchor, double* partial, unsigned* counter, double* total) {
+    pdl_launch();
+    const int64_t i0 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    int32_t c0 = 0;
+    double r0 = 1.0;
+    if (i0 < np) {
+        c0 = ld_static(cell + i0);
+        r0 = ld_static(rows + i0);
+    }
+    pdl_wait();
     double v = 0;
     CM_LOOP(i, np) {
-        const double q = src[i] / rows[i];
-        full[cell[i]] = q;
+        const double q = src[i] / (i == i0 ? r0 : rows[i]);
+        full[i == i0 ? c0 : cell[i]] = q;
         v += q;
     }
     if (anchor < 0) return;
     fold_sum(v, partial, counter, [&](double t) {
         full[anchor] = 0.0 - t;
+        if (total) *total = t + (0.0 - t);
     });
 }
 
 // one block per anchor: full[anchor] = -(sum of its component's values)
-__global__ void k_cm_anchor(const int32_t* __restrict__ gptr, const int32_t* __restrict__ gidx,
-                            const int32_t* __restrict__ ganchor, const double* __restrict__ src,
-                            const double* __restrict__ rows, double* __restrict__ full) {
+__global__ void k_cm_anchor(const int32_t* gptr, const int32_t* gidx, const int32_t* ganchor, const double* src,
+                            const double* rows, double* full) {
+    pdl_entry();
     const int g = blockIdx.x;
     double v = 0;
     for (int k = gptr[g] + threadIdx.x; k < gptr[g + 1]; k += blockDim.x) {
@@ -90,14 +115,28 @@ __global__ void k_cm_anchor(const int32_t* __restrict__ gptr, const int32_t* __r
     if (threadIdx.x == 0) full[ganchor[g]] = 0.0 - v;
 }
 
-// zp_i = z[cell_i] - z[anchor_i]; dst_i = zp_i / cols_i
-__global__ void k_cm_gather(int64_t np, const double* __restrict__ z, const int32_t* __restrict__ cell,
-                            const int32_t* __restrict__ anchor, const double* __restrict__ cols,
-                            double* __restrict__ zp, double* __restrict__ dst) {
+// zp_i = z[cell_i] - z[anchor_i]; dst_i = zp_i / cols_i, z the V-cycle's result
+// less its volume mean (read where the cycle left it: a pass that stores z
+// first took 2.5 us and its launch)
+template <typename T>
+__global__ void k_cm_gather(int64_t np, const T* x, const double* mean, const int32_t* cell, const int32_t* anchor,
+                            const double* cols, double* zp, double* dst) {
+    pdl_launch();
+    const int64_t i0 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    int32_t c0 = 0, a0 = 0;
+    double s0 = 1.0;
+    if (i0 < np) {
+        c0 = ld_static(cell + i0);
+        a0 = ld_static(anchor + i0);
+        s0 = ld_static(cols + i0);
+    }
+    pdl_wait();
+    const double m = mean ? *mean : 0.0;
     CM_LOOP(i, np) {
-        const double v = z[cell[i]] - z[anchor[i]];
+        const bool first = i == i0;
+        const double v = (double(x[first ? c0 : cell[i]]) - m) - (double(x[first ? a0 : anchor[i]]) - m);
         zp[i] = v;
-        dst[i] = v / cols[i];
+        dst[i] = v / (first ? s0 : cols[i]);
     }
 }
 
@@ -221,10 +260,10 @@ __device__ void tri_solve(const TriView& t, double* __restrict__ y, int nx) {
 // C zp, y = (L U)^-1 jr, dst_xi = y / D_c.  The vector lives in shared
 // memory, and the factors too when `staged`.
 __global__ void __launch_bounds__(kIluThreads)
-    k_cm_jump_solve(int nx, int64_t np, const double* __restrict__ src, const double* __restrict__ rows,
-                    const int64_t* __restrict__ cptr, const int32_t* __restrict__ ccol,
-                    const double* __restrict__ cval, const double* __restrict__ zp, TriView L, TriView U,
-                    int staged, const double* __restrict__ cols, double* __restrict__ dst) {
+    k_cm_jump_solve(int nx, int64_t np, const double* src, const double* rows, const int64_t* cptr,
+                    const int32_t* ccol, const double* cval, const double* zp, TriView L, TriView U, int staged,
+                    const double* cols, double* dst) {
+    pdl_entry();
     extern __shared__ double sm[];
     double* y = sm;
     for (int f = threadIdx.x; f < nx; f += blockDim.x) {
@@ -267,50 +306,176 @@ __global__ void __launch_bounds__(kIluThreads)
 
 // The jump block through the factors' inverses (triangular_inverses): jr =
 // src_xi / D_r - C zp, y = L^-1 jr, x = U^-1 y, dst_xi = x / D_c, each a
-// row-parallel product; one CTA, jr and y in shared memory.
+// row-parallel product; one CTA, jr and y in shared memory.  Bound by the
+// chain of loads along a row and from product to product, not by the 12,700
+// entries of a level-6 wave front.  So a row is taken by as many lanes (`shift`:
+// log2) as let one pass cover all rows, its bounds, its scales and the first
+// entries of its C row are loaded before the wait, and so are both inverses,
+// into shared memory, when they fit (`staged`).  By itself the kernel takes
+// 9.9 us on that front (a thread per row with nothing loaded ahead: 9.7 us;
+// eight lanes a row in four passes: 18.4 us), but its loads run beside the
+// kernel before it: the solve's 46 products of this kind and all else on the
+// device took 2.91 ms with it, 3.53 ms with the eight lanes.
 __global__ void __launch_bounds__(kIluThreads)
-    k_cm_jump_inverse(int nx, int64_t np, const double* __restrict__ src, const double* __restrict__ rows,
-                      const int64_t* __restrict__ cptr, const int32_t* __restrict__ ccol,
-                      const double* __restrict__ cval, const double* __restrict__ zp,
-                      const int64_t* __restrict__ lptr, const int32_t* __restrict__ lcol,
-                      const double* __restrict__ lval, const int64_t* __restrict__ uptr,
-                      const int32_t* __restrict__ ucol, const double* __restrict__ uval,
-                      const double* __restrict__ cols, double* __restrict__ dst) {
+    k_cm_jump_inverse(int nx, int64_t np, int shift, int staged, int lnnz, int unnz, const double* src,
+                      const double* rows, const int64_t* cptr, const int32_t* ccol, const double* cval,
+                      const double* zp, const int64_t* lptr, const int32_t* lcol, const double* lval,
+                      const int64_t* uptr, const int32_t* ucol, const double* uval, const double* cols, double* dst) {
+    constexpr int kHeld = 4;
+    pdl_launch();
     extern __shared__ double sm[];
     double* a = sm;
     double* b = sm + nx;
-    for (int f = threadIdx.x; f < nx; f += blockDim.x) {
+    const int lanes = 1 << shift, lane = threadIdx.x & (lanes - 1);
+    const int f0 = threadIdx.x >> shift;
+    int64_t c0 = 0, c1 = 0, l0 = 0, l1 = 0, u0 = 0, u1 = 0;
+    double scale_in = 1.0, scale_out = 1.0;
+    if (f0 < nx) {
+        c0 = ld_static(cptr + f0);
+        c1 = ld_static(cptr + f0 + 1);
+        l0 = ld_static(lptr + f0);
+        l1 = ld_static(lptr + f0 + 1);
+        u0 = ld_static(uptr + f0);
+        u1 = ld_static(uptr + f0 + 1);
+        scale_in = ld_static(rows + np + f0);
+        scale_out = ld_static(cols + np + f0);
+    }
+    if (staged) {
+        double* lv = b + nx;
+        double* uv = lv + lnnz;
+        int32_t* lc = reinterpret_cast<int32_t*>(uv + unnz);
+        int32_t* uc = lc + lnnz;
+#pragma unroll 4
+        for (int e = threadIdx.x; e < lnnz; e += kIluThreads) {
+            lv[e] = ld_static(lval + e);
+            lc[e] = ld_static(lcol + e);
+        }
+#pragma unroll 4
+        for (int e = threadIdx.x; e < unnz; e += kIluThreads) {
+            uv[e] = ld_static(uval + e);
+            uc[e] = ld_static(ucol + e);
+        }
+        lval = lv;
+        lcol = lc;
+        uval = uv;
+        ucol = uc;
+    }
+    int32_t hc[kHeld];
+    double hv[kHeld];
+#pragma unroll
+    for (int k = 0; k < kHeld; ++k) {
+        const int64_t e = c0 + lane + (k << shift);
+        hc[k] = e < c1 ? ld_static(ccol + e) : 0;
+        hv[k] = e < c1 ? ld_static(cval + e) : 0.0;
+    }
+    pdl_wait();
+    // this lane's part of a row, kHeld entries in flight; summed over the row's lanes
+    auto along = [&](int64_t e0, int64_t e1, const int32_t* col, const double* val, const double* v) {
         double acc = 0;
-        for (int64_t e = cptr[f]; e < cptr[f + 1]; ++e) acc += cval[e] * zp[ccol[e]];
-        a[f] = src[np + f] / rows[np + f] - acc;
+        for (int64_t e = e0 + lane; e < e1; e += int64_t(kHeld) << shift) {
+            double t[kHeld];
+#pragma unroll
+            for (int k = 0; k < kHeld; ++k) {
+                const int64_t q = e + (k << shift);
+                t[k] = q < e1 ? val[q] * v[col[q]] : 0.0;
+            }
+#pragma unroll
+            for (int k = 0; k < kHeld; ++k) acc += t[k];
+        }
+        return acc;
+    };
+    // every lane of a warp takes the same trips, so that the shuffles see all of them
+    auto total = [&](double acc) {
+        for (int o = lanes >> 1; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        return acc;
+    };
+    const int step = kIluThreads >> shift;
+    for (int base = 0; base < nx; base += step) {
+        const int f = base + f0;
+        double acc = 0;
+        if (base == 0) {
+#pragma unroll
+            for (int k = 0; k < kHeld; ++k)
+                if (c0 + lane + (k << shift) < c1) acc += hv[k] * zp[hc[k]];
+            acc += along(c0 + (int64_t(kHeld) << shift), c1, ccol, cval, zp);
+        } else if (f < nx) {
+            acc = along(cptr[f], cptr[f + 1], ccol, cval, zp);
+        }
+        acc = total(acc);
+        if (f < nx && lane == 0) a[f] = src[np + f] / (base ? rows[np + f] : scale_in) - acc;
     }
     __syncthreads();
-    for (int f = threadIdx.x; f < nx; f += blockDim.x) {
+    for (int base = 0; base < nx; base += step) {
+        const int f = base + f0;
         double acc = 0;
-        for (int64_t e = lptr[f]; e < lptr[f + 1]; ++e) acc += lval[e] * a[lcol[e]];
-        b[f] = acc;
+        if (f < nx) acc = along(base ? lptr[f] : l0, base ? lptr[f + 1] : l1, lcol, lval, a);
+        acc = total(acc);
+        if (f < nx && lane == 0) b[f] = acc;
     }
     __syncthreads();
-    for (int f = threadIdx.x; f < nx; f += blockDim.x) {
+    for (int base = 0; base < nx; base += step) {
+        const int f = base + f0;
         double acc = 0;
-        for (int64_t e = uptr[f]; e < uptr[f + 1]; ++e) acc += uval[e] * b[ucol[e]];
-        dst[np + f] = acc / cols[np + f];
+        if (f < nx) acc = along(base ? uptr[f] : u0, base ? uptr[f + 1] : u1, ucol, uval, b);
+        acc = total(acc);
+        if (f < nx && lane == 0) dst[np + f] = acc / (base ? cols[np + f] : scale_out);
     }
 }
 
 // ---------------------------------------------------------------- products
 
-// y = D_r M (D_c x) (scaled) or y = M x (rows, cols null)
-__global__ void k_cm_spmv(int64_t n, const int64_t* __restrict__ ptr, const int32_t* __restrict__ col,
-                          const double* __restrict__ val, const double* __restrict__ rows,
-                          const double* __restrict__ cols, const double* __restrict__ x, double* __restrict__ y) {
-    CM_LOOP(i, n) {
+// y = A x with A = D_r M D_c, and with it the block partials of c'y (p1) and,
+// with `yy`, of y'y (p2): a row per thread, whose pointers, scale and first
+// kHeld entries -- the whole row of a cell away from the front -- are loaded
+// before the wait, so that only x is read after it
+__global__ void __launch_bounds__(kT)
+    k_cm_product(int64_t n, const int64_t* ptr, const int32_t* col, const double* val, const double* rows,
+                 const double* cols, const double* x, double* y, const double* c, int yy, double* p1, double* p2) {
+    constexpr int kHeld = 6;
+    pdl_launch();
+    int32_t hc[kHeld];
+    double hv[kHeld], hs[kHeld];
+    int64_t e0 = 0, e1 = 0;
+    double scale = 0;
+    const int64_t i0 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i0 < n) {
+        e0 = ld_static(ptr + i0);
+        e1 = ld_static(ptr + i0 + 1);
+        scale = ld_static(rows + i0);
+    }
+#pragma unroll
+    for (int k = 0; k < kHeld; ++k) {
+        const bool in = e0 + k < e1;
+        hc[k] = in ? ld_static(col + e0 + k) : 0;
+        hv[k] = in ? ld_static(val + e0 + k) : 0.0;
+    }
+#pragma unroll
+    for (int k = 0; k < kHeld; ++k) hs[k] = e0 + k < e1 ? ld_static(cols + hc[k]) : 0.0;
+    pdl_wait();
+    double v = 0, w = 0;
+    auto put = [&](int64_t i, double yi) {
+        y[i] = yi;
+        v += c[i] * yi;
+        if (yy) w += yi * yi;
+    };
+    if (i0 < n) {
         double acc = 0;
-        if (cols)
-            for (int64_t e = ptr[i]; e < ptr[i + 1]; ++e) acc += val[e] * (cols[col[e]] * x[col[e]]);
-        else
-            for (int64_t e = ptr[i]; e < ptr[i + 1]; ++e) acc += val[e] * x[col[e]];
-        y[i] = rows ? rows[i] * acc : acc;
+#pragma unroll
+        for (int k = 0; k < kHeld; ++k)
+            if (e0 + k < e1) acc += hv[k] * (hs[k] * x[hc[k]]);
+        for (int64_t e = e0 + kHeld; e < e1; ++e) acc += val[e] * (cols[col[e]] * x[col[e]]);
+        put(i0, scale * acc);
+    }
+    for (int64_t i = i0 + int64_t(gridDim.x) * blockDim.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
+        double acc = 0;
+        for (int64_t e = ptr[i]; e < ptr[i + 1]; ++e) acc += val[e] * (cols[col[e]] * x[col[e]]);
+        put(i, rows[i] * acc);
+    }
+    v = block_sum_all(v);
+    if (yy) w = block_sum_all(w);
+    if (threadIdx.x == 0) {
+        p1[blockIdx.x] = v;
+        if (yy) p2[blockIdx.x] = w;
     }
 }
 
@@ -325,21 +490,12 @@ __global__ void k_cm_residual(int64_t n, const int64_t* __restrict__ ptr, const 
     }
 }
 
-// block partials of a'b and c'd (c, d may be null)
-__global__ void k_cm_dot2(int64_t n, const double* __restrict__ a, const double* __restrict__ b,
-                          const double* __restrict__ c, const double* __restrict__ d, double* __restrict__ p1,
-                          double* __restrict__ p2) {
-    double v = 0, w = 0;
-    CM_LOOP(i, n) {
-        v += a[i] * b[i];
-        if (c) w += c[i] * d[i];
-    }
+// block partials of a'a
+__global__ void k_cm_norm2(int64_t n, const double* __restrict__ a, double* __restrict__ p1) {
+    double v = 0;
+    CM_LOOP(i, n) v += a[i] * a[i];
     v = block_sum_all(v);
-    if (c) w = block_sum_all(w);
-    if (threadIdx.x == 0) {
-        p1[blockIdx.x] = v;
-        if (c) p2[blockIdx.x] = w;
-    }
+    if (threadIdx.x == 0) p1[blockIdx.x] = v;
 }
 
 // ---------------------------------------------------------------- BiCGSTAB
@@ -380,39 +536,42 @@ __global__ void k_cm_init_fold(const double* p1, int count, double rtol, int itm
     }
 }
 
-// rho = next_rho; alpha = rho / c'v
-__global__ void k_cm_alpha(const double* p1, int count, double* st) {
-    const double cv = fold_partials(p1, count);
-    if (threadIdx.x == 0) {
-        st[kRho] = st[kNextRho];
-        st[kAlpha] = st[kRho] / cv;
-    }
+// a fold's value, which thread 0 holds, handed to every thread of the CTA
+__device__ __forceinline__ double to_all(double v) {
+    __shared__ double one;
+    __syncthreads();
+    if (threadIdx.x == 0) one = v;
+    __syncthreads();
+    return one;
 }
 
+// rho = next_rho; alpha = rho / c'v (from the partials p1)
 // s = r - alpha v; x = x + alpha y
-__global__ void k_cm_update1(int64_t n, const double* __restrict__ r, const double* __restrict__ v,
-                             const double* __restrict__ y, double* __restrict__ s, double* __restrict__ x,
-                             const double* __restrict__ st) {
-    const double a = st[kAlpha];
+__global__ void k_cm_update1(int64_t n, const double* p1, int count, const double* r, const double* v,
+                             const double* y, double* s, double* x, double* st) {
+    pdl_entry();
+    const double rho = st[kNextRho];
+    const double a = rho / to_all(fold_partials(p1, count));
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        st[kRho] = rho;
+        st[kAlpha] = a;
+    }
     CM_LOOP(i, n) {
         s[i] = r[i] - a * v[i];
         x[i] = x[i] + a * y[i];
     }
 }
 
-// omega = t's / t't
-__global__ void k_cm_omega(const double* p1, const double* p2, int count, double* st) {
+// omega = t's / t't (from the partials p1, p2)
+// x = x + omega z; r = s - omega t; partials of c'r (p3) and r'r (p4)
+__global__ void k_cm_update2(int64_t n, const double* p1, const double* p2, int count, const double* s,
+                             const double* t, const double* z, const double* c, double* x, double* r, double* st,
+                             double* p3, double* p4) {
+    pdl_entry();
     const double ts = fold_partials(p1, count);
     const double tt = fold_partials(p2, count);
-    if (threadIdx.x == 0) st[kOmega] = ts / tt;
-}
-
-// x = x + omega z; r = s - omega t; partials of c'r and r'r
-__global__ void k_cm_update2(int64_t n, const double* __restrict__ s, const double* __restrict__ t,
-                             const double* __restrict__ z, const double* __restrict__ c, double* __restrict__ x,
-                             double* __restrict__ r, const double* __restrict__ st, double* __restrict__ p1,
-                             double* __restrict__ p2) {
-    const double w = st[kOmega];
+    const double w = to_all(ts / tt);
+    if (blockIdx.x == 0 && threadIdx.x == 0) st[kOmega] = w;
     double cr = 0, rr = 0;
     CM_LOOP(i, n) {
         x[i] = x[i] + w * z[i];
@@ -424,19 +583,26 @@ __global__ void k_cm_update2(int64_t n, const double* __restrict__ s, const doub
     cr = block_sum_all(cr);
     rr = block_sum_all(rr);
     if (threadIdx.x == 0) {
-        p1[blockIdx.x] = cr;
-        p2[blockIdx.x] = rr;
+        p3[blockIdx.x] = cr;
+        p4[blockIdx.x] = rr;
     }
 }
 
-// next_rho, beta, rNorm and the stopping rules of the iteration
-__global__ void k_cm_rho(const double* p1, const double* p2, int count, double* st,
-                         cudaGraphConditionalHandle handle, int set_cond) {
-    const double cr = fold_partials(p1, count);
-    const double rr = fold_partials(p2, count);
+// next_rho, beta, rNorm and the stopping rules of the iteration (from the
+// partials p3, p4), which one CTA stores; p = r + beta (p - omega v)
+__global__ void k_cm_pupdate(int64_t n, const double* p3, const double* p4, int count, const double* r,
+                             const double* v, double* p, double* st, cudaGraphConditionalHandle handle,
+                             int set_cond) {
+    pdl_entry();
+    const double a = st[kAlpha], w = st[kOmega];
+    const double cr = to_all(fold_partials(p3, count));
+    const double b = (cr / st[kRho]) * (a / w);
+    CM_LOOP(i, n) p[i] = r[i] + b * (p[i] - w * v[i]);
+    if (blockIdx.x != 0) return;
+    const double rr = fold_partials(p4, count);
     if (threadIdx.x == 0) {
         st[kNextRho] = cr;
-        st[kBeta] = (cr / st[kRho]) * (st[kAlpha] / st[kOmega]);
+        st[kBeta] = b;
         const double rnorm = sqrt(rr);
         st[kRnorm] = rnorm;
         const double iter = st[kIter] + 1;
@@ -444,18 +610,10 @@ __global__ void k_cm_rho(const double* p1, const double* p2, int count, double* 
         int flags = 0;
         if (rnorm <= st[kEps] || rnorm + 1.0 <= 1.0) flags |= kSolved;
         if (iter >= st[kItmax]) flags |= kTired;
-        const double a = st[kAlpha];
         if (a == 0.0 || a != a) flags |= kBreakdown;
         st[kFlags] = flags;
         if (set_cond) cudaGraphSetConditional(handle, (flags & (kSolved | kTired | kBreakdown)) ? 0u : 1u);
     }
-}
-
-// p = r + beta (p - omega v)
-__global__ void k_cm_pupdate(int64_t n, const double* __restrict__ r, const double* __restrict__ v,
-                             double* __restrict__ p, const double* __restrict__ st) {
-    const double b = st[kBeta], w = st[kOmega];
-    CM_LOOP(i, n) p[i] = r[i] + b * (p[i] - w * v[i]);
 }
 
 // ---------------------------------------------------------------- residual replacement
@@ -585,35 +743,37 @@ __global__ void k_cm_sum_fold(const double* p1, int count, double* out) {
 
 // ---------------------------------------------------------------- host driver
 
-void CmdgfmDevice::spmv(const double* x, double* y, int mode, cudaStream_t s) {
-    // mode 1: the scaled system D_r M D_c; 0: M
-    k_cm_spmv<<<grid_of(n_), kT, 0, s>>>(n_, mptr_.p, mcol_.p, mval_.p, mode ? rows_.p : nullptr,
-                                         mode ? cols_.p : nullptr, x, y);
-    ++launches_;
-}
-
 // dst = (N^-1 (src / D_r)) / D_c: `_ScaledProjectionPreconditioner` around
 // the block preconditioner (cmdgfm_projection.jl:158-179, 374-441)
-void CmdgfmDevice::precondition(DeviceSolver& ds, const CmdgfmFactor& f, const double* src, double* dst,
-                                int precision, cudaStream_t s) {
+void CmdgfmDevice::precondition(DeviceSolver& ds, const double* src, double* dst, int precision, cudaStream_t s) {
+    const Launch go{s, ds.pdl()};
     if (np_ > 0) {
-        TPA_CUDA(cudaMemsetAsync(full_.p, 0, sizeof(double) * size_t(ncells_), s));
-        // one component: the anchor's value folds in the scatter; several: one block each
-        k_cm_scatter<<<grid_of(np_), kT, 0, s>>>(np_, src, rows_.p, cell_.p, full_.p, ngroups_ == 1 ? anchor1_ : -1,
-                                                 partial_.p + 2 * kG, counter_.p);
+        // one component: the anchor's value folds in the scatter, and with it the
+        // cycle's right-hand-side sum; several: one block each, and a pass for the sum
+        const bool one = ngroups_ == 1;
+        go(k_cm_scatter, grid_of(np_), kT, 0, np_, src, rows_.p, cell_.p, full_.p, one ? anchor1_ : -1,
+           partial_.p + 2 * kG, counter_.p, ds.fused() ? ds.cycle_rhs_sum() : nullptr);
         ++launches_;
         if (ngroups_ > 1) {
-            k_cm_anchor<<<ngroups_, 1024, 0, s>>>(gptr_.p, gidx_.p, ganchor_.p, src, rows_.p, full_.p);
+            go(k_cm_anchor, ngroups_, 1024, 0, gptr_.p, gidx_.p, ganchor_.p, src, rows_.p, full_.p);
             ++launches_;
         }
         const int before = ds.kernel_launches();
-        ds.vcycle(full_.p, zfull_.p, precision);
-        launches_ += ds.kernel_launches() - before;
-        k_cm_gather<<<grid_of(np_), kT, 0, s>>>(np_, zfull_.p, cell_.p, anchor_.p, cols_.p, zp_.p, dst);
-        ++launches_;
+        if (ds.fused()) {
+            const DeviceSolver::CycleResult z = ds.vcycle_result(full_.p, precision, one);
+            if (precision)
+                go(k_cm_gather<float>, grid_of(np_), kT, 0, np_, z.xf, z.mean, cell_.p, anchor_.p, cols_.p, zp_.p, dst);
+            else
+                go(k_cm_gather<double>, grid_of(np_), kT, 0, np_, z.xd, z.mean, cell_.p, anchor_.p, cols_.p, zp_.p,
+                   dst);
+        } else {
+            ds.vcycle(full_.p, zfull_.p, precision);
+            go(k_cm_gather<double>, grid_of(np_), kT, 0, np_, zfull_.p, nullptr, cell_.p, anchor_.p, cols_.p, zp_.p,
+               dst);
+        }
+        launches_ += ds.kernel_launches() - before + 1;
     }
-    if (nx_ > 0) jump_apply(src, rows_.p, cols_.p, zp_.p, dst, s);
-    (void)f;
+    if (nx_ > 0) jump_apply(ds, src, rows_.p, cols_.p, zp_.p, dst, s);
 }
 
 // One BiCGSTAB iteration (Krylov.jl 0.10 `bicgstab!` with the right
@@ -621,45 +781,43 @@ void CmdgfmDevice::precondition(DeviceSolver& ds, const CmdgfmFactor& f, const d
 // z = N^-1 s, t = A z, omega; x += omega z, r = s - omega t; next rho, beta,
 // rNorm and the stopping rules (which set the loop condition when `set_cond`);
 // p = r + beta (p - omega v).
-void CmdgfmDevice::enqueue_iteration(DeviceSolver& ds, const CmdgfmFactor& f, bool preconditioned, int precision,
-                                     cudaStream_t s, cudaGraphConditionalHandle handle, int set_cond) {
+void CmdgfmDevice::enqueue_iteration(DeviceSolver& ds, bool preconditioned, int precision, cudaStream_t s,
+                                     cudaGraphConditionalHandle handle, int set_cond) {
+    const Launch go{s, ds.pdl()};
     const int g = grid_of(n_);
-    double* p1 = partial_.p;
-    double* p2 = partial_.p + kG;
+    double* const pt = partial_.p;
     double* st = state_.p;
+    // w = A u with the partials of c'w (and w'w)
+    auto product = [&](const double* u, double* w, const double* c, int ww) {
+        go(k_cm_product, g, kT, 0, n_, mptr_.p, mcol_.p, mval_.p, rows_.p, cols_.p, u, w, c, ww, pt, pt + kG);
+    };
     const double* y = p_.p;
     if (preconditioned) {
-        precondition(ds, f, p_.p, y_.p, precision, s);
+        precondition(ds, p_.p, y_.p, precision, s);
         y = y_.p;
     }
-    spmv(y, v_.p, 1, s);
-    k_cm_dot2<<<g, kT, 0, s>>>(n_, c_.p, v_.p, nullptr, nullptr, p1, nullptr);
-    k_cm_alpha<<<1, kT, 0, s>>>(p1, g, st);
-    k_cm_update1<<<g, kT, 0, s>>>(n_, r_.p, v_.p, y, s_.p, x_.p, st);
-    launches_ += 3;
+    product(y, v_.p, c_.p, 0);
+    go(k_cm_update1, g, kT, 0, n_, pt, g, r_.p, v_.p, y, s_.p, x_.p, st);
     const double* z = s_.p;
     if (preconditioned) {
-        precondition(ds, f, s_.p, z_.p, precision, s);
+        precondition(ds, s_.p, z_.p, precision, s);
         z = z_.p;
     }
-    spmv(z, t_.p, 1, s);
-    k_cm_dot2<<<g, kT, 0, s>>>(n_, t_.p, s_.p, t_.p, t_.p, p1, p2);
-    k_cm_omega<<<1, kT, 0, s>>>(p1, p2, g, st);
-    k_cm_update2<<<g, kT, 0, s>>>(n_, s_.p, t_.p, z, c_.p, x_.p, r_.p, st, p1, p2);
-    k_cm_rho<<<1, kT, 0, s>>>(p1, p2, g, st, handle, set_cond);
-    k_cm_pupdate<<<g, kT, 0, s>>>(n_, r_.p, v_.p, p_.p, st);
+    product(z, t_.p, s_.p, 1);
+    go(k_cm_update2, g, kT, 0, n_, pt, pt + kG, g, s_.p, t_.p, z, c_.p, x_.p, r_.p, st, pt + 2 * kG, pt + 3 * kG);
+    go(k_cm_pupdate, g, kT, 0, n_, pt + 2 * kG, pt + 3 * kG, g, r_.p, v_.p, p_.p, st, handle, set_cond);
     launches_ += 5;
 }
 
 // The iteration captured as the body of a graph WHILE node, kept while every
 // argument it captured is unchanged: the sizes, the jump-block layout, the
 // buffers and the pressure hierarchy's graph generation.
-cudaGraphExec_t CmdgfmDevice::loop_graph(DeviceSolver& ds, const CmdgfmFactor& f, bool preconditioned, int precision,
-                                         cudaStream_t s) {
+cudaGraphExec_t CmdgfmDevice::loop_graph(DeviceSolver& ds, bool preconditioned, int precision, cudaStream_t s) {
     std::vector<uintptr_t> key = {
         uintptr_t(n_), uintptr_t(np_), uintptr_t(nx_), uintptr_t(ncells_), uintptr_t(ngroups_),
         uintptr_t(int64_t(anchor1_)), uintptr_t(precision), uintptr_t(inverse_), uintptr_t(jstaged_),
-        uintptr_t(jsmem_), uintptr_t(ds.graph_generation()), uintptr_t(s)};
+        uintptr_t(jsmem_), uintptr_t(inverse_ ? ismem_ : 0), uintptr_t(inverse_ ? linnz_ : 0),
+        uintptr_t(inverse_ ? uinnz_ : 0), uintptr_t(ds.graph_generation()), uintptr_t(s)};
     for (const void* q : {(const void*)mptr_.p, (const void*)mcol_.p, (const void*)mval_.p, (const void*)rows_.p,
                           (const void*)cols_.p, (const void*)cell_.p, (const void*)anchor_.p, (const void*)gptr_.p,
                           (const void*)gidx_.p, (const void*)ganchor_.p, (const void*)cptr_.p, (const void*)ccol_.p,
@@ -698,7 +856,7 @@ cudaGraphExec_t CmdgfmDevice::loop_graph(DeviceSolver& ds, const CmdgfmFactor& f
     cudaGraph_t body = cp.conditional.phGraph_out[0];
     const int before = launches_, ds_before = ds.kernel_launches();
     TPA_CUDA(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    enqueue_iteration(ds, f, preconditioned, precision, s, handle, 1);
+    enqueue_iteration(ds, preconditioned, precision, s, handle, 1);
     cudaGraph_t captured;
     const cudaError_t ce = cudaStreamEndCapture(s, &captured);
     body_launches_[slot] = (launches_ - before);
@@ -719,15 +877,15 @@ cudaGraphExec_t CmdgfmDevice::loop_graph(DeviceSolver& ds, const CmdgfmFactor& f
 
 // dst_xi = (L U)^-1 (src_xi / rows_xi - C zp) / cols_xi: the jump block of the
 // block preconditioner (rows, cols: D_r, D_c) or of the warm start (ones)
-void CmdgfmDevice::jump_apply(const double* src, const double* rows, const double* cols, const double* zp,
-                              double* dst, cudaStream_t s) {
+void CmdgfmDevice::jump_apply(DeviceSolver& ds, const double* src, const double* rows, const double* cols,
+                              const double* zp, double* dst, cudaStream_t s) {
+    const Launch go{s, ds.pdl()};
     if (inverse_)
-        k_cm_jump_inverse<<<1, kIluThreads, 2 * size_t(nx_) * sizeof(double), s>>>(
-            int(nx_), np_, src, rows, cptr_.p, ccol_.p, cval_.p, zp, liptr_.p, licol_.p, lival_.p, uiptr_.p, uicol_.p,
-            uival_.p, cols, dst);
+        go(k_cm_jump_inverse, 1, kIluThreads, ismem_, int(nx_), np_, ishift_, istaged_, linnz_, uinnz_, src, rows,
+           cptr_.p, ccol_.p, cval_.p, zp, liptr_.p, licol_.p, lival_.p, uiptr_.p, uicol_.p, uival_.p, cols, dst);
     else
-        k_cm_jump_solve<<<1, kIluThreads, jsmem_, s>>>(int(nx_), np_, src, rows, cptr_.p, ccol_.p, cval_.p, zp,
-                                                       lview_, uview_, jstaged_, cols, dst);
+        go(k_cm_jump_solve, 1, kIluThreads, jsmem_, int(nx_), np_, src, rows, cptr_.p, ccol_.p, cval_.p, zp, lview_,
+           uview_, jstaged_, cols, dst);
     ++launches_;
 }
 
@@ -749,13 +907,13 @@ int CmdgfmDevice::bicgstab(DeviceSolver& ds, const CmdgfmInput& in, const Cmdgfm
     if (int(hs[kFlags]) & (kZeroRhs | kZeroRho | kSolved | kTired)) return 0;
     if (s && !std::getenv("TPAGMG_NO_GRAPH")) {
         // the whole run as one graph launch; the host reads the state at its end
-        cudaGraphExec_t exec = loop_graph(ds, f, preconditioned, in.precision, s);
+        cudaGraphExec_t exec = loop_graph(ds, preconditioned, in.precision, s);
         TPA_CUDA(cudaGraphLaunch(exec, s));
         read();
         launches_ += int(hs[kIter]) * body_launches_[preconditioned ? 1 : 0];
     } else {
         for (;;) {
-            enqueue_iteration(ds, f, preconditioned, in.precision, s, cudaGraphConditionalHandle(), 0);
+            enqueue_iteration(ds, preconditioned, in.precision, s, cudaGraphConditionalHandle(), 0);
             read();
             if (int(hs[kFlags]) & (kSolved | kTired | kBreakdown)) break;
         }
@@ -891,12 +1049,22 @@ void CmdgfmDevice::solve(DeviceSolver& ds, const CmdgfmInput& in, const CmdgfmFa
             uiptr_.upload(f.uinv.ptr.data(), f.uinv.ptr.size(), s);
             uicol_.upload(f.uinv.col.data(), f.uinv.col.size(), s);
             uival_.upload(f.uinv.val.data(), f.uinv.val.size(), s);
+            linnz_ = int(f.linv.col.size());
+            uinnz_ = int(f.uinv.col.size());
+            const size_t vectors = 2 * size_t(nx_) * sizeof(double);
+            const size_t entries = (size_t(linnz_) + size_t(uinnz_)) * (sizeof(double) + sizeof(int32_t));
+            istaged_ = vectors + entries <= size_t(200) * 1024 ? 1 : 0;
+            ismem_ = vectors + (istaged_ ? entries : 0);
+            for (ishift_ = 3; ishift_ > 0 && (nx_ << ishift_) > kIluThreads;) --ishift_;
             TPA_CUDA(cudaFuncSetAttribute(k_cm_jump_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          int(2 * size_t(nx_) * sizeof(double))));
+                                          int(ismem_)));
         }
     }
     for (auto* b : {&sol_, &corr_, &x_, &r_, &c_, &p_, &v_, &s_, &t_, &y_, &z_}) b->alloc(size_t(std::max<int64_t>(n_, 1)));
+    // cells that are no unknown and no anchor stay zero: the scatter writes the
+    // same cells in every iteration
     full_.alloc(size_t(std::max<int64_t>(ncells_, 1)));
+    TPA_CUDA(cudaMemsetAsync(full_.p, 0, sizeof(double) * size_t(std::max<int64_t>(ncells_, 1)), s));
     zfull_.alloc(size_t(std::max<int64_t>(ncells_, 1)));
     zp_.alloc(size_t(std::max<int64_t>(np_, 1)));
     jr_.alloc(size_t(std::max<int64_t>(nx_, 1)));
@@ -968,7 +1136,7 @@ void CmdgfmDevice::solve(DeviceSolver& ds, const CmdgfmInput& in, const CmdgfmFa
                 TPA_CUDA(cudaMemcpyAsync(y_.p, in.initial.data(), sizeof(double) * size_t(np_),
                                          cudaMemcpyHostToDevice, s));
             }
-            if (nx_ > 0) jump_apply(rhs_.p, ones_.p, ones_.p, y_.p, y_.p, s);
+            if (nx_ > 0) jump_apply(ds, rhs_.p, ones_.p, ones_.p, y_.p, y_.p, s);
             if (count([&] { k_cm_nonfinite<<<g, kT, 0, s>>>(n_, y_.p, p1); }) != 0.0) continue;
             k_cm_residual<<<g, kT, 0, s>>>(n_, mptr_.p, mcol_.p, mval_.p, rhs_.p, y_.p, t_.p);
             ++launches_;
@@ -1023,7 +1191,7 @@ void CmdgfmDevice::solve(DeviceSolver& ds, const CmdgfmInput& in, const CmdgfmFa
     st.pressure_defect = hs[kPressureDefect];
     st.jump_defect = hs[kJumpDefect];
     st.anchor_defect = na_ > 0 ? hs[kAnchorDefect] : 0.0;
-    st.final_residual = std::sqrt(count([&] { k_cm_dot2<<<g, kT, 0, s>>>(n_, corr_.p, corr_.p, nullptr, nullptr, p1, nullptr); }));
+    st.final_residual = std::sqrt(count([&] { k_cm_norm2<<<g, kT, 0, s>>>(n_, corr_.p, p1); }));
     const double worst = std::max(st.pressure_defect, std::max(st.jump_defect, st.anchor_defect));
     st.converged = std::isfinite(worst) && worst <= tol;
     st.iterations = iterations;

@@ -90,16 +90,13 @@ private:
     // one BiCGSTAB run on b (device): returns iterations; x holds the result
     int bicgstab(DeviceSolver& ds, const CmdgfmInput& in, const CmdgfmFactor& f, bool preconditioned, double rtol,
                  int itmax, cudaStream_t s);
-    void precondition(DeviceSolver& ds, const CmdgfmFactor& f, const double* src, double* dst, int precision,
-                      cudaStream_t s);
-    void spmv(const double* x, double* y, int mode, cudaStream_t s);
-    void jump_apply(const double* src, const double* rows, const double* cols, const double* zp, double* dst,
+    void precondition(DeviceSolver& ds, const double* src, double* dst, int precision, cudaStream_t s);
+    void jump_apply(DeviceSolver& ds, const double* src, const double* rows, const double* cols, const double* zp, double* dst,
                     cudaStream_t s);
     DevBuf<double> ones_;
-    void enqueue_iteration(DeviceSolver& ds, const CmdgfmFactor& f, bool preconditioned, int precision,
-                           cudaStream_t s, cudaGraphConditionalHandle handle, int set_cond);
-    cudaGraphExec_t loop_graph(DeviceSolver& ds, const CmdgfmFactor& f, bool preconditioned, int precision,
-                               cudaStream_t s);
+    void enqueue_iteration(DeviceSolver& ds, bool preconditioned, int precision, cudaStream_t s,
+                           cudaGraphConditionalHandle handle, int set_cond);
+    cudaGraphExec_t loop_graph(DeviceSolver& ds, bool preconditioned, int precision, cudaStream_t s);
     // captured BiCGSTAB loops (without / with the preconditioner) and what they captured
     cudaGraphExec_t exec_[2] = {nullptr, nullptr};
     std::vector<uintptr_t> key_[2];
@@ -122,6 +119,8 @@ private:
     TriView lview_{}, uview_{};
     // the factors' inverses by rows (used when `inverse_`)
     bool inverse_ = false;
+    int linnz_ = 0, uinnz_ = 0, istaged_ = 0, ishift_ = 0;  // entries, in shared memory or not, lanes per row (log2)
+    size_t ismem_ = 0;
     DevBuf<int64_t> liptr_, uiptr_;
     DevBuf<int32_t> licol_, uicol_;
     DevBuf<double> lival_, uival_;

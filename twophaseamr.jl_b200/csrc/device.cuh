@@ -160,6 +160,18 @@ public:
     void apply(const double* x, double* y);
     // z = V-cycle(r), device pointers; precision 0 = FP64, 1 = FP32 cycle.
     void vcycle(const double* r, double* z, int precision);
+    // The same cycle with its result left where the cycle put it: z = x - mean
+    // in FP64, x in the cycle's precision (xf or xd).  `summed`: the sum of r
+    // stands in cycle_rhs_sum() already.  Only with fused(); valid until the
+    // next cycle.
+    struct CycleResult {
+        const float* xf;
+        const double* xd;
+        const double* mean;
+    };
+    CycleResult vcycle_result(const double* r, int precision, bool summed);
+    double* cycle_rhs_sum() { return lsum_.p; }
+    bool pdl() const { return pdl_; }
     // `solve!`: rhs (strong form) and x (initial guess in, solution out) are
     // device pointers in cell order.
     void solve(const double* rhs, double* x, double rtol, double atol, int max_cycles, int compatibility,

@@ -1010,19 +1010,27 @@ void DeviceSolver::enqueue_vcycle_epi(const R* r, const double* rsum, double* me
 template void DeviceSolver::enqueue_vcycle<double>(const double*, const double*, double*);
 template void DeviceSolver::enqueue_vcycle<float>(const double*, const double*, double*);
 
-void DeviceSolver::vcycle_fused(const double* r, double* z, int precision) {
+DeviceSolver::CycleResult DeviceSolver::vcycle_result(const double* r, int precision, bool summed) {
     const Launch go{stream_, pdl_};
     const int n = levels_[0].n;
     const int nl = int(levels_.size());
     double* rsum = lsum_.p;  // slot 0: level-0 RHS sum
     double* mean = lsum_.p + nl;
-    go(k_sum_into, fold_grid(k_sum_into, kThreads, blocks_for(n), kMaxGrid), kThreads, 0, n, r, fpartial_.p,
-       counters_.p + kRsum, rsum);
-    ++launches_;
+    if (!summed) {
+        go(k_sum_into, fold_grid(k_sum_into, kThreads, blocks_for(n), kMaxGrid), kThreads, 0, n, r, fpartial_.p,
+           counters_.p + kRsum, rsum);
+        ++launches_;
+    }
     if (precision == 0) enqueue_vcycle<double>(r, rsum, mean);
     else enqueue_vcycle<float>(r, rsum, mean);
-    go(k_z_out, blocks_for(n), kThreads, 0, n, precision ? vf_[0].x : nullptr,
-                                                      precision ? nullptr : vd_[0].x, mean, z);
+    return {precision ? vf_[0].x : nullptr, precision ? nullptr : vd_[0].x, mean};
+}
+
+void DeviceSolver::vcycle_fused(const double* r, double* z, int precision) {
+    const Launch go{stream_, pdl_};
+    const int n = levels_[0].n;
+    const CycleResult c = vcycle_result(r, precision, false);
+    go(k_z_out, blocks_for(n), kThreads, 0, n, c.xf, c.xd, c.mean, z);
     ++launches_;
     TPA_CUDA(cudaGetLastError());
 }
