@@ -273,13 +273,16 @@ __global__ void kr_coarse_spd(int n, const int* __restrict__ rp, const int* __re
 
 // One block step: with D the diagonal block kb of `in`, C its block column and
 // R its block row,  out = D^-1 at (kb, kb), D^-1 R in row kb, -C D^-1 in column
-// kb, in - C D^-1 R elsewhere.  One CTA per tile of `out`; each inverts D in
-// shared memory (rows beyond n: the identity).  On the last step the tiles are
+// kb, in - C D^-1 R elsewhere.  One CTA per tile of `out`; each inverts D
+// (rows beyond n: the identity), which is what a step waits for: 32 dependent
+// pivots (at 256 cells 18.0 us a step with D in shared memory and two barriers a
+// pivot, 12.5 us with one).  On the last step the tiles are
 // stored as G, less the components' shift.
 __global__ void __launch_bounds__(256) kr_gj_step(int n, int kb, const double* __restrict__ in,
                                                   double* __restrict__ out, int last, const int* __restrict__ slot,
                                                   int ncomp, const double* __restrict__ shift, int* err) {
     __shared__ double D[kGj][kGj + 1], C[kGj][kGj + 1], R[kGj][kGj + 1];
+    __shared__ double prow[2][kGj], pcol[2][kGj], pinv[2];
     const int ti = blockIdx.y, tj = blockIdx.x;
     const int r = threadIdx.x >> 3, q = threadIdx.x & 7;  // this thread's row and columns q, q + 8, q + 16, q + 24
     auto load = [&](int bi, int bj, int u) {
@@ -288,28 +291,44 @@ __global__ void __launch_bounds__(256) kr_gj_step(int n, int kb, const double* _
     };
     double own[4];
     for (int u = 0; u < 4; ++u) {
-        D[r][q + 8 * u] = load(kb, kb, u);
         C[r][q + 8 * u] = load(ti, kb, u);
         R[r][q + 8 * u] = load(kb, tj, u);
         own[u] = load(ti, tj, u);
     }
-    // D^-1 in place, pivot by pivot: row p scaled by 1 / d_pp, the rest updated
-    // with the old column p, which becomes -d_ip / d_pp
+    // D^-1 pivot by pivot: row p scaled by 1 / d_pp, the rest updated with the
+    // old column p, which becomes -d_ip / d_pp.  D lies in the threads' registers;
+    // the threads that hold row and column p + 1 publish them, with the pivot's
+    // reciprocal, as soon as they are updated, in the other of two buffers: one
+    // barrier a pivot.
+    double d[4];
+    for (int u = 0; u < 4; ++u) d[u] = load(kb, kb, u);
+    auto publish = [&](int p) {
+        const int s = p & 1;
+        if (r == p)
+            for (int u = 0; u < 4; ++u) prow[s][q + 8 * u] = d[u];
+        if (q == (p & 7)) {
+            pcol[s][r] = d[p >> 3];
+            if (r == p) pinv[s] = 1.0 / d[p >> 3];
+        }
+    };
+    publish(0);
     bool bad = false;
+#pragma unroll
     for (int p = 0; p < kGj; ++p) {
+        const int s = p & 1;
         __syncthreads();
-        const double piv = D[p][p], f = D[r][p];
-        double row[4];
-        for (int u = 0; u < 4; ++u) row[u] = D[p][q + 8 * u];
-        bad = bad || !(piv > 0.0);
-        const double inv = 1.0 / piv;
-        __syncthreads();
+        const double inv = pinv[s], f = pcol[s][r];
+        bad = bad || !(pcol[s][p] > 0.0);
+#pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int j = q + 8 * u;
-            if (r == p) D[r][j] = j == p ? inv : row[u] * inv;
-            else D[r][j] = j == p ? -f * inv : D[r][j] - f * inv * row[u];
+            const double row = prow[s][j];
+            if (r == p) d[u] = j == p ? inv : row * inv;
+            else d[u] = j == p ? -f * inv : d[u] - f * inv * row;
         }
+        if (p + 1 < kGj) publish(p + 1);
     }
+    for (int u = 0; u < 4; ++u) D[r][q + 8 * u] = d[u];
     __syncthreads();
     if (bad && threadIdx.x == 0 && ti == kb && tj == kb) atomicCAS(err, 0, 3);
     double o[4];

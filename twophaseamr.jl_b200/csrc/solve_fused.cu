@@ -744,9 +744,12 @@ void DeviceSolver::build_dense_tail() {
         dense_n_ = n;
         dense_ld_ = ld;
     };
-    build(k_dense_tail_build<4>, 4);
-    build(k_dense_tail_build<2>, 2);
-    build(k_dense_tail_build<1>, 1);
+    // the most columns that still leave a CTA for every SM: 8 above 4 x 148 cells
+    if (n > 592 && n <= 2 * kDenseBuildThreads) build(k_dense_tail_build<8, 2>, 8);
+    if (n <= 2 * kDenseBuildThreads) build(k_dense_tail_build<4, 2>, 4);
+    build(k_dense_tail_build<4, 4>, 4);
+    build(k_dense_tail_build<2, 4>, 2);
+    build(k_dense_tail_build<1, 4>, 1);
 }
 
 void DeviceSolver::destroy_graphs() {
