@@ -70,13 +70,16 @@ inline int blocks_for(int64_t n) {
     return int(g < 1 ? 1 : g);
 }
 
-constexpr int kMaxGrid = 1184;
+constexpr int kMaxGrid = 1184;  // 8 CTAs on each of 148 SMs: bounds the partials every fold reads
 // tiles = 3: the largest constant-coefficient level on stencil tiles.  A level
 // of 2^19 cells is 2048 tiles, under two resident waves of 256-thread CTAs;
 // the next level up streams HBM at a rate the tiles' index arithmetic cannot
 // keep.
-constexpr int kRzCells = 1 << 20;  // rz_foldable
-constexpr int kStencilTileCells = 1 << 19;  // 8 CTAs on each of 148 SMs: bounds the partials every fold reads
+constexpr int kStencilTileCells = 1 << 19;
+// rz_foldable: the largest streamed or stencil-tiled finest level whose r'z rides
+// on the up kernel.  1024 x 512 with mixed_ir: 748 us a solve with the pass of its
+// own, 707 us folded; 2048^2: the up kernel 21 -> 34 us, the pass 12.8 us.
+constexpr int kRzCells = 1 << 20;
 #define TPA_GRID_STRIDE(i, n) for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += gridDim.x * blockDim.x)
 
 // r = b - A x, folds sum(r) into s->rsum
@@ -1109,7 +1112,7 @@ void DeviceSolver::enqueue_cg_body(int precision, cudaGraphConditionalHandle han
 // constant-coefficient level.  Above kRzCells a streamed level's extra r loads
 // cost what the separate pass takes (2048^2: the up kernel 21 -> 34 us, plain or
 // staged by cp.async, the pass 12.8 us); below, the pass is a launch's latency
-// (periodic 128^2 FP64: see kRzCells).  The vectorized and structured
+// (figures at kRzCells).  The vectorized and structured
 // post-smoothings (v_sweep, s_post2) have capped grids that stride over the
 // level and lost by it (2048^2: 3.35 -> 3.38 ms).
 bool DeviceSolver::rz_foldable() const {

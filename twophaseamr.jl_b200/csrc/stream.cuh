@@ -23,7 +23,7 @@
 // neighbour order west, east, south, north, v_pre2, v_residual, v_restrict,
 // v_prolong, v_sweep), which follow the default V-cycle of
 // src/solvers/multigrid/cycles.jl:46-77 (ronaldremmerswaal/TwoPhaseAMR.jl).
-// Only the order of the coarse right-hand-side and mean sums differs.
+// Only the order of the mean's sum differs.
 #pragma once
 
 #include <cuda_runtime.h>

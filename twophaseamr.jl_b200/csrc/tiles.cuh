@@ -10,7 +10,7 @@
 //                rings <= 2: x2 = x1 + w D^-1 (bp - A x1);
 //                rings <= 1: r = bp - A x2, s = Dt^-1 r;
 //                the block:  b_c = P_tent'(r - wt A s) for its coarse cells,
-//                            x2 and bp stored (x2 into L.y), the coarse RHS sum
+//                            x2 and bp stored (x2 into L.y)
 //   k_tile_up    rings <= 3: e = x_c(owner);
 //                rings <= 2: x = x2 + e - wt Dt^-1 A e;
 //                rings <= 1: x' = x + w D^-1 (bp - A x);
@@ -18,7 +18,7 @@
 //                            finest level's mean (and epilogue)
 // Every row is summed in CSR order with the arithmetic of the unfused kernels
 // (pre2_cell, residual_cell, restrict_quad, prolong_cell, sweep_cell), so the
-// two paths give the same V-cycle up to the order of the coarse RHS sum.
+// two paths give the same V-cycle up to rounding.
 //
 // A thread owns one row of the tile (two on tiles of more than 1024 rows): it
 // holds the row's entries, right-hand side, diagonals and iterate in registers
