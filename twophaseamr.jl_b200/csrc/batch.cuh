@@ -247,11 +247,15 @@ __device__ __forceinline__ BItem batch_item(const BItem* items) {
     return BItem{q.x, q.y, q.z, q.w};
 }
 
-// A row of an item: its first 8 entries in registers, loaded before the wait;
-// `col` is ci or cc.
+// A row of an item: its first kPre entries in registers, loaded before the wait;
+// `col` is ci or cc.  Six entries hold a row away from refinement jumps and its
+// right-hand side in 32 registers (FP32; 40 in FP64), every thread of an SM;
+// eight take 40 and 48 and cost more in resident warps than they save at the
+// jumps: 16 problems mixed 6.85 ms with eight, 6.54 with six; 256 problems 98 and
+// 88 ms, FP64 126 and 111.
 template <typename T>
 struct BRow {
-    static constexpr int kPre = 8;
+    static constexpr int kPre = 6;
     T a[kPre];
     int c[kPre];
     int w;
