@@ -201,11 +201,15 @@ def refresh_device(solver, kappa):
     """`_refresh_geometric_multigrid!` from device face coefficients."""
     torch = _torch()
     _sync_stream(solver)
-    # the operator's host copy: into page-locked memory on the same stream, so
-    # that the refresh's own synchronization completes it
+    # the operator's host copy: into page-locked memory on torch's stream, beside
+    # the refresh.  The library may run on a stream of its own, so that copy is
+    # waited for by itself, whatever becomes of the refresh.
     host = torch.empty(kappa.shape, dtype=kappa.dtype, pin_memory=True)
     host.copy_(kappa.detach(), non_blocking=True)
-    solver.ctx.call("tpa_refresh_device", _ptr(kappa))
+    try:
+        solver.ctx.call("tpa_refresh_device", _ptr(kappa))
+    finally:
+        torch.cuda.current_stream(kappa.device).synchronize()
     solver.operator.face_coefficient = host.numpy()
 
 
