@@ -291,7 +291,8 @@ tpa_status tpa_get_tuning(tpa_context* ctx, tpa_tune_config* config);
  * on faces of hanging-vertex patches (TPA_ERR_INVALID_ARG otherwise). */
 tpa_status tpa_adjoint(tpa_context* ctx, const double* p, const double* pbar, double* rhs_bar, double* kappa_bar,
                        double rtol, double atol, int32_t max_cycles, int32_t precision, tpa_stats* stats);
-/* Same with device pointers (cell and face order, on the context's device). */
+/* Same with device pointers (cell and face order, on the context's device);
+ * returns after its results are complete. */
 tpa_status tpa_adjoint_device(tpa_context* ctx, const double* p, const double* pbar, double* rhs_bar,
                               double* kappa_bar, double rtol, double atol, int32_t max_cycles, int32_t precision,
                               tpa_stats* stats);

@@ -717,6 +717,7 @@ tpa_status tpa_adjoint_device(tpa_context* ctx, const double* p, const double* p
     return guard(ctx, [&] {
         if (!p || !pbar) throw tpa::Error(TPA_ERR_INVALID_ARG, "null solution or cotangent");
         adjoint_on_device(ctx, p, pbar, rhs_bar, kappa_bar, rtol, atol, max_cycles, precision, stats);
+        TPA_CUDA(cudaStreamSynchronize(ctx->dev->stream()));
     });
 }
 
