@@ -222,6 +222,7 @@ const char* tpa_batch_last_error(const tpa_batch* batch);
 tpa_status tpa_batch_sizes(const tpa_batch* batch, int64_t out[4]);
 /* offsets[k] = first fine cell of problem k in the concatenated arrays (count + 1 entries). */
 tpa_status tpa_batch_offsets(const tpa_batch* batch, int64_t* offsets);
+/* As tpa_set_stream. */
 tpa_status tpa_batch_set_stream(tpa_batch* batch, void* stream);
 /* solve! of every problem: rhs and x are the problems' cell arrays concatenated
  * in problem order (tpa_batch_offsets), host memory.  stats and statuses
@@ -348,9 +349,11 @@ tpa_status tpa_tiled_levels(tpa_context* ctx, int32_t* count);
  * reference counterpart. */
 tpa_status tpa_streamed_levels(tpa_context* ctx, int32_t* count);
 /* Run subsequent device work on the caller's CUDA stream (a cudaStream_t
- * passed as void*; NULL restores the context's own stream).  Replaces nothing
- * in the reference (it has no device); it lets a caller order the solve with
- * its own device work and time it with events on that stream. */
+ * passed as void*; NULL restores the context's own stream, which does not
+ * synchronize with the legacy default stream: each call with NULL orders the
+ * device work that follows it behind what the default stream holds by then).
+ * Replaces nothing in the reference (it has no device); it lets a caller order
+ * the solve with its own device work and time it with events on that stream. */
 tpa_status tpa_set_stream(tpa_context* ctx, void* stream);
 /* Average device time in ms of `iters` back-to-back launches of one kernel on
  * level `level`: which = 0 smoothing sweep, 1 restriction, 4 first two

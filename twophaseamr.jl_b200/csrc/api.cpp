@@ -745,7 +745,7 @@ tpa_status tpa_adjoint(tpa_context* ctx, const double* p, const double* pbar, do
 
 tpa_status tpa_set_stream(tpa_context* ctx, void* stream) {
     return guard(ctx, [&] {
-        if (ctx->dev) TPA_CUDA(cudaStreamSynchronize(ctx->dev->stream()));
+        if (ctx->dev && stream != ctx->user_stream) TPA_CUDA(cudaStreamSynchronize(ctx->dev->stream()));
         ctx->user_stream = stream;
         if (ctx->dev) ctx->dev->set_stream(static_cast<cudaStream_t>(stream));
     });

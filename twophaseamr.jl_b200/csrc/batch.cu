@@ -293,6 +293,7 @@ BatchSolver::BatchSolver(int device, const std::vector<const Hierarchy*>& hs) : 
     TPA_CUDA(cudaSetDevice(device_));
     TPA_CUDA(cudaStreamCreateWithFlags(&own_stream_, cudaStreamNonBlocking));
     stream_ = own_stream_;
+    TPA_CUDA(cudaEventCreateWithFlags(&ev_order_, cudaEventDisableTiming));
     build(hs);
 }
 
@@ -303,6 +304,7 @@ BatchSolver::~BatchSolver() {
     if (host_state_) cudaFreeHost(host_state_);
     if (ev0_) cudaEventDestroy(ev0_);
     if (ev1_) cudaEventDestroy(ev1_);
+    if (ev_order_) cudaEventDestroy(ev_order_);
     if (own_stream_) cudaStreamDestroy(own_stream_);
 }
 

@@ -28,7 +28,12 @@ public:
     int tail_levels() const { return 1; }  // the dense coarsest level
     int64_t level_rows(int j) const { return lev_[size_t(j)].n; }
     cudaStream_t stream() const { return stream_; }
-    void set_stream(cudaStream_t s) { stream_ = s ? s : own_stream_; }
+    // as DeviceSolver::set_stream
+    void set_stream(cudaStream_t s) {
+        TPA_CUDA(cudaSetDevice(device_));
+        stream_ = s ? s : own_stream_;
+        if (!s) follow_default_stream(own_stream_, ev_order_);
+    }
     int kernel_launches() const { return launches_; }
     void reset_launches() { launches_ = 0; }
     float last_ms() const { return last_ms_; }
@@ -102,7 +107,7 @@ private:
     DevArray<BState> state_;
     DevArray<SolveState> sstate_;
     SolveState* host_state_ = nullptr;  // pinned
-    cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
+    cudaEvent_t ev0_ = nullptr, ev1_ = nullptr, ev_order_ = nullptr;
     DevArray<int> active_, again_;
     cudaGraphExec_t exec_[2] = {nullptr, nullptr};
     int body_launches_[2] = {0, 0};

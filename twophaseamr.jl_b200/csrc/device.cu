@@ -426,6 +426,16 @@ __global__ void k_cg_init(const double* __restrict__ partial, int np, CgScalars*
 
 // ---------------------------------------------------------------------------------
 
+void follow_default_stream(cudaStream_t own, cudaEvent_t event) {
+    cudaStreamCaptureStatus status;
+    if (cudaStreamIsCapturing(cudaStreamLegacy, &status) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    TPA_CUDA(cudaEventRecord(event, cudaStreamLegacy));
+    TPA_CUDA(cudaStreamWaitEvent(own, event, 0));
+}
+
 DeviceSolver::DeviceSolver(int device) : device_(device) {
     TPA_CUDA(cudaSetDevice(device));
     TPA_CUDA(cudaStreamCreateWithFlags(&own_stream_, cudaStreamNonBlocking));
@@ -435,6 +445,7 @@ DeviceSolver::DeviceSolver(int device) : device_(device) {
     TPA_CUDA(cudaMallocHost(&host_solve_, sizeof(SolveState)));
     TPA_CUDA(cudaEventCreate(&ev0_));
     TPA_CUDA(cudaEventCreate(&ev1_));
+    TPA_CUDA(cudaEventCreateWithFlags(&ev_order_, cudaEventDisableTiming));
     partial_.alloc(static_cast<size_t>(4 * kReduceBlocks));
     sc_.alloc(1);
     sums_.alloc(64);
@@ -450,6 +461,7 @@ DeviceSolver::~DeviceSolver() {
     if (host_solve_) cudaFreeHost(host_solve_);
     if (ev0_) cudaEventDestroy(ev0_);
     if (ev1_) cudaEventDestroy(ev1_);
+    if (ev_order_) cudaEventDestroy(ev_order_);
     if (rstage_) cudaFreeHost(rstage_);
     if (own_stream_) cudaStreamDestroy(own_stream_);
 }

@@ -142,6 +142,12 @@ double red_black_weight(const Csr& A, const std::vector<unsigned char>& colours)
 
 struct SolveState;
 
+// Work enqueued on `own` from here on waits for what the legacy default stream
+// (torch's default stream) holds by now.  `own` is a non-blocking stream, which
+// is not ordered with it by itself.  Left out while a blocking stream is being
+// captured, which forbids any use of the default stream.
+void follow_default_stream(cudaStream_t own, cudaEvent_t event);
+
 class DeviceSolver {
 public:
     explicit DeviceSolver(int device);
@@ -150,8 +156,13 @@ public:
     int ncells() const { return levels_.empty() ? 0 : levels_[0].n; }
     int nlevels() const { return int(levels_.size()); }
     cudaStream_t stream() const { return stream_; }
-    // Run on a caller-owned stream (nullptr: the solver's own stream).
-    void set_stream(cudaStream_t s) { stream_ = s ? s : own_stream_; }
+    // Run on a caller-owned stream (nullptr: the solver's own stream, behind the
+    // work that the legacy default stream holds by now).
+    void set_stream(cudaStream_t s) {
+        TPA_CUDA(cudaSetDevice(device_));
+        stream_ = s ? s : own_stream_;
+        if (!s) follow_default_stream(own_stream_, ev_order_);
+    }
     // Average time (ms) of `iters` launches of one kernel family on level `level`:
     // 0 = smoothing sweep, 1 = residual+restriction, 2 = prolongation, 3 = CG operator.
     double time_kernel(int which, int level, int precision, int iters);
@@ -264,6 +275,7 @@ private:
     DevArray<char> sstate_;          // SolveState (cg_state.cuh)
     SolveState* host_solve_ = nullptr;  // its pinned host copy
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;  // around a solve (its device time)
+    cudaEvent_t ev_order_ = nullptr;             // the default stream's work before a call
     double vol_total_ = 0;  // finest-level volume of cells with V > 0
 
     bool fused_ok_ = false;

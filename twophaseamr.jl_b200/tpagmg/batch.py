@@ -67,6 +67,7 @@ class BatchedSolver:
         return out
 
     def set_stream(self, stream):
+        """As `EllipticSolver.set_stream`."""
         self._call("tpa_batch_set_stream", C.c_void_p(int(stream) or None))
 
     def _stats(self, raw):

@@ -276,7 +276,9 @@ class EllipticSolver:
         return g
 
     def set_stream(self, stream):
-        """Order device work after the given CUDA stream handle (int; 0 = own)."""
+        """Run device work on the given CUDA stream handle (int).  0, torch's
+        default stream: the solver's own stream, behind what the default stream
+        holds at this call."""
         self.ctx.call("tpa_set_stream", C.c_void_p(int(stream) or None))
 
     def solve_device(self, rhs_ptr, x_ptr, *, rtol=1e-10, atol=0.0, max_cycles=100, compatibility="project",
