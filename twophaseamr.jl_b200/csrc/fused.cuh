@@ -42,8 +42,12 @@ constexpr int kTailThreads = 1024;
 // First statement of every cycle kernel (programmatic dependent launch, sm_90
 // and later): allow the next kernel of the stream to be scheduled now, then wait
 // until the kernels this one depends on have completed and their writes are
-// visible.  Nothing is read or written before the wait.  For a launch without
-// the programmatic attribute both instructions return at once.
+// visible.  Nothing is read or written before the wait, which takes plain
+// pointers: a __restrict__ parameter, const or not, tells the compiler that
+// nothing else touches its memory, the wait's memory clobber included, and its
+// loads may then move above the wait.  Only what no kernel of a solve writes may
+// carry the qualifier.  For a launch without the programmatic attribute both
+// instructions return at once.
 __device__ __forceinline__ void pdl_entry() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -53,11 +57,9 @@ __device__ __forceinline__ void pdl_entry() {
 // the cycle writes: the lists and operator values of its level, which only
 // set-up and refresh write, and the host waits for those before it launches a
 // cycle.  Such loads may run while the kernels before this one drain; anything a
-// kernel of the cycle writes is read after pdl_wait.  Two rules keep the halves
-// apart.  What is read after the wait comes through plain pointers: a const
-// __restrict__ parameter marks its loads as invariant, and the compiler then
-// moves them across the wait.  What is read before it comes through ld_static,
-// past the L1, whose lines may be older than the kernel's predecessor.
+// kernel of the cycle writes is read after pdl_wait, through plain pointers as in
+// pdl_entry.  What is read before it comes through ld_static, past the L1, whose
+// lines may be older than the kernel's predecessor.
 __device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <typename V>
@@ -402,7 +404,7 @@ __device__ __forceinline__ void rb_pair_cell(const LevelView<T>& L, const T* in,
 // `level_sum` (may be null): the RHS sum of this level, folded by the kernel
 // that produced b; mean = sum * cvol_inv.
 template <typename T, typename TB>
-__global__ void k_pre2(LevelView<T> L, const TB* __restrict__ b, const double* level_sum) {
+__global__ void k_pre2(LevelView<T> L, const TB* b, const double* level_sum) {
     pdl_entry();
     L = with_weights(L);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -413,7 +415,7 @@ __global__ void k_pre2(LevelView<T> L, const TB* __restrict__ b, const double* l
 // one red-black half-sweep (colour c) from in into out; with `mean_out`, also
 // the volume-weighted mean of out
 template <typename T>
-__global__ void k_rb_half(LevelView<T> L, const T* __restrict__ in, T* __restrict__ out, int c, double* partial,
+__global__ void k_rb_half(LevelView<T> L, const T* in, T* out, int c, double* partial,
                           unsigned* counter, double* mean_out) {
     pdl_entry();
     L = with_weights(L);
@@ -432,7 +434,7 @@ __global__ void k_rb_half(LevelView<T> L, const T* __restrict__ in, T* __restric
 
 // first red-black sweep from zero into out
 template <typename T, typename TB>
-__global__ void k_rb_pre(LevelView<T> L, const TB* __restrict__ b, const double* level_sum, T* out) {
+__global__ void k_rb_pre(LevelView<T> L, const TB* b, const double* level_sum, T* out) {
     pdl_entry();
     L = with_weights(L);
     int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -443,7 +445,7 @@ __global__ void k_rb_pre(LevelView<T> L, const TB* __restrict__ b, const double*
 // one red-black sweep (colour c, then the other) from in into out; with
 // `mean_out`, also the volume-weighted mean of out
 template <typename T>
-__global__ void k_rb_pair(LevelView<T> L, const T* __restrict__ in, T* __restrict__ out, int c, double* partial,
+__global__ void k_rb_pair(LevelView<T> L, const T* in, T* out, int c, double* partial,
                           unsigned* counter, double* mean_out) {
     pdl_entry();
     L = with_weights(L);
@@ -469,7 +471,7 @@ __global__ void k_residual(LevelView<T> L) {
 
 // b_c = P_tent'(r - wt A s), four threads per coarse cell (grid over 4 nc)
 template <typename T>
-__global__ void k_restrict(LevelView<T> L, T* __restrict__ bc) {
+__global__ void k_restrict(LevelView<T> L, T* bc) {
     pdl_entry();
     L = with_weights(L);
     // grid-stride over whole warps (the shuffles need every lane of a warp)
@@ -488,7 +490,7 @@ __global__ void k_restrict(LevelView<T> L, T* __restrict__ bc) {
 // cell, as k_restrict).  Saves the residual phase and the r / s round trip at
 // the price of about nnz_row^2 products per fine cell.
 template <typename T>
-__global__ void k_resrest(LevelView<T> L, T* __restrict__ bc) {
+__global__ void k_resrest(LevelView<T> L, T* bc) {
     pdl_entry();
     L = with_weights(L);
     const int quads = (4 * L.nc + 31) & ~31;
@@ -516,7 +518,7 @@ __global__ void k_resrest(LevelView<T> L, T* __restrict__ bc) {
 }
 
 template <typename T>
-__global__ void k_prolong(LevelView<T> L, const T* __restrict__ xc) {
+__global__ void k_prolong(LevelView<T> L, const T* xc) {
     pdl_entry();
     L = with_weights(L);
     int i = blockIdx.x * blockDim.x + threadIdx.x;

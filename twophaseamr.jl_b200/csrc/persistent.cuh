@@ -68,7 +68,7 @@ __device__ __forceinline__ void grid_barrier(unsigned* bar, int* err, unsigned l
 
 template <typename T>
 __global__ void __launch_bounds__(kTailThreads, 1)
-    k_vcycle_grid(const LevelView<T>* __restrict__ levels, int t, int nl, const double* __restrict__ r,
+    k_vcycle_grid(const LevelView<T>* __restrict__ levels, int t, int nl, const double* r,
                   const double* rsum, double* mean_out, const double* __restrict__ G, int gn, double* partial,
                   unsigned* bar, double* lsum, int* err, unsigned long long spins) {
     pdl_entry();

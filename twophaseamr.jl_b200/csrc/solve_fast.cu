@@ -45,7 +45,7 @@ __device__ __forceinline__ void publish_fold(const double (&v)[N], unsigned max_
 
 // sums of b = V f, |b| and V x0 over cells with V > 0; the means to remove.
 // vol null: every cell's volume is vol0.
-__global__ void k_prep(int n, const double* __restrict__ rhs, const double* __restrict__ xin,
+__global__ void k_prep(int n, const double* rhs, const double* xin,
                        const double* __restrict__ vol, double vol0, SolveAsk q, double* partial, unsigned* counter,
                        SolveState* S) {
     pdl_entry();
@@ -95,7 +95,7 @@ __global__ void k_pres(LevelView<double> A, PresIo io, int masked, SolveAsk q, d
     pdl_entry();
     const double m = First ? S->mx : S->xm, mb = First ? S->mb : 0.0;
     const bool store = First || S->ok;
-    const double* __restrict__ x0 = io.xin;
+    const double* x0 = io.xin;
     double v[5] = {0, 0, 0, 0, 0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < A.n; i += gridDim.x * blockDim.x) {
         const double V = A.vol[i];
@@ -210,7 +210,7 @@ __global__ void __launch_bounds__(256) v_pres(SView<double> L, PresIo io, int wi
 
 // the iterate's mean sum V x / cvol, taken off by the next residual pass (none
 // when no run was made).  vol null: every cell's volume is vol0.
-__global__ void k_xmean(int n, const double* __restrict__ x, const double* __restrict__ vol, double vol0, double cvol,
+__global__ void k_xmean(int n, const double* x, const double* __restrict__ vol, double vol0, double cvol,
                         double* partial, unsigned* counter, SolveState* S) {
     pdl_entry();
     double v[1] = {0};

@@ -83,8 +83,8 @@ constexpr int kRzCells = 1 << 20;
 #define TPA_GRID_STRIDE(i, n) for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += gridDim.x * blockDim.x)
 
 // r = b - A x, folds sum(r) into s->rsum
-__global__ void k_cg_residual(LevelView<double> A, const double* __restrict__ b, const double* __restrict__ x,
-                              double* __restrict__ r, double* partial, unsigned* counter, CgState* s) {
+__global__ void k_cg_residual(LevelView<double> A, const double* b, const double* x,
+                              double* r, double* partial, unsigned* counter, CgState* s) {
     pdl_entry();
     double v = 0;
     TPA_GRID_STRIDE(i, A.n) {
@@ -97,7 +97,7 @@ __global__ void k_cg_residual(LevelView<double> A, const double* __restrict__ b,
     });
 }
 
-__global__ void k_sum_into(int n, const double* __restrict__ v, double* partial, unsigned* counter, double* out) {
+__global__ void k_sum_into(int n, const double* v, double* partial, unsigned* counter, double* out) {
     pdl_entry();
     double acc = 0;
     TPA_GRID_STRIDE(i, n) acc += v[i];
@@ -136,7 +136,7 @@ __device__ __forceinline__ void cg_after_update(CgState* s, bool halted, cudaGra
 // Ap = A p and alpha = gamma / p'Ap with the zero-curvature guard: the CG
 // operator product alone, as time_fused times it (the CG loop runs the
 // *_cg_dir_ap kernels, which also form p)
-__global__ void k_cg_ap(LevelView<double> A, const double* __restrict__ p, double* __restrict__ ap, double* partial,
+__global__ void k_cg_ap(LevelView<double> A, const double* p, double* ap, double* partial,
                         unsigned* counter, CgState* s) {
     pdl_entry();
     double v = 0;
@@ -167,11 +167,11 @@ __device__ __forceinline__ P* dir_new(P* pa, P* pb, int iter) {
 // storage type of r, p and Ap (FP32 in the refinement solve's inner runs);
 // x and the arithmetic stay FP64, and the norms are those of the stored r.
 template <typename P>
-__global__ void k_cg_update(int n, double* __restrict__ x, P* __restrict__ r, P* pa, P* pb, const P* __restrict__ ap,
+__global__ void k_cg_update(int n, double* x, P* r, P* pa, P* pb, const P* ap,
                             const double* __restrict__ vol, double vol0, double* pmax, double* psum,
                             unsigned* counter, CgState* s, cudaGraphConditionalHandle handle, int set_cond) {
     pdl_entry();
-    const P* __restrict__ p = dir_new(pa, pb, s->iter);
+    const P* p = dir_new(pa, pb, s->iter);
     const bool skip = s->flags & kCgHalt;
     const double alpha = s->alpha;
     double m = 0, sum = 0;
@@ -215,7 +215,7 @@ __global__ void k_cg_update(int n, double* __restrict__ x, P* __restrict__ r, P*
 
 // block-structured finest level: Ap = A p and alpha
 template <int NXC>
-__global__ void s_cg_ap(SView<double> L, const double* __restrict__ p, double* __restrict__ ap, double* partial,
+__global__ void s_cg_ap(SView<double> L, const double* p, double* ap, double* partial,
                         unsigned* counter, CgState* s) {
     pdl_entry();
     s_apply_dot<double, NXC>(L, p, ap, partial, counter, [&](double pAp) { alpha_from(pAp, s); });
@@ -223,8 +223,8 @@ __global__ void s_cg_ap(SView<double> L, const double* __restrict__ p, double* _
 
 // block-structured finest level: r = b - A x, folds sum(r) into s->rsum
 template <int NXC>
-__global__ void s_cg_residual(SView<double> L, const double* __restrict__ b, const double* __restrict__ x,
-                              double* __restrict__ r, double* partial, unsigned* counter, CgState* s) {
+__global__ void s_cg_residual(SView<double> L, const double* b, const double* x,
+                              double* r, double* partial, unsigned* counter, CgState* s) {
     pdl_entry();
     double part = 0;
     for (int bk = blockIdx.x; bk < L.nblocks; bk += gridDim.x) {
@@ -240,16 +240,16 @@ __global__ void s_cg_residual(SView<double> L, const double* __restrict__ b, con
 }
 
 // constant-coefficient 16x16 finest level: Ap = A p and alpha (vectorized quads)
-__global__ void __launch_bounds__(256) v_cg_ap(SView<double> L, const double* __restrict__ p,
-                                               double* __restrict__ ap, double* partial, unsigned* counter,
+__global__ void __launch_bounds__(256) v_cg_ap(SView<double> L, const double* p,
+                                               double* ap, double* partial, unsigned* counter,
                                                CgState* s) {
     pdl_entry();
     v_apply_dot(L, p, ap, partial, counter, [&](double pAp) { alpha_from(pAp, s); });
 }
 
 // constant-coefficient 16x16 finest level: r = b - A x, folds sum(r) into s->rsum
-__global__ void __launch_bounds__(256) v_cg_residual(SView<double> L, const double* __restrict__ b,
-                                                     const double* __restrict__ x, double* __restrict__ r,
+__global__ void __launch_bounds__(256) v_cg_residual(SView<double> L, const double* b,
+                                                     const double* x, double* r,
                                                      double* partial, unsigned* counter, CgState* s) {
     pdl_entry();
     const int groups = (L.nblocks + 3) / 4;
@@ -286,7 +286,7 @@ __device__ void cg_after_z(CgState* s, double g);
 // next operator product forms z and p where it reads them), then beta or the
 // start of a run (cg_after_z)
 template <typename T, typename R>
-__global__ void k_cg_z(int n, const T* __restrict__ xv, const double* mean, const R* __restrict__ r,
+__global__ void k_cg_z(int n, const T* xv, const double* mean, const R* r,
                        double* partial, unsigned* counter, CgState* s) {
     pdl_entry();
     const double m = mean ? *mean : 0.0;
@@ -424,26 +424,26 @@ __global__ void k_cg_dir_ap(LevelView<double> A, const T* xv, const double* mean
 
 // the same on a block-structured finest level
 template <typename T, typename P, int NXC>
-__global__ void s_cg_dir_ap(SView<double> L, const T* __restrict__ xv, const double* mean, P* pa, P* pb,
-                            P* __restrict__ ap, double* partial, unsigned* counter, CgState* s) {
+__global__ void s_cg_dir_ap(SView<double> L, const T* xv, const double* mean, P* pa, P* pb,
+                            P* ap, double* partial, unsigned* counter, CgState* s) {
     pdl_entry();
     if (s->flags & kCgHalt) return;  // the run ended at this body's r'z
     const NextDir<T, P> d = next_dir(xv, mean, pa, pb, s);
-    P* __restrict__ pn = dir_new(pa, pb, s->iter);
+    P* pn = dir_new(pa, pb, s->iter);
     s_apply_dot_ld<double, NXC>(L, d, [&](int c, double v) { pn[c] = P(v); }, ap, partial, counter,
                                 [&](double pAp) { alpha_from(pAp, s); });
 }
 
 // the same on a constant-coefficient 16x16 finest level (vectorized quads)
 template <typename T, typename P>
-__global__ void __launch_bounds__(256) v_cg_dir_ap(SView<double> L, const T* __restrict__ xv, const double* mean,
-                                                   P* pa, P* pb, P* __restrict__ ap, double* partial,
+__global__ void __launch_bounds__(256) v_cg_dir_ap(SView<double> L, const T* xv, const double* mean,
+                                                   P* pa, P* pb, P* ap, double* partial,
                                                    unsigned* counter, CgState* s) {
     pdl_entry();
     if (s->flags & kCgHalt) return;  // the run ended at this body's r'z
     const int k = s->iter;
-    const P* __restrict__ po = dir_old(pa, pb, k);
-    P* __restrict__ pn = dir_new(pa, pb, k);
+    const P* po = dir_old(pa, pb, k);
+    P* pn = dir_new(pa, pb, k);
     const double mu = *mean, beta = s->beta;
     const bool first = k == 0;
     auto ld = [&](int c) {
@@ -471,8 +471,8 @@ constexpr int kStreamCgCtas = 6;  // resident CTAs per SM the kernel is built fo
 
 template <typename T, typename P, int ROWS>
 __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCgCtas)
-    v_stream_dir_ap(SView<double> L, StreamGeom g, const T* __restrict__ xv, const double* mean, P* pa, P* pb,
-                    P* __restrict__ ap, double* partial, unsigned* counter, CgState* s) {
+    v_stream_dir_ap(SView<double> L, StreamGeom g, const T* xv, const double* mean, P* pa, P* pb,
+                    P* ap, double* partial, unsigned* counter, CgState* s) {
     pdl_entry();
     if (s->flags & kCgHalt) return;  // the run ended at this body's r'z
     constexpr int S = ROWS + 2, D = kStreamDepth;
@@ -480,8 +480,8 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCgCtas)
     __shared__ P2<P> sp[kStreamWarps][D][32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int it = s->iter;
-    const P* __restrict__ po = dir_old(pa, pb, it);
-    P* __restrict__ pn = dir_new(pa, pb, it);
+    const P* po = dir_old(pa, pb, it);
+    P* pn = dir_new(pa, pb, it);
     const double mu = *mean, beta = s->beta;
     const bool first = it == 0;
     const int W = g.nbx * 16, H = g.nby * 16;
@@ -537,7 +537,7 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCgCtas)
 // Start of an inner run of the refinement solve: the FP64 true residual
 // rounded to the FP32 recurrence residual, and the sum of the stored values
 // (the V-cycle's right-hand-side projection uses it)
-__global__ void k_ir_start(int n, const double* __restrict__ r, float* __restrict__ r32, double* partial,
+__global__ void k_ir_start(int n, const double* r, float* r32, double* partial,
                            unsigned* counter, CgState* s) {
     pdl_entry();
     double v = 0;
@@ -565,8 +565,8 @@ __global__ void k_cg_set(CgState* s, double target, int itmax) {
     s->fresh = 1;
 }
 
-__global__ void k_z_out(int n, const float* __restrict__ xf, const double* __restrict__ xd, const double* mean,
-                        double* __restrict__ z) {
+__global__ void k_z_out(int n, const float* xf, const double* xd, const double* mean,
+                        double* z) {
     pdl_entry();
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;

@@ -116,7 +116,7 @@ __device__ __forceinline__ int s_owner(const SView<T>& L, int q) {
     const int c = (bk) * Blk<NXC>::cpb(L) + t;
 
 template <typename T, typename TB, int NXC>
-__global__ void s_pre2(SView<T> L, const TB* __restrict__ bin, const double* level_sum) {
+__global__ void s_pre2(SView<T> L, const TB* bin, const double* level_sum) {
     pdl_entry();
     const int b = blockIdx.x;
     TPA_S_CELL(b);
@@ -147,7 +147,7 @@ __global__ void s_residual(SView<T> L) {
 // t = r - wt A s per fine cell, aggregated over the 2x2 (or 1x1) children into
 // the coarse block quadrant.
 template <typename T, int NXC>
-__global__ void s_restrict(SView<T> L, T* __restrict__ bc) {
+__global__ void s_restrict(SView<T> L, T* bc) {
     pdl_entry();
     extern __shared__ unsigned char smem_raw[];
     T* tile = reinterpret_cast<T*>(smem_raw);
@@ -173,7 +173,7 @@ __global__ void s_restrict(SView<T> L, T* __restrict__ bc) {
 
 // x += e - wt Dt^-1 A e with e = x_c[owner(.)], in place
 template <typename T, int NXC>
-__global__ void s_prolong(SView<T> L, const T* __restrict__ xc) {
+__global__ void s_prolong(SView<T> L, const T* xc) {
     pdl_entry();
     const int b = blockIdx.x;
     TPA_S_CELL(b);

@@ -167,7 +167,7 @@ __device__ __forceinline__ Quad<T> q_dinv(const SView<T>& L, int c) {
 
 // both pre-sweeps from x = 0, with the level's RHS projection
 template <typename T, typename TB>
-__global__ void __launch_bounds__(256) v_pre2(SView<T> L, const TB* __restrict__ bin, const double* level_sum) {
+__global__ void __launch_bounds__(256) v_pre2(SView<T> L, const TB* bin, const double* level_sum) {
     pdl_entry();
     const double mean = (L.singular && level_sum) ? *level_sum * L.cvol_inv : 0.0;
     const int groups = (L.nblocks + 3) / 4;
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(256) v_residual(SView<T> L) {
 // b_c = P_tent'(r - wt A s): 2x2 (scale 2) or 1x1 (scale 1) aggregation into the
 // coarse block's quadrant
 template <typename T>
-__global__ void __launch_bounds__(256) v_restrict(SView<T> L, T* __restrict__ bc) {
+__global__ void __launch_bounds__(256) v_restrict(SView<T> L, T* bc) {
     pdl_entry();
     const int groups = (L.nblocks + 3) / 4;
     TPA_Q_LOOP(groups) {
@@ -304,7 +304,7 @@ __device__ __forceinline__ T q_coarse_cell(const SView<T>& L, const T* xc, int b
 
 // x += e - wt D^-1 A e, e = P_tent x_c
 template <typename T>
-__global__ void __launch_bounds__(256) v_prolong(SView<T> L, const T* __restrict__ xc) {
+__global__ void __launch_bounds__(256) v_prolong(SView<T> L, const T* xc) {
     pdl_entry();
     const int groups = (L.nblocks + 3) / 4;
     TPA_Q_LOOP(groups) {
@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(256) v_prolong(SView<T> L, const T* __restrict
 // out = in + w D^-1 (bp - A in); with `partial`, folds the volume-weighted sum of
 // out into mean_out (times cvol_inv)
 template <typename T, bool Fold, typename Epi = MeanOnly>
-__global__ void __launch_bounds__(256) v_sweep(SView<T> L, const T* __restrict__ in, T* __restrict__ out,
+__global__ void __launch_bounds__(256) v_sweep(SView<T> L, const T* in, T* out,
                                                double* partial, unsigned* counter, double* mean_out,
                                                Epi epi = Epi()) {
     pdl_entry();

@@ -109,8 +109,8 @@ __device__ __forceinline__ P2<T> st_apply(const SView<T>& L, const P2<T>& s, con
 // cells past the edge are walked but not written).
 template <typename T, typename TB, int ROWS>
 __global__ void __launch_bounds__(kStreamWarps * 32, stream_ctas_per_sm<T>())
-    v_stream_down(SView<T> L, StreamGeom g, const TB* __restrict__ bin, const double* level_sum,
-                  T* __restrict__ bc, T* bp_out) {
+    v_stream_down(SView<T> L, StreamGeom g, const TB* bin, const double* level_sum,
+                  T* bc, T* bp_out) {
     pdl_entry();
     constexpr int S = ROWS + 6, D = kStreamDepth;
     __shared__ P2<TB> stage[kStreamWarps][D][32];
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kStreamWarps * 32, stream_ctas_per_sm<T>())
 // of L.x (and the epilogue's sums) folded.
 template <typename T, typename Epi, int ROWS>
 __global__ void __launch_bounds__(kStreamWarps * 32, stream_ctas_per_sm<T>())
-    v_stream_up(SView<T> L, StreamGeom g, const T* __restrict__ xc, const T* __restrict__ bp_in, double* partial,
+    v_stream_up(SView<T> L, StreamGeom g, const T* xc, const T* bp_in, double* partial,
                 unsigned* counter, double* mean_out, Epi epi) {
     pdl_entry();
     constexpr int S = ROWS + 6, D = kStreamDepth;
