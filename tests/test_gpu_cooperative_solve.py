@@ -1,0 +1,37 @@
+"""`solve!` on the cooperative V-cycle (csrc/persistent.cuh) where it ends with an
+error: the caller's solution stays as it was.  A poll limit of 0
+(TPAGMG_BARRIER_SPINS) makes a grid barrier that has to wait give up at once; the
+launch runs to its end and nothing waits without a bound."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+import torch  # noqa: E402
+
+from tpagmg import BlockTreeMesh, EllipticSolver, PoissonOperator  # noqa: E402
+from tpagmg import workloads as W  # noqa: E402
+from tpagmg._lib import TPA_ERR_TIMEOUT, TpaError  # noqa: E402
+
+
+def build():
+    m = BlockTreeMesh(**W.droplet_spec(levels=2))
+    s = EllipticSolver(PoissonOperator(m, W.droplet_inputs(m)[1]))
+    s.set_tuning(structured=0, persistent=1, tail_ctas=1)
+    assert s.tuning()["persistent"] == 1
+    return m, s, torch.from_numpy(W.gaussian_rhs(m, 31)).cuda()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_a_barrier_timeout_leaves_the_solution(precision, monkeypatch):
+    m, s, rhs = build()
+    x = torch.full((m.ncells,), 3.0, dtype=torch.float64, device="cuda")
+    monkeypatch.setenv("TPAGMG_BARRIER_SPINS", "0")
+    s.set_tuning(structured=0, persistent=1, tail_ctas=1)
+    s.set_stream(0)
+    with pytest.raises(TpaError) as e:
+        s.solve_device(rhs.data_ptr(), x.data_ptr(), max_cycles=5, precision=precision)
+    assert e.value.code == TPA_ERR_TIMEOUT and bool((x == 3.0).all())
+    monkeypatch.delenv("TPAGMG_BARRIER_SPINS")
+    s.set_tuning(structured=0, persistent=1, tail_ctas=1)
+    assert s.solve_device(rhs.data_ptr(), x.data_ptr(), precision=precision).converged

@@ -283,6 +283,9 @@ void DeviceSolver::solve_fast(const double* rhs, double* x_user, double rtol, do
     };
     for (bool first_run = true;; first_run = false) {
         if (max_cycles > 0) cg_loop(precision);
+        // a run whose cooperative cycle gave up ends here, before the caller's
+        // solution is written
+        if (coop_grid_ > 0) check_barrier();
         // gauge of the iterate, then the true residual and its norms
         if (L.ncomp == 1) {
             plain(k_xmean, fold_grid(k_xmean, kThreads, want, kGrid), kThreads, 0, n, (const double*)xw_.p, vol, L.vol0,
@@ -308,7 +311,6 @@ void DeviceSolver::solve_fast(const double* rhs, double* x_user, double rtol, do
         if (linf <= guarded(linf, roundoff_floor(hs.fin[2], hs.fin[3]))) break;
         if (!std::isfinite(linf) || hs.niter == 0 || hs.total >= max_cycles) break;
     }
-    if (coop_grid_ > 0) check_barrier();
     auto l2 = [&](double s) { return vt > 0 ? std::sqrt(s / vt) : 0.0; };
     const double tfinal = guarded(hs.fin[1], roundoff_floor(hs.fin[2], hs.fin[3]));
     float ms = 0;
