@@ -249,7 +249,9 @@ void DeviceSolver::solve_fast(const double* rhs, double* x_user, double rtol, do
     double vt = 0;  // total volume of cells with V > 0
     for (double v : L.comp_volume) vt += v;
     if (L.ncomp == 0) vt = vol_total_;
-    if (precision == 2) ensure_ir();
+    // the refinement's runs need the multi-launch cycle
+    const bool no_run = precision == 2 && coop_grid_ > 0;
+    if (precision == 2 && !no_run) ensure_ir();
     TPA_CUDA(cudaEventRecord(ev0_, stream_));
     st = SolveStats();
 
@@ -276,13 +278,19 @@ void DeviceSolver::solve_fast(const double* rhs, double* x_user, double rtol, do
     };
     pres(std::true_type(), first, first.rhs == rhs ? go : plain);
     launches_ += 2;
+    if (no_run && max_cycles > 0) {
+        // refused where a run is due, with the caller's solution untouched
+        TPA_CUDA(cudaMemcpyAsync(host_solve_, S, sizeof(SolveState), cudaMemcpyDeviceToHost, stream_));
+        TPA_CUDA(cudaStreamSynchronize(stream_));
+        if (!hs.skip) ensure_ir();
+    }
     double target = 0, init_linf = 0;
     auto guarded = [&](double cur, double fl) {
         if (!(std::isfinite(init_linf) && std::isfinite(cur) && target < cur && cur < init_linf)) return target;
         return (std::isfinite(fl) && fl < init_linf / 100) ? std::max(target, fl) : target;
     };
     for (bool first_run = true;; first_run = false) {
-        if (max_cycles > 0) cg_loop(precision);
+        if (max_cycles > 0 && !no_run) cg_loop(precision);
         // a run whose cooperative cycle gave up ends here, before the caller's
         // solution is written
         if (coop_grid_ > 0) check_barrier();
