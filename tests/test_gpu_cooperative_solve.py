@@ -14,7 +14,7 @@ import torch  # noqa: E402
 
 from tpagmg import BlockTreeMesh, EllipticSolver, PoissonOperator  # noqa: E402
 from tpagmg import workloads as W  # noqa: E402
-from tpagmg._lib import TPA_ERR_TIMEOUT, TpaError  # noqa: E402
+from tpagmg._lib import TPA_ERR_NONFINITE, TPA_ERR_TIMEOUT, TPA_ERR_UNSUPPORTED, TpaError  # noqa: E402
 
 
 def build():
@@ -66,4 +66,4 @@ def test_refinement_without_a_run():
     s.set_stream(0)
     with pytest.raises(TpaError) as e:
         s.solve_device(b.data_ptr(), x.data_ptr(), precision="mixed_ir")
-    assert e.value.code == 4 and bool((x == 3.0).all())
+    assert e.value.code == TPA_ERR_NONFINITE and bool((x == 3.0).all())
