@@ -406,7 +406,8 @@ private:
     void coarse_inverse_lu();
     void finish_refresh(const std::function<void()>& meanwhile);
     bool refresh_lu_ = false;  // the coarse inverse by the pivoted LU at once
-    DevArray<double> coarse_shift_;
+    DevArray<int> coarse_held_;     // the cells the elimination holds at zero
+    DevArray<double> coarse_mean_;  // row means of its inverse
     double* host_wtw_ = nullptr;  // in rstage_'s allocation: the weights and the error word read back
     int* host_rerr_ = nullptr;
     DevArray<double> coarse_M_, coarse_MT_, rpart_;

@@ -216,58 +216,126 @@ __global__ void kr_coarse_fill(int n, int N, const int* __restrict__ rp, const i
     }
 }
 
-// ---- the coarse inverse by block elimination ------------------------------------
+// ---- the coarsest level's inverse -------------------------------------------------
 //
 // The coarse solve needs the n x n block G of [A v; v' 0]^-1 (v: the volumes, one
-// column per ungauged component).  A is symmetric, its null space is the
-// components' constants, so B = A + sum_s c_s v_s v_s' is positive definite and
-//   G = B^-1 - sum_s 1_s 1_s' / (c_s (1'v_s)^2)
-// (B 1_s = c_s (1'v_s) v_s, and the multiplier of the augmented system is
-// 1'b / 1'v).  c_s = d n_s / (1'v_s)^2, d the component's mean diagonal, puts the
-// added eigenvalue among A's.  B^-1 is formed in place by Gauss-Jordan
+// column per ungauged component).  A is symmetric and its null space is the
+// components' constants.  With one cell of each component held at zero (its row
+// and column taken out) A is positive definite; H, the inverse of that matrix
+// with zeros in the held rows and columns, solves A x = b for b of zero sum, and
+//   G = P H P',  P = I - sum_s 1_s v_s' / (1'v_s),
+// takes the sum off b and the volume mean off x.  H is formed by Gauss-Jordan
 // elimination over blocks of 32 rows, which needs no pivoting for a positive
 // definite matrix: ceil(n / 32) launches, each over all 32 x 32 tiles.
+//
+// The cell held is the one of the largest diagonal.  The potentials are then
+// measured from the strongest coefficients, and no entry of A meets one that A
+// does not have, so weak coefficients keep their digits beside strong ones.
+// Distance from the exact G over its largest entry, 16 x 16 cells with a disc of
+// coefficients K times the rest: 1e-15 at K = 1e3, 2e-15 at 1e6 and 1e10 (the
+// pivoted LU of the augmented matrix: 6e-15, 1e-12, 4e-8; a positive definite
+// matrix made by adding the volumes' outer product at the size of A's mean
+// diagonal: 3e-13, 3e-7, 0.2).
+//
 // Measured at n = 256: 8 launches in place of 257 dependent pivot steps in one
 // cluster (724 us) and the triangular solves (132 us).  A block whose pivots are
-// not positive (B singular to working precision) sets err 3, and the refresh
+// not positive (singular to working precision) sets err 3, and the refresh
 // takes the pivoted LU of the augmented matrix below instead.
 
 constexpr int kGj = 32;
 
-// B (row-major n x n) and shift[s] = 1 / (c_s (1'v_s)^2); a warp per row
-__global__ void kr_coarse_spd(int n, const int* __restrict__ rp, const int* __restrict__ ci,
-                              const double* __restrict__ val, const int* __restrict__ slot,
-                              const double* __restrict__ vol, int ncomp, double* __restrict__ B,
-                              double* __restrict__ shift) {
-    __shared__ double c[kMaxComponents];
+struct CompScale {
+    double inv[kMaxComponents];  // 1 / volume of an ungauged component
+};
+
+// (value, row) pairs: the larger value wins, ties go to the smaller row (the
+// first maximum of a sequential scan)
+__device__ __forceinline__ void better(double& v, int& i, double ov, int oi) {
+    if (ov > v || (ov == v && oi < i)) {
+        v = ov;
+        i = oi;
+    }
+}
+
+// B (row-major n x n): A with the held rows and columns replaced by the
+// identity's; held[s]: component s's cell.  A warp per row.
+__global__ void kr_coarse_held(int n, const int* __restrict__ rp, const int* __restrict__ ci,
+                               const double* __restrict__ val, const int* __restrict__ slot, int ncomp,
+                               double* __restrict__ B, int* __restrict__ held) {
+    __shared__ int g[kMaxComponents];
+    __shared__ double wv[32];
+    __shared__ int wi[32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = int(blockDim.x >> 5);
     for (int s = 0; s < ncomp; ++s) {
-        double tr = 0, cells = 0, vs = 0;
+        double v = -1.0;
+        int at = n;
         for (int i = threadIdx.x; i < n; i += blockDim.x) {
             if (slot[i] != s) continue;
-            cells += 1;
-            vs += vol[i];
             for (int k = rp[i]; k < rp[i + 1]; ++k)
-                if (ci[k] == i) tr += val[k];
+                if (ci[k] == i) better(v, at, val[k], i);
         }
-        tr = block_sum_all(tr);
-        cells = block_sum_all(cells);
-        vs = block_sum_all(vs);
+        for (int o = 16; o; o >>= 1)
+            better(v, at, __shfl_down_sync(0xffffffffu, v, o), __shfl_down_sync(0xffffffffu, at, o));
+        if (!lane) {
+            wv[wid] = v;
+            wi[wid] = at;
+        }
+        __syncthreads();
         if (threadIdx.x == 0) {
-            // an isolated component (no couplings) takes a unit diagonal
-            const double d = tr > 0 ? tr : cells;  // mean diagonal times cells
-            c[s] = d / (vs * vs);
-            if (blockIdx.x == 0) shift[s] = 1.0 / d;
+            for (int w = 1; w < nw; ++w) better(v, at, wv[w], wi[w]);
+            g[s] = at;
+            if (blockIdx.x == 0) held[s] = at;
         }
+        __syncthreads();
+    }
+    for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += (gridDim.x * blockDim.x) >> 5) {
+        double* row = B + size_t(r) * n;
+        const int s = ncomp ? slot[r] : -1, h = s >= 0 ? g[s] : -1;
+        for (int j = lane; j < n; j += 32) row[j] = r == h && j == r ? 1.0 : 0.0;
+        __syncwarp();
+        if (r == h) continue;
+        for (int k = rp[r] + lane; k < rp[r + 1]; k += 32)
+            if (ci[k] != h) row[ci[k]] = val[k];
+    }
+}
+
+// mean[i] = the volume mean of row i of H over its component; a warp per row
+__global__ void kr_coarse_means(int n, const double* __restrict__ H, const int* __restrict__ slot,
+                                const double* __restrict__ vol, const int* __restrict__ held, CompScale scale,
+                                double* __restrict__ mean) {
+    const int lane = threadIdx.x & 31;
+    for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += (gridDim.x * blockDim.x) >> 5) {
+        const int s = slot[r], h = s >= 0 ? held[s] : -1;
+        double a = 0;
+        if (s >= 0 && r != h)
+            for (int j = lane; j < n; j += 32)
+                if (slot[j] == s && j != h) a += H[size_t(r) * n + j] * vol[j];
+        for (int o = 16; o; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+        if (!lane) mean[r] = s >= 0 ? a * scale.inv[s] : 0.0;
+    }
+}
+
+// G = P H P': H less the means of its rows and columns, plus the mean of all
+__global__ void kr_coarse_gauge(int n, const double* __restrict__ H, const int* __restrict__ slot,
+                                const double* __restrict__ vol, const int* __restrict__ held, int ncomp,
+                                CompScale scale, const double* __restrict__ mean, double* __restrict__ G) {
+    __shared__ double all[kMaxComponents];
+    for (int s = 0; s < ncomp; ++s) {
+        double a = 0;
+        for (int i = threadIdx.x; i < n; i += blockDim.x)
+            if (slot[i] == s) a += vol[i] * mean[i];
+        a = block_sum_all(a);
+        if (threadIdx.x == 0) all[s] = a * scale.inv[s];
     }
     __syncthreads();
     const int lane = threadIdx.x & 31;
     for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += (gridDim.x * blockDim.x) >> 5) {
-        double* row = B + size_t(r) * n;
-        const int s = ncomp ? slot[r] : -1;
-        const double cv = s >= 0 ? c[s] * vol[r] : 0.0;
-        for (int j = lane; j < n; j += 32) row[j] = (s >= 0 && slot[j] == s) ? cv * vol[j] : 0.0;
-        __syncwarp();
-        for (int k = rp[r] + lane; k < rp[r + 1]; k += 32) row[ci[k]] += val[k];
+        const int s = slot[r], h = s >= 0 ? held[s] : -1;
+        for (int j = lane; j < n; j += 32) {
+            double v = r == h || j == h ? 0.0 : H[size_t(r) * n + j];
+            if (s >= 0 && slot[j] == s) v = v - mean[r] - mean[j] + all[s];
+            G[size_t(r) * n + j] = v;
+        }
     }
 }
 
@@ -276,11 +344,9 @@ __global__ void kr_coarse_spd(int n, const int* __restrict__ rp, const int* __re
 // kb, in - C D^-1 R elsewhere.  One CTA per tile of `out`; each inverts D
 // (rows beyond n: the identity), which is what a step waits for: 32 dependent
 // pivots (at 256 cells 18.0 us a step with D in shared memory and two barriers a
-// pivot, 12.5 us with one).  On the last step the tiles are
-// stored as G, less the components' shift.
+// pivot, 12.5 us with one).
 __global__ void __launch_bounds__(256) kr_gj_step(int n, int kb, const double* __restrict__ in,
-                                                  double* __restrict__ out, int last, const int* __restrict__ slot,
-                                                  int ncomp, const double* __restrict__ shift, int* err) {
+                                                  double* __restrict__ out, int* err) {
     __shared__ double D[kGj][kGj + 1], C[kGj][kGj + 1], R[kGj][kGj + 1];
     __shared__ double prow[2][kGj], pcol[2][kGj], pinv[2];
     const int ti = blockIdx.y, tj = blockIdx.x;
@@ -357,21 +423,11 @@ __global__ void __launch_bounds__(256) kr_gj_step(int n, int kb, const double* _
     for (int u = 0; u < 4; ++u) {
         const int j = tj * kGj + q + 8 * u;
         if (i >= n || j >= n) continue;
-        if (last && ncomp && slot[i] >= 0 && slot[i] == slot[j]) o[u] -= shift[slot[i]];
         out[size_t(i) * n + j] = o[u];
     }
 }
 
 // ---- the pivoted LU of the augmented matrix --------------------------------------
-
-// (value, row) pairs: the larger value wins, ties go to the smaller row (the
-// first maximum of a sequential scan)
-__device__ __forceinline__ void better(double& v, int& i, double ov, int oi) {
-    if (ov > v || (ov == v && oi < i)) {
-        v = ov;
-        i = oi;
-    }
-}
 
 template <bool Cl>
 __device__ __forceinline__ void lu_sync() {
@@ -810,7 +866,8 @@ void DeviceSolver::prepare_refresh(const Hierarchy& h) {
     TPA_CUDA(cudaMallocHost(&rstage_, sizeof(double) * (stage + 1)));
     host_wtw_ = rstage_ + std::max<size_t>(1, size_t(rl_[0].nf));
     host_rerr_ = reinterpret_cast<int*>(rstage_ + stage);
-    coarse_shift_.alloc(size_t(kMaxComponents));
+    coarse_held_.alloc(size_t(kMaxComponents));
+    coarse_mean_.alloc(size_t(std::max(1, levels_.back().n)));
     refresh_lu_ = std::getenv("TPAGMG_REFRESH_LU") != nullptr;  // the pivoted LU at once (diagnosis)
     rpart_.alloc(size_t(3 * 1184));
     rcnt_.alloc(1);
@@ -902,17 +959,24 @@ void DeviceSolver::refresh_levels(const std::function<void()>& meanwhile) {
     if (refresh_lu_) {
         coarse_inverse_lu();
     } else {
-        const int nb = (C.n + kGj - 1) / kGj;
-        kr_coarse_spd<<<std::min(148, (C.n + 7) / 8), 256, 0, s>>>(C.n, C.rowptr.p, C.col.p, C.d.val.p, C.slot.p,
-                                                                   C.d.vol.p, coarse_ncomp_, coarse_M_.p,
-                                                                   coarse_shift_.p);
+        const int nb = (C.n + kGj - 1) / kGj, rows = std::min(148, (C.n + 7) / 8);
+        kr_coarse_held<<<rows, 256, 0, s>>>(C.n, C.rowptr.p, C.col.p, C.d.val.p, C.slot.p, coarse_ncomp_,
+                                            coarse_M_.p, coarse_held_.p);
         const double* in = coarse_M_.p;
         for (int kb = 0; kb < nb; ++kb) {
-            const bool last = kb == nb - 1;
-            double* out = last ? coarse_inv_.p : in == coarse_M_.p ? coarse_MT_.p : coarse_M_.p;
-            kr_gj_step<<<dim3(nb, nb), 256, 0, s>>>(C.n, kb, in, out, last ? 1 : 0, C.slot.p, coarse_ncomp_,
-                                                    coarse_shift_.p, rerr_.p);
+            double* out = kb == nb - 1 && coarse_ncomp_ == 0 ? coarse_inv_.p
+                          : in == coarse_M_.p                ? coarse_MT_.p
+                                                             : coarse_M_.p;
+            kr_gj_step<<<dim3(nb, nb), 256, 0, s>>>(C.n, kb, in, out, rerr_.p);
             in = out;
+        }
+        if (coarse_ncomp_ > 0) {
+            CompScale scale{};
+            for (int k = 0; k < coarse_ncomp_; ++k) scale.inv[k] = 1.0 / C.comp_volume[size_t(k)];
+            kr_coarse_means<<<rows, 256, 0, s>>>(C.n, in, C.slot.p, C.d.vol.p, coarse_held_.p, scale,
+                                                 coarse_mean_.p);
+            kr_coarse_gauge<<<rows, 256, 0, s>>>(C.n, in, C.slot.p, C.d.vol.p, coarse_held_.p, coarse_ncomp_, scale,
+                                                 coarse_mean_.p, coarse_inv_.p);
         }
     }
     finish_refresh(meanwhile);
