@@ -729,7 +729,8 @@ void DeviceSolver::build_dense_tail() {
     const int n = levels_[size_t(t)].n;
     dense_n_ = 0;
     if (!fused_ok_ || rb_ || (n > kDenseTailCells && t != nl - 1)) return;
-    int optin = 0;
+    int optin = 0, sms = 0;
+    TPA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_));
     TPA_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
     const size_t room = size_t(optin) - 2048;  // the kernel's static shared memory
     const int ld = (n + 1) & ~1;
@@ -747,8 +748,8 @@ void DeviceSolver::build_dense_tail() {
         dense_n_ = n;
         dense_ld_ = ld;
     };
-    // the most columns that still leave a CTA for every SM: 8 above 4 x 148 cells
-    if (n > 592 && n <= 2 * kDenseBuildThreads) build(k_dense_tail_build<8, 2>, 8);
+    // the most columns that still leave a CTA for every SM: 8 above 4 cells an SM
+    if (n > 4 * sms && n <= 2 * kDenseBuildThreads) build(k_dense_tail_build<8, 2>, 8);
     if (n <= 2 * kDenseBuildThreads) build(k_dense_tail_build<4, 2>, 4);
     build(k_dense_tail_build<4, 4>, 4);
     build(k_dense_tail_build<2, 4>, 2);

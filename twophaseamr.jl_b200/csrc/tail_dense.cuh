@@ -20,8 +20,9 @@
 //
 // The map is used for tails of at most kDenseTailCells cells (n^2 doubles: 32
 // MB at 2048, about the time of the multi-CTA launches a smaller tail would
-// add) and, at any size that the set-up's shared memory holds, when the tail is
-// the coarsest level alone, whose dense inverse has n^2 entries already.
+// add) and, at any size, when the tail is the coarsest level alone, whose dense
+// inverse has n^2 entries already: at most 8191 cells (hierarchy.cpp), where the
+// map takes another 537 MB and one unit vector 131 KB of shared memory.
 #pragma once
 
 #include "fused.cuh"
@@ -34,11 +35,10 @@ constexpr int kDenseRows = 8;  // rows (warps) per CTA of the product
 
 // Shared memory of the set-up for `C` unit vectors: a right-hand side and an
 // iterate per level, the first level's right-hand side (known in closed form)
-// giving its place to a scratch vector; the coarsest level alone keeps room for
-// four vectors.
+// giving its place to a scratch vector.
 inline size_t dense_build_smem(const std::vector<LevelView<double>>& v, int first, int C) {
-    size_t cells = (size_t(first) + 1 == v.size() ? 4 : 2) * size_t(v[size_t(first)].n);
-    for (size_t l = size_t(first) + 1; l < v.size(); ++l) cells += 2 * size_t(v[l].n);
+    size_t cells = 0;
+    for (size_t l = size_t(first); l < v.size(); ++l) cells += 2 * size_t(v[l].n);
     return cells * size_t(C) * sizeof(double);
 }
 
