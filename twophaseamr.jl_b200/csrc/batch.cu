@@ -57,7 +57,6 @@ __global__ void bk_prep(const BFItem* fi, FineFold f, const double* __restrict__
     fine_fold<3>(f, v, 0u, it.prob, [&](const double (&t)[3]) {
         SolveState& s = S[it.prob];
         const double cv = comp_vol[it.prob];
-        s.sum_b = t[0];
         s.abs_b = t[1];
         s.ok = !(q.strict && cv > 0 && fabs(t[0]) > 256 * kEps * std_max(1.0, t[1]));
         s.mb = cv > 0 && s.ok ? t[0] / cv : 0.0;

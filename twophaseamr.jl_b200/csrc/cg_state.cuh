@@ -18,7 +18,7 @@ constexpr int kCgHalt = 2 | 4 | 8;
 // `solve!` around the runs (solve_fast.cu): every decision up to the end of the
 // first run is taken on the device, and the host reads this once per run.
 struct SolveState {
-    double sum_b, abs_b;                 // sum and sum of magnitudes of b = V f
+    double abs_b;                        // sum of magnitudes of b = V f
     double mb, mx, xm;                   // means removed from b, from the guess, from the iterate
     double init[4], fin[4];              // sum_V r^2 / V, max |r| / V, max |A||x| / V, max |b| / V
     double target;

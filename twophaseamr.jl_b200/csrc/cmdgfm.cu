@@ -1067,7 +1067,6 @@ void CmdgfmDevice::solve(DeviceSolver& ds, const CmdgfmInput& in, const CmdgfmFa
     TPA_CUDA(cudaMemsetAsync(full_.p, 0, sizeof(double) * size_t(std::max<int64_t>(ncells_, 1)), s));
     zfull_.alloc(size_t(std::max<int64_t>(ncells_, 1)));
     zp_.alloc(size_t(std::max<int64_t>(np_, 1)));
-    jr_.alloc(size_t(std::max<int64_t>(nx_, 1)));
     partial_.alloc(4 * size_t(kG));
     state_.alloc(kStateSize);
     TPA_CUDA(cudaMemsetAsync(sol_.p, 0, sizeof(double) * size_t(n_), s));

@@ -103,7 +103,6 @@ private:
     int body_launches_[2] = {0, 0};
     int64_t n_ = 0, np_ = 0, nx_ = 0, na_ = 0, ncells_ = 0;
     int launches_ = 0;
-    int precision_ = 0;
     // system
     DevBuf<int64_t> mptr_, eptr_;
     DevBuf<int32_t> mcol_, ecol_, cell_, anchor_, gptr_, gidx_, ganchor_;
@@ -125,7 +124,7 @@ private:
     DevBuf<int32_t> licol_, uicol_;
     DevBuf<double> lival_, uival_;
     // vectors
-    DevBuf<double> sol_, corr_, x_, r_, c_, p_, v_, s_, t_, y_, z_, full_, zfull_, zp_, jr_, partial_;
+    DevBuf<double> sol_, corr_, x_, r_, c_, p_, v_, s_, t_, y_, z_, full_, zfull_, zp_, partial_;
     DevBuf<double> state_;
 };
 

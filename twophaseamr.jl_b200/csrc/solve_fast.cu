@@ -60,7 +60,6 @@ __global__ void k_prep(int n, const double* rhs, const double* xin,
     }
     // in the order of the plain solve's sums: the removed mean is often rounding alone
     publish_fold<3, 0>(v, 0u, partial, counter, [&](const double (&t)[3]) {
-        S->sum_b = t[0];
         S->abs_b = t[1];
         const bool comp = q.cvol != 0;
         S->mb = comp ? t[0] / q.cvol : 0.0;

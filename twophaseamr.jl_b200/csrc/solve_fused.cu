@@ -51,16 +51,6 @@ static void with_stream_rows(int rows, F f) {
     else f(std::integral_constant<int, 36>{});
 }
 
-// the strip heights of the streamed CG direction kernel (finest level)
-template <typename F>
-static void with_cg_rows(int rows, F f) {
-    if (rows == 4) f(std::integral_constant<int, 4>{});
-    else if (rows == 8) f(std::integral_constant<int, 8>{});
-    else if (rows == 16) f(std::integral_constant<int, 16>{});
-    else if (rows == 24) f(std::integral_constant<int, 24>{});
-    else f(std::integral_constant<int, 36>{});
-}
-
 namespace {
 
 enum Counter { kPostMean = 1, kCgAp = 2, kCgUpdate = 3, kCgZ = 4, kCgRes = 5, kRsum = 6 };
@@ -499,7 +489,7 @@ __global__ void __launch_bounds__(kStreamWarps * 32, kStreamCgCtas)
         };
 #pragma unroll
         for (int k = 0; k < D - 1; ++k) {
-            stage(k);
+            if (k < S) stage(k);
             st_commit();
         }
         P2<double> q[S];

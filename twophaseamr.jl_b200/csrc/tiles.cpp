@@ -120,7 +120,6 @@ TileLevelHost build_tiles(const Csr& A, int64_t nblocks, int64_t cpb, const std:
         T.info.push_back(info);
         T.n3max = std::max(T.n3max, ring[3]);
         T.n2max = std::max(T.n2max, ring[2]);
-        T.n1max = std::max(T.n1max, ring[1]);
     }
     // every coarse cell belongs to exactly one tile
     if (int64_t(T.co.size()) != nc) return TileLevelHost();

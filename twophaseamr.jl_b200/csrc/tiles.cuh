@@ -512,14 +512,6 @@ __global__ void __launch_bounds__(kTileThreads)
     }
 }
 
-// e = P_tent x_c at the cell (li, lj) of block B (its map: coarse block, x / y offset, scale)
-template <typename T>
-__device__ __forceinline__ T vt_coarse(const SView<T>& L, const T* xc, int B, int li, int lj) {
-    const int4 mp = *reinterpret_cast<const int4*>(L.map + 4 * B);
-    if (mp.w == 1) return xc[mp.x * 256 + (mp.z + lj) * 16 + mp.y + li];
-    return xc[mp.x * 256 + (mp.z + (lj >> 1)) * 16 + mp.y + (li >> 1)];
-}
-
 template <typename T, typename Epi>
 __global__ void __launch_bounds__(kTileThreads)
     v_tile_up(SView<T> L, const T* xc, const T* bp_in, double* partial, unsigned* counter, double* mean_out, Epi epi) {

@@ -37,7 +37,7 @@ struct alignas(16) TileInfo {
 struct TileLevelHost {
     bool ok = false;
     int ntiles = 0;
-    int n3max = 0, n2max = 0, n1max = 0;  // largest ring counts (cumulative) over the tiles
+    int n3max = 0, n2max = 0;  // largest ring counts (cumulative) over the tiles
     std::vector<TileInfo> info;
     // the tiles' cells: the block's in order, then ring 1, ring 2, ring 3, each
     // with its tentative owner (coarse cell)
