@@ -1061,7 +1061,7 @@ void DeviceSolver::enqueue_cg_body(int precision, cudaGraphConditionalHandle han
         // p = z + beta p_old, Ap and alpha = gamma / p'Ap
         if (sdev_[0].vec && tdev_.size() && tdev_[0].stream) {
             const StreamGeom g = stream_cg_geom();
-            with_cg_rows(g.rows, [&](auto rows) {
+            with_stream_rows(g.rows, [&](auto rows) {
                 constexpr int RW = decltype(rows)::value;
                 go(v_stream_dir_ap<T, P, RW>, tdev_[0].cg_grid, kStreamWarps * 32, 0, sd_[0], g, (const T*)xv, mean,
                    pa, pb, ap, fpartial_.p, counters_.p + kCgAp, s);
