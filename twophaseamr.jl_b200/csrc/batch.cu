@@ -94,8 +94,8 @@ __global__ void bk_pres(const BFItem* fi, FineFold f, FineRows A, const double* 
         }
         const double xi = First && !(V > 0) ? -m : xin[i] - m;
         double acc = 0, aacc = 0;
-        const int* ci = A.ci + sl.x + (threadIdx.x & 31);
-        const double* val = A.val + sl.x + (threadIdx.x & 31);
+        const int* ci = A.ci + 32 * size_t(sl.x) + (threadIdx.x & 31);
+        const double* val = A.val + 32 * size_t(sl.x) + (threadIdx.x & 31);
 #pragma unroll 4
         for (int u = 0; u < sl.y; ++u) {
             const int j = ci[32 * u];
@@ -171,13 +171,17 @@ __global__ void __launch_bounds__(kItemRows)
     int c[kPre];
     double a[kPre];
     int2 sl;
+    const int* ci = nullptr;
+    const double* val = nullptr;
     auto load = [&](int q) {
         sl = fine_slice(A, q);
+        ci = A.ci + 32 * size_t(sl.x) + (threadIdx.x & 31);
+        val = A.val + 32 * size_t(sl.x) + (threadIdx.x & 31);
 #pragma unroll
         for (int u = 0; u < kPre; ++u)
             if (u < sl.y) {
-                c[u] = ld_static(A.ci + sl.x + 32 * u + (threadIdx.x & 31));
-                a[u] = ld_static(A.val + sl.x + 32 * u + (threadIdx.x & 31));
+                c[u] = ld_static(ci + 32 * u);
+                a[u] = ld_static(val + 32 * u);
             }
     };
     load(0);
@@ -192,8 +196,7 @@ __global__ void __launch_bounds__(kItemRows)
 #pragma unroll
         for (int u = 0; u < kPre; ++u)
             if (u < sl.y) y += a[u] * p[c[u]];
-        for (int u = kPre; u < sl.y; ++u)
-            y += A.val[sl.x + 32 * u + (threadIdx.x & 31)] * p[A.ci[sl.x + 32 * u + (threadIdx.x & 31)]];
+        for (int u = kPre; u < sl.y; ++u) y += val[32 * u] * p[ci[32 * u]];
         ap[i] = y;
         v[0] += p[i] * y;
     }
@@ -524,8 +527,8 @@ void BatchSolver::build(const std::vector<const Hierarchy*>& hs) {
                 int width = 0;
                 for (int i = it.begin + b; i < std::min(it.end, it.begin + b + 32); ++i)
                     width = std::max<int>(width, int(A.ptr[size_t(i - F) + 1] - A.ptr[size_t(i - F)]));
-                if (entries > INT32_MAX - 32 * int64_t(width)) throw Error(5, "batch has too many operator entries");
-                slice.push_back(int(entries));
+                if (entries / 32 > INT32_MAX - int64_t(width)) throw Error(5, "batch has too many operator entries");
+                slice.push_back(int(entries / 32));
                 slice.push_back(width);
                 entries += 32 * int64_t(width);
             }
@@ -545,7 +548,7 @@ void BatchSolver::build(const std::vector<const Hierarchy*>& hs) {
                     const bool in = i < it.end;
                     const int64_t e0 = in ? A.ptr[size_t(i - F)] : 0, e1 = in ? A.ptr[size_t(i - F) + 1] : 0;
                     for (int u = 0; u < slice[sl + 1]; ++u) {
-                        const size_t at = size_t(slice[sl]) + size_t(32 * u + r);
+                        const size_t at = 32 * size_t(slice[sl]) + size_t(32 * u + r);
                         ci[at] = e0 + u < e1 ? A.col[size_t(e0 + u)] + F : (in ? i : it.begin);
                         if (e0 + u < e1) val[at] = A.val[size_t(e0 + u)];
                     }
@@ -691,8 +694,8 @@ void BatchSolver::merge_rows(BLevelHost& H, const std::vector<const HostLevel*>&
             int64_t width = 0;
             for (int i = items[q].begin + 32 * w; i < std::min(items[q].end, items[q].begin + 32 * w + 32); ++i)
                 width = std::max(width, A.ptr[size_t(i - r0) + 1] - A.ptr[size_t(i - r0)]);
-            if (entries > INT32_MAX - 32 * width) throw Error(5, "batch level has too many nonzeros");
-            slice[2 * (q * (kItemRows / 32) + size_t(w))] = int(entries);
+            if (entries / 32 > INT32_MAX - width) throw Error(5, "batch level has too many nonzeros");
+            slice[2 * (q * (kItemRows / 32) + size_t(w))] = int(entries / 32);
             slice[2 * (q * (kItemRows / 32) + size_t(w)) + 1] = int(width);
             entries += 32 * width;
         }
@@ -714,7 +717,7 @@ void BatchSolver::merge_rows(BLevelHost& H, const std::vector<const HostLevel*>&
             const int l = i - it.begin;
             const size_t s = 2 * (q * (kItemRows / 32) + size_t(l / 32));
             for (int u = 0; u < slice[s + 1]; ++u) {
-                const size_t at = size_t(slice[s]) + size_t(32 * u + l % 32);
+                const size_t at = 32 * size_t(slice[s]) + size_t(32 * u + l % 32);
                 const int64_t e = A.ptr[size_t(i - r0)] + u;
                 const bool real = e < A.ptr[size_t(i - r0) + 1];
                 const int c = real ? A.col[size_t(e)] : i - r0;

@@ -54,7 +54,7 @@ struct BFItem {
 };
 
 // The finest rows of every problem in FP64 (fine space): slices of 32 rows of an
-// item, {first entry, width}, entry u of row k at 32 u + k (columns are
+// item, {first entry / 32, width}, entry u of row k at 32 u + k (columns are
 // fine-space rows; padding holds 0 on the row itself), so that a warp's loads
 // are consecutive.
 struct FineRows {
@@ -74,7 +74,7 @@ struct FineFold {
 };
 
 // One batch level: its vectors and, when its phases stream over the rows, the
-// work items with the operator in slices of 32 rows of an item ({first entry,
+// work items with the operator in slices of 32 rows of an item ({first entry / 32,
 // width}, entry u of row k at 32 u + k; padding: value 0).  ci holds the columns,
 // cc their owners (rows of the next coarser batch level).
 template <typename T>
@@ -264,8 +264,9 @@ struct BRow {
     __device__ __forceinline__ void load(const BLevel<T>& L, const int* cols) {
         const int2 s = ld_static(L.slice + size_t(blockIdx.x) * (kItemRows / 32) + (threadIdx.x >> 5));
         w = s.y;
-        val = L.val + s.x + (threadIdx.x & 31);
-        col = cols + s.x + (threadIdx.x & 31);
+        const size_t at = 32 * size_t(s.x) + (threadIdx.x & 31);
+        val = L.val + at;
+        col = cols + at;
 #pragma unroll
         for (int u = 0; u < kPre; ++u)
             if (u < w) {
