@@ -171,17 +171,14 @@ __global__ void __launch_bounds__(kItemRows)
     int c[kPre];
     double a[kPre];
     int2 sl;
-    const int* ci = nullptr;
-    const double* val = nullptr;
     auto load = [&](int q) {
         sl = fine_slice(A, q);
-        ci = A.ci + 32 * size_t(sl.x) + (threadIdx.x & 31);
-        val = A.val + 32 * size_t(sl.x) + (threadIdx.x & 31);
+        const size_t at = 32 * size_t(unsigned(sl.x)) + (threadIdx.x & 31);
 #pragma unroll
         for (int u = 0; u < kPre; ++u)
             if (u < sl.y) {
-                c[u] = ld_static(ci + 32 * u);
-                a[u] = ld_static(val + 32 * u);
+                c[u] = ld_static(A.ci + at + 32 * u);
+                a[u] = ld_static(A.val + at + 32 * u);
             }
     };
     load(0);
@@ -196,7 +193,10 @@ __global__ void __launch_bounds__(kItemRows)
 #pragma unroll
         for (int u = 0; u < kPre; ++u)
             if (u < sl.y) y += a[u] * p[c[u]];
-        for (int u = kPre; u < sl.y; ++u) y += val[32 * u] * p[ci[32 * u]];
+        for (int u = kPre; u < sl.y; ++u) {
+            const size_t at = 32 * size_t(unsigned(sl.x)) + size_t(32 * u) + (threadIdx.x & 31);
+            y += A.val[at] * p[A.ci[at]];
+        }
         ap[i] = y;
         v[0] += p[i] * y;
     }

@@ -264,7 +264,7 @@ struct BRow {
     __device__ __forceinline__ void load(const BLevel<T>& L, const int* cols) {
         const int2 s = ld_static(L.slice + size_t(blockIdx.x) * (kItemRows / 32) + (threadIdx.x >> 5));
         w = s.y;
-        const size_t at = 32 * size_t(s.x) + (threadIdx.x & 31);
+        const size_t at = 32 * size_t(unsigned(s.x)) + (threadIdx.x & 31);
         val = L.val + at;
         col = cols + at;
 #pragma unroll
