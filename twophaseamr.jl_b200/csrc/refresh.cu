@@ -307,9 +307,13 @@ __global__ void kr_coarse_means(int n, const double* __restrict__ H, const int* 
     for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += (gridDim.x * blockDim.x) >> 5) {
         const int s = slot[r], h = s >= 0 ? held[s] : -1;
         double a = 0;
-        if (s >= 0 && r != h)
-            for (int j = lane; j < n; j += 32)
-                if (slot[j] == s && j != h) a += H[size_t(r) * n + j] * vol[j];
+        if (s >= 0 && r != h) {
+#pragma unroll 8
+            for (int j = lane; j < n; j += 32) {
+                const double t = H[size_t(r) * n + j] * vol[j];
+                a += slot[j] == s && j != h ? t : 0.0;
+            }
+        }
         for (int o = 16; o; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
         if (!lane) mean[r] = s >= 0 ? a * scale.inv[s] : 0.0;
     }
@@ -331,10 +335,13 @@ __global__ void kr_coarse_gauge(int n, const double* __restrict__ H, const int* 
     const int lane = threadIdx.x & 31;
     for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < n; r += (gridDim.x * blockDim.x) >> 5) {
         const int s = slot[r], h = s >= 0 ? held[s] : -1;
+        const double mr = mean[r], ms = s >= 0 ? all[s] : 0.0;
+#pragma unroll 8
         for (int j = lane; j < n; j += 32) {
-            double v = r == h || j == h ? 0.0 : H[size_t(r) * n + j];
-            if (s >= 0 && slot[j] == s) v = v - mean[r] - mean[j] + all[s];
-            G[size_t(r) * n + j] = v;
+            const double t = H[size_t(r) * n + j], mj = mean[j];
+            const int sj = slot[j];
+            const double v = r == h || j == h ? 0.0 : t;
+            G[size_t(r) * n + j] = s >= 0 && sj == s ? v - mr - mj + ms : v;
         }
     }
 }
