@@ -218,7 +218,7 @@ typedef struct tpa_batch tpa_batch;
 tpa_status tpa_batch_create(tpa_batch** out, tpa_context* const* ctxs, int32_t count);
 void tpa_batch_destroy(tpa_batch* batch);
 const char* tpa_batch_last_error(const tpa_batch* batch);
-/* out = {problems, fine cells (all problems), batch levels, levels of the per-problem one-CTA tail} */
+/* out = {problems, fine cells (all problems), batch levels, levels solved by a dense product (1: the last)} */
 tpa_status tpa_batch_sizes(const tpa_batch* batch, int64_t out[4]);
 /* offsets[k] = first fine cell of problem k in the concatenated arrays (count + 1 entries). */
 tpa_status tpa_batch_offsets(const tpa_batch* batch, int64_t* offsets);
@@ -240,7 +240,9 @@ tpa_status tpa_batch_solve_device(tpa_batch* batch, const double* rhs, double* x
 /* Device layout of the V-cycle (no reference counterpart: the reference's
  * cycle runs on the host).  Negative fields mean "default".  tail_cells: levels
  * with at most this many cells run in the coarse tail; tail_ctas: CTAs of the
- * tail's thread-block cluster (1-8); structured: 0 CSR kernels everywhere, 1
+ * tail's thread-block cluster (1-8; no effect where the tail runs as one dense
+ * product: damped Jacobi, at most 2048 cells or the coarsest level alone);
+ * structured: 0 CSR kernels everywhere, 1
  * stencil kernels on constant-coefficient levels without coarse-fine rows,
  * 2 stencil kernels wherever the transfer has a block map; vectorized: 4-cell
  * kernels on constant-coefficient 16x16 levels; pdl: programmatic dependent
@@ -249,7 +251,7 @@ tpa_status tpa_batch_solve_device(tpa_batch* batch, const double* rhs, double* x
  * recomputed inside the restriction (one launch instead of two); persistent:
  * when every multi-CTA level is a CSR level, the whole V-cycle runs as one
  * cooperative launch with grid barriers (bounded waits; a barrier that gives up
- * makes the solve return TPA_ERR_TIMEOUT); tiles: 1 runs each
+ * makes the solve return TPA_ERR_TIMEOUT with x as it was); tiles: 1 runs each
  * CSR level of the multi-CTA part as two launches on haloed block tiles (both
  * pre-sweeps, the residual and the restriction in one, the prolongation and
  * both post-sweeps in the other; the halo is recomputed in each tile), 2 also
@@ -336,7 +338,7 @@ tpa_status tpa_residual_norms_noalloc(tpa_context* ctx, const double* r, const d
                                       double out[2]);
 /* Device layout of the uploaded hierarchy: out = {levels on the block-
  * structured stencil path, exception (CSR) rows on those levels, first level
- * of the single-CTA coarse tail, 1 if the fused default cycle is used}.
+ * of the coarse tail, 1 if the fused default cycle is used}.
  * Uploads the hierarchy if needed. */
 tpa_status tpa_device_info(tpa_context* ctx, int64_t out[4]);
 /* Number of levels whose V-cycle phases run on haloed block tiles under the

@@ -31,7 +31,8 @@ namespace tpa {
 
 // Levels at or below this many cells run in the coarse tail, one cluster of
 // kTailCtasDefault CTAs of kTailThreads threads (TPAGMG_TAIL_CELLS, TPAGMG_TAIL_CTAS).
-// At most kDenseTailCells cells run as one dense product (tail_dense.cuh, 3 us);
+// At most kDenseTailCells cells run as one dense product (tail_dense.cuh: 4.7 us
+// at 1024 cells, 9 us at 2048);
 // k_tail walks the rest: it is bound by the latency of its dependent loads, so
 // more CTAs or a larger tail (4096 to 32768 cells, 4 or 8 CTAs) were 2-15 %
 // slower than 2048 cells in one CTA (droplet AMR and uniform 2048^2 solves).

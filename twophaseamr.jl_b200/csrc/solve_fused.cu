@@ -67,8 +67,11 @@ constexpr int kMaxGrid = 1184;  // 8 CTAs on each of 148 SMs: bounds the partial
 // keep.
 constexpr int kStencilTileCells = 1 << 19;
 // rz_foldable: the largest streamed or stencil-tiled finest level whose r'z rides
-// on the up kernel.  1024 x 512 with mixed_ir: 748 us a solve with the pass of its
-// own, 707 us folded; 2048^2: the up kernel 21 -> 34 us, the pass 12.8 us.
+// on the up kernel.  Periodic solves with a pass of its own and folded, mixed /
+// FP64 / mixed_ir, us: 2^19 cells 626 / 737 / 682 and 589 / 690 / 647; 2^20 761 /
+// 949 / 814 and 758 / 938 / 779; 2^21 1103 / 1468 / 1144 and 1106 / 1450 / 1131;
+// 2^22 1686 / 2160 / 1667 and 1722 / 2275 / 1692 (the up kernel 21 -> 34 us, the
+// pass 12.8 us).  Above 2^20 nothing is left to gain in the mixed solve.
 constexpr int kRzCells = 1 << 20;
 #define TPA_GRID_STRIDE(i, n) for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += gridDim.x * blockDim.x)
 

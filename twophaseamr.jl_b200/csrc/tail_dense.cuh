@@ -19,10 +19,14 @@
 // 1581 -> 1321, droplet of 110k cells 1955 -> 1707 us.
 //
 // The map is used for tails of at most kDenseTailCells cells (n^2 doubles: 32
-// MB at 2048, about the time of the multi-CTA launches a smaller tail would
-// add) and, at any size, when the tail is the coarsest level alone, whose dense
-// inverse has n^2 entries already: at most 8191 cells (hierarchy.cpp), where the
-// map takes another 537 MB and one unit vector 131 KB of shared memory.
+// MB at 2048) and, at any size, when the tail is the coarsest level alone, whose
+// dense inverse has n^2 entries already: at most 8191 cells (hierarchy.cpp), where
+// the map takes another 537 MB and one unit vector 131 KB of shared memory.
+// At 2048 + 512 cells against a tail of 512 below two launches of the 2048-cell
+// level: solves of 64 x 32 to 1024 x 512 periodic cells 0-8 % slower mixed (325
+// and 300 us at 128 x 64), 0-8 % FP64, and 256 x 128 walled cells on tiles 473 and
+// 459 us; a refresh that forms the map 776 and 549 us.  The walked tail of that
+// size takes 37 us a V-cycle in place of 9.
 #pragma once
 
 #include "fused.cuh"

@@ -283,7 +283,8 @@ class EllipticSolver:
 
     def solve_device(self, rhs_ptr, x_ptr, *, rtol=1e-10, atol=0.0, max_cycles=100, compatibility="project",
                      precision=None):
-        """`solve!` on device arrays (raw CUDA pointers, cell order)."""
+        """`solve!` on device arrays (raw CUDA pointers, cell order), on the stream
+        of the last `set_stream`; other streams' work on them must be over."""
         st = _lib.StatsC()
         self.ctx.call("tpa_solve_device", C.c_void_p(rhs_ptr), C.c_void_p(x_ptr), float(rtol), float(atol),
                       int(max_cycles), _compat(compatibility), _PRECISION[precision or self.precision], C.byref(st))
@@ -308,8 +309,8 @@ def solve_batched(solutions, solvers, rhs, *, rtol=1e-10, atol=0.0, max_cycles=1
     """`solve!` for many independent problems at once (one `EllipticSolver`
     per problem; solvers must be distinct).  `solutions[k]` (initial guess in,
     solution out) and `rhs[k]` are float64 cell arrays of problem k: numpy
-    arrays, or raw CUDA pointers (ints) on the solvers' device.  Returns a
-    `BatchResult`; raises on the first failed problem after all have run."""
+    arrays, or raw CUDA pointers (ints) on the solvers' device (each problem runs
+    on its own solver's stream).  Returns a `BatchResult`; raises on the first failed problem after all have run."""
     count = len(solvers)
     if len(solutions) != count or len(rhs) != count:
         raise ValueError("one solution and one right-hand side are required per solver")
